@@ -43,6 +43,7 @@ struct hb_handle {
     hb::DevMesh<hb::F64Exact> m64{};
     hb::DevMesh<hb::F32Fast> m32{};
     hb::DevMesh<hb::F32Split> ms{};
+    int ncseg = 0;                   // CTAs of cell_kernel (hb_cells_build; 0 = not used)
     uint32_t *d_err = nullptr;
     long long *d_ctr = nullptr;
     int32_t *d_perm = nullptr;       // scenario permutations, concatenated
@@ -141,6 +142,14 @@ int hb_tiles_launch(hb_handle *h, int n, cudaStream_t st);
 int hb_tiles_set_smem(hb_handle *h);
 // CTAs per SM of a tile-layout launch shape with tiles of about tile_cells cells
 int hb_tiles_resident(hb_handle *h, int config, int tile_cells, int *per_sm);
+// Small fp64 meshes (hb_cells.cu): whether the handle's steps run as one
+// cell_kernel launch each, the slot table those kernels read, and n such
+// steps (without the counter's tick; coef: also the update coefficients)
+bool hb_cells_used(const hb_handle *h);
+int hb_cells_build(hb_handle *h, const std::vector<int4> &rix, const std::vector<uint8_t> &rmeta,
+                   const std::vector<double> &rgeo);
+int hb_cells_launch(hb_handle *h, const hb::DevMesh<hb::F64Exact> &m, int k0, int n, int write_last, bool coef,
+                    cudaStream_t st);
 // One fp64 edge-layout step t0 + k (the device step counter must hold t0)
 // from state `in` to state `out` ([C][4] each), keeping the slots' terms of
 // the cell sums in `terms` ([4C][4]) and the update coefficients of the wet

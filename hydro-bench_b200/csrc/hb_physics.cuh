@@ -69,23 +69,22 @@ struct F64Exact {
     static __device__ __forceinline__ double div(double a, double b) { return __ddiv_rn(a, b); }
     // x / c for a constant c, correctly rounded: RN(x/c) == __ddiv_rn(x, c).
     // Method: Markstein's theorem (P. Markstein, IBM J. Res. Dev. 34(1), 1990;
-    // J.-M. Muller et al., Handbook of Floating-Point Arithmetic, ch. 4): if y is
-    // within half an ulp of 1/c and q within one ulp of x/c, then
+    // J.-M. Muller et al., Handbook of Floating-Point Arithmetic, ch. 4): if
+    // y = RN(1/c) and q is within one ulp of x/c, then
     // RN(q + RN(x - q*c)*y) = RN(x/c), the remainder being exact in an FMA.
-    // y = RN(1/c) is folded at compile time; one refinement of q0 = RN(x*y)
-    // brings q within one ulp, the second step rounds correctly.  Zeros,
-    // infinities, NaNs and |x| outside [2^-900, 2^900] (far from over/underflow
-    // of every quotient here) take __ddiv_rn.  Five FP64 operations instead
-    // of the ~18 instructions of __ddiv_rn.
+    // q = RN(x*y) is within 1/2 ulp + e * 2^53 ulp of x/c, e the relative
+    // error of y: below one ulp where e <= 2^-54, which holds for every
+    // constant divided by here (3, 10 and 0.1: 2^-54; 9.81 and its multiples
+    // by powers of two 39.24, 4.905, 313.92: 0.27 * 2^-54).  Zeros,
+    // infinities, NaNs and |x| outside [2^-900, 2^900) (far from
+    // over/underflow of every quotient here) take __ddiv_rn; one unsigned
+    // compare of the high word tells them.
     static __device__ __forceinline__ double divk(double x, double c) {
         const double y = 1.0 / c;
-        const double ax = ::fabs(x);
-        if (ax >= 0x1p-900 && ax <= 0x1p+900) {
-            double q = __dmul_rn(x, y);
-            double r = __fma_rn(-q, c, x);
-            q = __fma_rn(r, y, q);
-            r = __fma_rn(-q, c, x);
-            return __fma_rn(r, y, q);
+        const unsigned e = ((unsigned)__double2hiint(x) & 0x7FFFFFFFu) - ((1023u - 900u) << 20);
+        if (e < (1800u << 20)) {
+            const double q = __dmul_rn(x, y);
+            return __fma_rn(__fma_rn(-q, c, x), y, q);
         }
         return __ddiv_rn(x, c);
     }
@@ -845,11 +844,9 @@ struct CellUpdateIn {
     R h, u, v, fnc;
     L zbc;
     R hlo;             // split precision: the depth's compensation term
-    R dta_or_area;     // variant H: DT/AREA; variant F: AREA
-    R sidex;           // variant F: the CFL length of the cell (v0 functors.cu:752-763)
 };
 template <class R, class L = R>
-struct CellUpdateOut { R h, u, v, w; L z; R hlo; };
+struct CellUpdateOut { R h, u, v; L z; R hlo; };
 
 // accumulate slot j's contribution (functors.cu:732-742), in slot order
 template <class A>
@@ -876,24 +873,56 @@ __device__ __forceinline__ void st_global_f64x4(double *p, double x, double y, d
     asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" :: "l"(p), "d"(x), "d"(y), "d"(z), "d"(w) : "memory");
 }
 
-// COEF: also write the cell's update coefficients to `coef` when the cell is
-// wet after the step (H2 > HM2; fp64 only).
-template <class A, int VARIANT, bool COEF = false>
-__device__ __forceinline__ CellUpdateOut<typename A::real, typename A::level>
-update_cell(const CellUpdateIn<typename A::real, typename A::level> &c, typename A::real wh, typename A::real wu,
-            typename A::real wv, const StepParams &p, double *coef = nullptr) {
+// Bed friction of a cell's velocity update, DTW = DT FNC |(U, V)| / H^0.33333
+// (functors.cu:766-772); sq and hp are its square root and power.  It depends
+// on the state before the step alone.
+template <class R> struct Friction { R sq, hp, dtw; };
+template <class A>
+__device__ __forceinline__ Friction<typename A::real> cell_friction(typename A::real h, typename A::real u,
+                                                                    typename A::real v, typename A::real fnc,
+                                                                    const StepParams &p) {
+    Friction<typename A::real> f;
+    f.sq = A::sqrt(A::dot(u, u, v, v, M_SQ1));
+    f.hp = A::pow(h, A::c(0.33333));
+    f.dtw = A::mul(A::c(p.dt), A::div(A::mul(fnc, f.sq), f.hp));
+    return f;
+}
+
+// DT/AREA of the cell's step: a constant in variant H; in variant F from the
+// CFL length and the state before the step (v0 functors.cu:752-763).
+template <class A, int VARIANT>
+__device__ __forceinline__ typename A::real cell_dta(typename A::real h, typename A::real u,
+                                                     typename A::real dta_or_area, typename A::real sidex,
+                                                     const StepParams &p) {
     using R = typename A::real;
-    const R HM1 = A::c(p.hm1), HM2 = A::c(p.hm2), DT = A::c(p.dt);
-    R dta;
     if (VARIANT == 1) {
-        R hside = A::fmax(c.h, HM1);
-        R dt2 = A::div(c.sidex, A::add(c.u, A::sqrt(A::mul(A::c(9.81), hside))));
+        const R DT = A::c(p.dt);
+        R hside = A::fmax(h, A::c(p.hm1));
+        R dt2 = A::div(sidex, A::add(u, A::sqrt(A::mul(A::c(9.81), hside))));
         dt2 = A::fmin(DT, dt2);
         dt2 = A::fmax(dt2, A::divk(DT, 10.0));
-        dta = A::div(dt2, c.dta_or_area);
-    } else {
-        dta = c.dta_or_area;
+        return A::div(dt2, dta_or_area);
     }
+    return dta_or_area;
+}
+
+// W = |(U, V)| (functors.cu:777)
+template <class A>
+__device__ __forceinline__ typename A::real speed(typename A::real u, typename A::real v) {
+    return A::sqrt(A::dot(u, u, v, v, M_SQ2));
+}
+
+// The cell's new state from the slot sums.  `friction` returns the cell's
+// Friction and is called for the cells that are wet after the step (H2 > HM2)
+// only.  COEF: also write those cells' update coefficients to `coef` (fp64
+// only).
+template <class A, int VARIANT, bool COEF = false, class FrictionOf>
+__device__ __forceinline__ CellUpdateOut<typename A::real, typename A::level>
+update_cell(const CellUpdateIn<typename A::real, typename A::level> &c, typename A::real dta, typename A::real wh,
+            typename A::real wu, typename A::real wv, const StepParams &p, const FrictionOf &friction,
+            double *coef = nullptr) {
+    using R = typename A::real;
+    const R HM1 = A::c(p.hm1), HM2 = A::c(p.hm2);
     const R cap = A::c(VARIANT == 1 ? 5.0 : 15.0);
     CellUpdateOut<R, typename A::level> o;
     o.hlo = R(0);
@@ -918,22 +947,18 @@ update_cell(const CellUpdateIn<typename A::real, typename A::level> &c, typename
         o.u = A::copysign(A::fmin(A::c(K::VMIN), A::fabs(c.u)), c.u);
         o.v = A::copysign(A::fmin(A::c(K::VMIN), A::fabs(c.v)), c.v);
     } else {
-        const R sq = A::sqrt(A::dot(c.u, c.u, c.v, c.v, M_SQ1));
-        const R hp = A::pow(c.h, A::c(0.33333));
-        R wsf = A::div(A::mul(c.fnc, sq), hp);
-        R dtw = A::mul(DT, wsf);
-        R u2 = A::div(A::madd(-dtw, c.u, A::dot(c.h, c.u, -dta, wu, M_U2A), M_U2B), o.h);
-        R v2 = A::div(A::madd(-dtw, c.v, A::dot(c.h, c.v, -dta, wv, M_U2A), M_U2B), o.h);
+        const Friction<R> f = friction();
+        R u2 = A::div(A::madd(-f.dtw, c.u, A::dot(c.h, c.u, -dta, wu, M_U2A), M_U2B), o.h);
+        R v2 = A::div(A::madd(-f.dtw, c.v, A::dot(c.h, c.v, -dta, wv, M_U2A), M_U2B), o.h);
         o.u = A::copysign(A::fmin(A::fabs(u2), cap), u2);
         o.v = A::copysign(A::fmin(A::fabs(v2), cap), v2);
         if constexpr (COEF) {
             static_assert(std::is_same<R, double>::value, "update coefficients are fp64");
-            const double ihp = 1.0 / hp;
-            st_global_f64x4(coef, dtw, 1.0 / o.h, DT * sq * ihp, DT * c.fnc * sq * (-0.33333) * ihp / c.h);
-            st_global_f64x4(coef + 4, sq > 0.0 ? DT * c.fnc * ihp / sq : 0.0, 0.0, 0.0, 0.0);
+            const double DT = p.dt, ihp = 1.0 / f.hp;
+            st_global_f64x4(coef, f.dtw, 1.0 / o.h, DT * f.sq * ihp, DT * c.fnc * f.sq * (-0.33333) * ihp / c.h);
+            st_global_f64x4(coef + 4, f.sq > 0.0 ? DT * c.fnc * ihp / f.sq : 0.0, 0.0, 0.0, 0.0);
         }
     }
-    o.w = A::sqrt(A::dot(o.u, o.u, o.v, o.v, M_SQ2));
     return o;
 }
 

@@ -74,23 +74,26 @@ __global__ void __launch_bounds__(256) ref_update_kernel(typename RefView<typena
     }
     CellUpdateIn<R> ci;
     ci.h = c.H[pos]; ci.u = c.U[pos]; ci.v = c.V[pos]; ci.zbc = c.ZBC[pos]; ci.fnc = c.FNC[pos];
+    ci.hlo = R(0);
+    R dta, sidex = R(0);
     if (VARIANT == 1) {
         // SIDEX: triangle inradius or smaller mid-width of a quad (v0 functors.cu:752-763)
         const R s0 = sd.SIDE[4 * pos], s1 = sd.SIDE[4 * pos + 1], s2 = sd.SIDE[4 * pos + 2], s3 = sd.SIDE[4 * pos + 3];
         if (s3 > R(0)) {
-            ci.sidex = A::fmin(A::mul(A::c(0.5), A::add(s0, s2)), A::mul(A::c(0.5), A::add(s1, s3)));
+            sidex = A::fmin(A::mul(A::c(0.5), A::add(s0, s2)), A::mul(A::c(0.5), A::add(s1, s3)));
         } else {
             R ss = A::mul(A::c(0.5), A::add(A::add(s0, s1), s2));
-            ci.sidex = A::sqrt(A::div(A::mul(A::mul(A::sub(ss, s0), A::sub(ss, s1)), A::sub(ss, s2)), ss));
+            sidex = A::sqrt(A::div(A::mul(A::mul(A::sub(ss, s0), A::sub(ss, s1)), A::sub(ss, s2)), ss));
         }
-        ci.dta_or_area = c.AREA[pos];
+        dta = c.AREA[pos];
     } else {
-        ci.sidex = R(0);
-        ci.dta_or_area = A::div(A::c((double)m.DT), c.AREA[pos]);
+        dta = A::div(A::c((double)m.DT), c.AREA[pos]);
     }
     StepParams p{(double)m.HM1, (double)m.HM2, (double)m.JL, (double)m.DT, 0, 0};
-    CellUpdateOut<R> o = update_cell<A, VARIANT>(ci, wh, wu, wv, p);
-    c.H[pos] = o.h; c.U[pos] = o.u; c.V[pos] = o.v; c.Z[pos] = o.z; c.W[pos] = o.w;
+    dta = cell_dta<A, VARIANT>(ci.h, ci.u, dta, sidex, p);
+    CellUpdateOut<R> o = update_cell<A, VARIANT>(ci, dta, wh, wu, wv, p,
+                                                 [&]() { return cell_friction<A>(ci.h, ci.u, ci.v, ci.fnc, p); });
+    c.H[pos] = o.h; c.U[pos] = o.u; c.V[pos] = o.v; c.Z[pos] = o.z; c.W[pos] = speed<A>(o.u, o.v);
 }
 
 template <class A, class View>
@@ -266,22 +269,25 @@ __global__ void __launch_bounds__(256) static_update_kernel(hb_ref_mesh_view m, 
     }
     CellUpdateIn<double> ci;
     ci.h = c.H[pos]; ci.u = c.U[pos]; ci.v = c.V[pos]; ci.zbc = c.ZBC[pos]; ci.fnc = c.FNC[pos];
+    ci.hlo = 0.0;
+    double dta, sidex = 0.0;
     if (VARIANT == 1) {
         const double s0 = sd.SIDE[4 * pos], s1 = sd.SIDE[4 * pos + 1], s2 = sd.SIDE[4 * pos + 2], s3 = sd.SIDE[4 * pos + 3];
         if (s3 > 0.0) {
-            ci.sidex = A::fmin(A::mul(0.5, A::add(s0, s2)), A::mul(0.5, A::add(s1, s3)));
+            sidex = A::fmin(A::mul(0.5, A::add(s0, s2)), A::mul(0.5, A::add(s1, s3)));
         } else {
             double ss = A::mul(0.5, A::add(A::add(s0, s1), s2));
-            ci.sidex = A::sqrt(A::div(A::mul(A::mul(A::sub(ss, s0), A::sub(ss, s1)), A::sub(ss, s2)), ss));
+            sidex = A::sqrt(A::div(A::mul(A::mul(A::sub(ss, s0), A::sub(ss, s1)), A::sub(ss, s2)), ss));
         }
-        ci.dta_or_area = c.AREA[pos];
+        dta = c.AREA[pos];
     } else {
-        ci.sidex = 0.0;
-        ci.dta_or_area = A::div(m.DT, c.AREA[pos]);
+        dta = A::div(m.DT, c.AREA[pos]);
     }
     StepParams p{m.HM1, m.HM2, m.JL, m.DT, 0, 0};
-    CellUpdateOut<double> o = update_cell<A, VARIANT>(ci, wh, wu, wv, p);
-    c.H[pos] = o.h; c.U[pos] = o.u; c.V[pos] = o.v; c.Z[pos] = o.z; c.W[pos] = o.w;
+    dta = cell_dta<A, VARIANT>(ci.h, ci.u, dta, sidex, p);
+    CellUpdateOut<double> o = update_cell<A, VARIANT>(ci, dta, wh, wu, wv, p,
+                                                      [&]() { return cell_friction<A>(ci.h, ci.u, ci.v, ci.fnc, p); });
+    c.H[pos] = o.h; c.U[pos] = o.u; c.V[pos] = o.v; c.Z[pos] = o.z; c.W[pos] = speed<A>(o.u, o.v);
 }
 
 }  // namespace hb

@@ -580,6 +580,7 @@ int build_device_mesh(hb_handle *h, const hb_mesh_desc *mds, int n, hb::DevMesh<
     for (const auto &sc : h->scn) perms.insert(perms.end(), sc.perm.begin(), sc.perm.end());
     TRY(dev_upload(h, &h->d_perm, perms));
     TRY(dev_alloc(h, &h->d_stage, 5 * (size_t)h->max_cells));
+    if constexpr (std::is_same<A, hb::F64Exact>::value) TRY(hb_cells_build(h, hm.rix, hm.rmeta, hm.rgeo));
     return HB_OK;
 }
 
@@ -601,6 +602,12 @@ int launch_tick(hb_handle *h, int n, cudaStream_t st) {
 
 template <class A, int VARIANT, bool SEG>
 int launch_steps_t(hb_handle *h, hb::DevMesh<A> m, int n, cudaStream_t st) {
+    if constexpr (std::is_same<A, hb::F64Exact>::value && !SEG) {
+        if (hb_cells_used(h)) {
+            TRY(hb_cells_launch(h, m, 0, n, 1, false, st));
+            return launch_tick(h, n, st);
+        }
+    }
     // Programmatic dependent launch: each kernel may start while its predecessor
     // drains and waits in cudaGridDependencySynchronize for its results.
     cudaLaunchAttribute attr[1];
@@ -760,6 +767,7 @@ int hb_forward_step_into(hb_handle *h, long long t0, int k, const double *in, do
     m.S[par ^ 1] = out;
     m.slotw = terms;
     m.ucoef = coef;
+    if (hb_cells_used(h)) return hb_cells_launch(h, m, k, 1, write_flux, true, st);
     // programmatic dependent launch, as in the step sequence (launch_steps_t)
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -88,6 +88,8 @@ struct DevMesh {
                                // slot 4*a+j, and for a pair the slot of b (-1 otherwise)
     uint8_t *rmeta;            // code | own_first | has_nb of slot a (code changes on breach)
     const R *rgeo;             // [nrecords][4] {COSF, SINF, SIDE, 0} of slot a
+    const R *sgeo;             // [real slots][4] {COSF, SINF, SIDE, SlotRef::pack} (cell_kernel; else null)
+    const int4 *cseg;          // cell_kernel CTAs {first cell, cells, first slot record, slot records}
     R *f0, *f1, *f2, *f3;      // [4C] fluxes of the last step, index 4*cell + j
     const R *bqt, *bdqt;       // [ndays*nb]
     const L *bzt, *bdzt;       // [ndays*nb]
@@ -117,9 +119,11 @@ struct DevMesh {
 
 struct StepIndex { int par, kt, jt; long long step; };
 
-template <class A>
+// EARLY: read ahead of the dependency wait, so from L2 (a line that an earlier
+// launch left in L1 may be old).
+template <bool EARLY = false, class A>
 __device__ __forceinline__ StepIndex step_index(const DevMesh<A> &m, int k, int per_day, int ndays) {
-    const long long step = *m.step_ctr + k;
+    const long long step = (EARLY ? __ldcg(m.step_ctr) : *m.step_ctr) + k;
     StepIndex si;
     si.step = step;
     si.par = (int)(step & 1);
@@ -495,19 +499,41 @@ __global__ void __launch_bounds__(THREADS, MINB) flux_kernel(DevMesh<A> m, int k
 // (flux_slot's ZERO_LEN) unless fluxes are written out, and only where its
 // zero addends can change the sums.
 // SMEM_TERMS: `terms` is in shared memory (tile layout), else global.
-// update_core takes the cell's stored state record `raw` and bed `zbc`.
-template <class A, int VARIANT, bool COEF = false, bool SMEM_TERMS = false>
-__device__ __forceinline__ void update_core(const DevMesh<A> &m, int c, const Vec4<typename A::real> &raw,
-                                            typename A::level zbc, const StepIndex &si, const StepParams &p,
-                                            int write_flux, const typename A::real *terms) {
+// update_core takes the cell's state and constants `in`, and two functions
+// that give its DT/AREA and its friction: a caller that formed them while it
+// waited for the terms returns them, others compute them where they are used.
+template <class A>
+struct CellIn {
+    Vec4<typename A::real> raw;         // the stored state record
+    typename A::level zbc;
+    unsigned mask;
+    typename A::real fnc, dta, sidex;   // dta: DT/AREA (variant H) or AREA (variant F)
+};
+template <class A, int VARIANT>
+__device__ __forceinline__ CellIn<A> load_cell_in(const DevMesh<A> &m, int par, int c) {
+    using R = typename A::real;
+    CellIn<A> in;
+    in.raw = ldg4(m.S[par] + 4 * (size_t)c);
+    in.zbc = m.zbc[c];
+    in.mask = m.cmask[c];
+    in.fnc = m.fnc[c];
+    in.dta = m.dta[c];
+    in.sidex = VARIANT == 1 ? m.sidex[c] : R(0);
+    return in;
+}
+
+template <class A, int VARIANT, bool COEF, bool SMEM_TERMS, class DtaOf, class FrictionOf>
+__device__ __forceinline__ void update_core(const DevMesh<A> &m, int c, const CellIn<A> &cin, const StepIndex &si,
+                                            const StepParams &p, int write_flux, const typename A::real *terms,
+                                            const DtaOf &dta_of, const FrictionOf &friction_of) {
     using R = typename A::real;
     using L = typename A::level;
+    const Vec4<R> raw = cin.raw;
+    const unsigned mask = cin.mask;
     CellStateA<A> st;
-    st.h = raw.x; st.u = raw.y; st.v = raw.z; st.zbc = zbc;
+    st.h = raw.x; st.u = raw.y; st.v = raw.z; st.zbc = cin.zbc;
     if constexpr (is_split<A>::value) st.z = split_level<A>(raw.x, raw.w, st.zbc);
     else st.z = raw.w;
-    const unsigned mask = m.cmask[c];
-    const R fnc = m.fnc[c], dta = m.dta[c], sidex = VARIANT == 1 ? m.sidex[c] : R(0);
     // only the real slots' terms are read (a triangle's zero-length fourth
     // slot is evaluated below and has none)
     Vec4<R> t[4];
@@ -575,15 +601,14 @@ __device__ __forceinline__ void update_core(const DevMesh<A> &m, int c, const Ve
     CellUpdateIn<R, L> ci;
     ci.h = st.h; ci.u = st.u; ci.v = st.v; ci.zbc = st.zbc;
     ci.hlo = is_split<A>::value ? raw.w : R(0);
-    ci.fnc = fnc;
-    ci.dta_or_area = dta;
-    ci.sidex = sidex;
-    CellUpdateOut<R, L> o =
-        update_cell<A, VARIANT, COEF>(ci, wh, wu, wv, p, COEF ? m.ucoef + UPDATE_COEF * (size_t)c : nullptr);
+    ci.fnc = cin.fnc;
+    CellUpdateOut<R, L> o = update_cell<A, VARIANT, COEF>(ci, dta_of(), wh, wu, wv, p, friction_of,
+                                                          COEF ? m.ucoef + UPDATE_COEF * (size_t)c : nullptr);
     const int np = si.par ^ 1;
     if constexpr (is_split<A>::value) stg4(m.S[np] + 4 * (size_t)c, o.h, o.u, o.v, o.hlo);
     else stg4(m.S[np] + 4 * (size_t)c, o.h, o.u, o.v, o.z);
-    m.W[c] = o.w;
+    // W enters no step: only the last one of a sequence leaves it
+    if (write_flux) m.W[c] = speed<A>(o.u, o.v);
     if (!(isfinite((double)o.h) && isfinite((double)o.u) && isfinite((double)o.v))) atomicOr(m.err, ERRBIT_NONFINITE);
     if constexpr (std::is_same<A, F64Exact>::value) {
         if (m.ckpt != nullptr) {
@@ -602,8 +627,11 @@ __device__ __forceinline__ void update_core(const DevMesh<A> &m, int c, const Ve
 template <class A, int VARIANT, bool COEF = false, bool SMEM_TERMS = false>
 __device__ __forceinline__ void update_one(const DevMesh<A> &m, int c, const StepIndex &si, const StepParams &p,
                                            int write_flux, const typename A::real *terms) {
-    const Vec4<typename A::real> raw = ldg4(m.S[si.par] + 4 * (size_t)c);
-    update_core<A, VARIANT, COEF, SMEM_TERMS>(m, c, raw, m.zbc[c], si, p, write_flux, terms);
+    const CellIn<A> in = load_cell_in<A, VARIANT>(m, si.par, c);
+    update_core<A, VARIANT, COEF, SMEM_TERMS>(
+        m, c, in, si, p, write_flux, terms,
+        [&]() { return cell_dta<A, VARIANT>(in.raw.x, in.raw.y, in.dta, in.sidex, p); },
+        [&]() { return cell_friction<A>(in.raw.x, in.raw.y, in.raw.z, in.fnc, p); });
 }
 
 // Every cell of one step.  Single mesh: a grid-stride loop over the cells.
@@ -630,6 +658,127 @@ __global__ void __launch_bounds__(UPDATE_THREADS, UMINB) update_kernel(DevMesh<A
         const StepParams p{m.hm1, m.hm2, m.jl, m.dt, si.kt, si.jt};
         for (int c = blk * UPDATE_THREADS + threadIdx.x; c < m.C; c += gridDim.x * UPDATE_THREADS)
             update_one<A, VARIANT, COEF>(m, c, si, p, write_flux, m.slotw + 16 * (size_t)c);
+    }
+}
+
+// What a slot of cell_kernel needs besides its geometry, packed into the
+// fourth value of its sgeo record: the neighbour (device order), the slot's
+// place in its CTA, its code byte at creation, and its record, whose rmeta
+// holds the current code of a slot that may breach.
+struct SlotRef {
+    static constexpr int NO_NB = 0xFFFFFF, MAX_RECORD = 1 << 24;
+    int nb;                    // -1 = none
+    int place;                 // 4 * (cell - the CTA's first cell) + j
+    uint8_t meta;
+    int record;
+    static inline unsigned long long pack(int nb, int place, uint8_t meta, int record) {
+        return (unsigned long long)((unsigned)record << 8 | meta) << 32 |
+               ((unsigned)place << 24 | (unsigned)(nb < 0 ? NO_NB : nb));
+    }
+    static __device__ __forceinline__ SlotRef unpack(unsigned long long w) {
+        const unsigned lo = (unsigned)w, hi = (unsigned)(w >> 32);
+        const int nb = (int)(lo & 0xFFFFFFu);
+        return {nb == NO_NB ? -1 : nb, (int)(lo >> 24), (uint8_t)(hi & 0xFFu), (int)(hi >> 8)};
+    }
+};
+
+// One whole step in one launch for small fp64 meshes: a CTA takes a run of at
+// most 32 consecutive cells with at most CELL_SLOTS real slots.  One thread
+// per real slot computes that slot's flux from its own side (as the reference
+// does) into shared memory; meanwhile the last warp, one lane per cell, loads
+// its cells and forms what does not depend on the fluxes (friction, variant
+// F's time step); after a block barrier it sums the terms and updates the
+// cells.  Every edge is computed twice and nothing passes through device
+// memory between flux and update, so a step is one chain of latencies instead
+// of two; that pays while the chip is not full (hb_cells.cu has the line).
+// Same operations per slot and per cell, so the same bits as the two-kernel
+// step.  COEF as in update_kernel.
+//
+// Bound by that chain: of a 4.3 us step at 6,675 cells about 1.3 us is the
+// launch and the state's way through L2, the rest dependent fp64 operations.
+// What shortened it there: one launch 8.4 -> 5.1 us; the update warp's early
+// work and the step index read ahead of the wait 5.1 -> 4.3 us.  96 slots per
+// CTA are 32 triangles, one update warp; 7 CTAs per SM hold 32,000 cells at
+// once (5.0 us; 7.0 us at 6 per SM).
+constexpr int CELL_SLOTS = 96, CELL_MAX = 32, CELL_THREADS = CELL_SLOTS + CELL_MAX;
+constexpr int CELL_TERMS = 18;   // values per cell in shared memory: 4 slots x 4, padded off the bank period
+constexpr int CELL_CTAS = 7;     // CTAs per SM asked of the compiler
+template <class A, int VARIANT, bool COEF>
+__global__ void __launch_bounds__(CELL_THREADS, CELL_CTAS) cell_kernel(DevMesh<A> m, int k, int write_flux) {
+    using R = typename A::real;
+    using L = typename A::level;
+    __shared__ __align__(16) R terms[CELL_TERMS * CELL_MAX];
+    const int t = threadIdx.x;
+    const int4 d = m.cseg[blockIdx.x];   // {first cell, cells, first slot record, slot records}
+    // The step counter was last written before this sequence.  From the
+    // second step on it is read before the dependency wait: this kernel can
+    // only have been launched once every CTA of the step before had passed
+    // its own wait, so everything before that step is complete.
+    StepIndex si;
+    if (k > 0) si = step_index<true>(m, k, m.per_day, m.ndays);
+    if (t < CELL_SLOTS) {
+        // constant tables: read before the dependency wait (ZBC and FNC, which
+        // the adjoint's parameters change between sequences, from L2)
+        Vec4<R> g{R(0), R(0), R(0), R(0)};
+        SlotRef ref{-1, 0, 0, 0};
+        L zb = L(0), zbn = L(0);
+        if (t < d.w) {
+            g = ldg4(m.sgeo + 4 * (size_t)(d.z + t));
+            ref = SlotRef::unpack((unsigned long long)__double_as_longlong((double)g.w));
+            zb = __ldcg(m.zbc + d.x + (ref.place >> 2));
+            if (ref.nb >= 0) zbn = __ldcg(m.zbc + ref.nb);
+        }
+        cudaGridDependencySynchronize();
+        cudaTriggerProgrammaticLaunchCompletion();
+        if (k == 0) si = step_index(m, k, m.per_day, m.ndays);
+        if (t < d.w) {
+            const StepParams p{m.hm1, m.hm2, m.jl, m.dt, si.kt, si.jt};
+            const R *S = m.S[si.par];
+            const int c = d.x + (ref.place >> 2), sa = 4 * d.x + ref.place;
+            const Vec4<R> a = ldg4(S + 4 * (size_t)c);
+            CellStateA<A> nb{R(0), R(0), R(0), L(0), L(0)};
+            if (ref.nb >= 0) {
+                const Vec4<R> b = ldg4(S + 4 * (size_t)ref.nb);
+                nb = {b.x, b.y, b.z, b.w, zbn};
+            }
+            uint8_t meta = ref.meta;
+            if ((meta & META_CODE) == CODE_K7) meta = m.rmeta[ref.record];   // breached since?
+            const Terms<R, true> tout{terms + CELL_TERMS * (ref.place >> 2) + 4 * (ref.place & 3), sa};
+            single_core<A, VARIANT>(m, ref.record, c, sa, CellStateA<A>{a.x, a.y, a.z, a.w, zb}, nb, meta, g, si, p,
+                                    write_flux, tout);
+        }
+        __syncthreads();
+    } else {
+        const int i = t - CELL_SLOTS, c = d.x + i;
+        const bool on = i < d.y;
+        CellIn<A> in{};
+        if (on) {
+            in.zbc = __ldcg(m.zbc + c);
+            in.mask = m.cmask[c];
+            in.fnc = __ldcg(m.fnc + c);
+            in.dta = m.dta[c];
+            in.sidex = VARIANT == 1 ? m.sidex[c] : R(0);
+        }
+        cudaGridDependencySynchronize();
+        cudaTriggerProgrammaticLaunchCompletion();
+        if (k == 0) si = step_index(m, k, m.per_day, m.ndays);
+        const StepParams p{m.hm1, m.hm2, m.jl, m.dt, si.kt, si.jt};
+        // a cell that is shallow now rarely needs its friction: it is formed late if it does
+        Friction<R> f{R(0), R(0), R(0)};
+        R dta = R(0);
+        auto friction = [&]() { return cell_friction<A>(in.raw.x, in.raw.y, in.raw.z, in.fnc, p); };
+        bool ready = false;
+        if (on) {
+            in.raw = ldg4(m.S[si.par] + 4 * (size_t)c);
+            dta = cell_dta<A, VARIANT>(in.raw.x, in.raw.y, in.dta, in.sidex, p);
+            ready = in.raw.x > A::c(p.hm2);
+            if (ready) f = friction();
+        }
+        __syncthreads();
+        if (on)
+            update_core<A, VARIANT, COEF, true>(m, c, in, si, p, write_flux, terms + CELL_TERMS * i,
+                                                [&]() { return dta; },
+                                                [&]() { return ready ? f : friction(); });
     }
 }
 
