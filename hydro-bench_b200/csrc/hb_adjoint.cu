@@ -20,15 +20,16 @@
 // pass recomputes each k-step segment from its checkpoint, keeping that
 // segment's states and the update coefficients of its steps (written by
 // the recomputed update kernels), then runs the segment's reverse steps, one
-// kernel each (adj_step_kernel, four lanes per cell):
+// kernel each (adj_step_kernel, one thread per slot and one per cell):
+//   - every slot's flux linearised at the state before the step;
 //   - the state adjoint after the step, gathered from the later step's
 //     direct terms, the cell's own slots' contributions and those of the
-//     neighbours' slots that face it (fixed order, no atomics: the gradient
-//     is deterministic);
-//   - lane 0: the cell update's reverse (from the stored coefficients),
-//     shared with the other lanes;
-//   - lane j: slot j's flux reverse, leaving its contributions to its own
-//     cell and its neighbour for the next (earlier) step.
+//     neighbours' slots that face it (fixed order: the gradient is
+//     deterministic);
+//   - the cell update's reverse (from the stored coefficients);
+//   - every slot's linearisation applied to its cell's adjoint, leaving its
+//     contributions to its own cell and its neighbour for the next (earlier)
+//     step.
 // The forward rollout is replayed from a CUDA graph of k steps whose
 // checkpoint and gauge kernels take their slot from the device step counter.
 #include <cmath>
@@ -461,17 +462,34 @@ __device__ void slot_rev(const SlotInA<A> &in, const StepParams &p, const TableF
     }
 }
 
-// Adjoint-side mesh: per device slot its geometry, neighbour, code and the
-// neighbour's slot that faces back.
+// Adjoint-side mesh.  The reverse step's CTAs take runs of at most
+// ADJ_CELLS consecutive cells with at most ADJ_SLOTS real slots (seg); sgeo
+// holds the real slots' {COSF, SINF, SIDE, AdjSlot::pack} in that order.
 struct AdjMesh {
-    const double *cs4, *sn4, *side4;
-    const int32_t *nbr4, *mirror4;
-    const uint8_t *meta4;        // code | own_first | has_nb; 0xFF = no real slot
+    const double *sgeo;          // [real slots][4]
+    const int4 *seg;             // {first cell, cells, first slot record, slot records} per CTA
+    const int32_t *mirror4;      // [4C] the neighbour's slot that faces the slot, -1 = none
     const int32_t *gauge_of;     // [C] gauge index of the cell, -1
     double *fnc_g, *zbc_g;       // [C] accumulated gradients
     double *lam;                 // [C][4] state adjoint {H, U, V, Z} (the seed, and at the end that of x_0)
     const double *res;           // [nobs][ng] residuals H - Hobs
-    int ng, obs_every;
+    int ng, obs_every, nseg;
+};
+constexpr int ADJ_SLOTS = 96, ADJ_CELLS = 32, ADJ_THREADS = ADJ_SLOTS + ADJ_CELLS;
+
+// The fourth value of a slot's record: neighbour (-1 = none), place in the
+// CTA (4 * (cell - first cell) + j), code byte.
+struct AdjSlot {
+    int nb, place;
+    uint8_t meta;
+    static inline unsigned long long pack(int nb, int place, uint8_t meta) {
+        return (unsigned long long)((unsigned)place << 8 | meta) << 32 | (unsigned)nb;
+    }
+    static __device__ __forceinline__ AdjSlot unpack(double d) {
+        const unsigned long long w = (unsigned long long)__double_as_longlong(d);
+        const unsigned hi = (unsigned)(w >> 32);
+        return {(int)(unsigned)w, (int)(hi >> 8), (uint8_t)(hi & 0xFFu)};
+    }
 };
 
 // What one reverse step leaves for the next (earlier) one: per cell the
@@ -514,17 +532,251 @@ __device__ __forceinline__ void gather4(const AdjMesh &a, const double *dir, con
 // The update coefficients of a step (update_cell with COEF, written by the
 // recomputed step's update kernel) for the reverse of the cell update.
 struct UpdateCoef { double dtw, ih2, d_fnc, d_h, d_s; };
-__device__ __forceinline__ UpdateCoef ld_coef(const double *p) {
-    const Vec4<double> a = ldg4(p), b = ldg4(p + 4);
-    return {a.x, a.y, a.z, a.w, b.x};
+
+// The boundary tables of cell c at interval jt.
+__device__ __forceinline__ BoundaryInA<A> boundary_of(const DevMesh<A> &m, int c, int jt) {
+    BoundaryInA<A> bi;
+    const int row = m.bcell[c];
+    if (row >= 0) {
+        const size_t q = (size_t)jt * m.nb + row;
+        bi.qt = m.bqt[q]; bi.dqt = m.bdqt[q]; bi.zt = m.bzt[q]; bi.dzt = m.bdzt[q];
+        bi.top = m.btop[row]; bi.nhq1 = m.bnhq1[row];
+        bi.zw = m.bzw + (size_t)row * m.nhq; bi.qw = m.bqw + (size_t)row * m.nhq;
+    } else {
+        bi.qt = bi.dqt = 0.0; bi.zt = bi.dzt = bi.top = 0.0; bi.nhq1 = 0;
+        bi.zw = m.bzw + (size_t)m.nb * m.nhq; bi.qw = m.bqw + (size_t)m.nb * m.nhq;
+    }
+    bi.nhq = m.nhq;
+    return bi;
 }
 
-// One reverse step t, four lanes per cell.  x: the state before the step; xn:
-// the state after it.  The adjoint of the state after the step is gathered
-// first from step t + 1's contributions (`first`: it is the seed a.lam
-// instead), with the loss term of row `obs_row` when step t + 1 ends on an
-// observation.  Lane 0 reverses the cell update and shares the adjoints of the
-// slot sums; lane j then reverses slot j.
+// A state record through L2 (it may be read ahead of the dependency wait, and
+// a line that an earlier launch left in L1 may be old).
+__device__ __forceinline__ Vec4<double> ldcg4(const double *p) {
+    const double2 a = __ldcg(reinterpret_cast<const double2 *>(p)), b = __ldcg(reinterpret_cast<const double2 *>(p) + 1);
+    return {a.x, a.y, b.x, b.y};
+}
+
+// A slot whose linearisation is not held in registers (LIN_GENERAL): reversed
+// from the state by slot_rev, its contributions stored.  Kept out of line so
+// that its register need stays out of the common path.
+__device__ __noinline__ void general_slot(const DevMesh<A> &m, const double *x, const double *g, int c, const StepParams &p,
+                                          double fb0, double fb1, double fb2, double *so, double *sno) {
+    const AdjSlot ref = AdjSlot::unpack(g[3]);
+    const Vec4<double> a = ldg4(x + 4 * (size_t)c);
+    SlotInA<A> in;
+    in.own = CellStateA<A>{a.x, a.y, a.z, a.w, m.zbc[c]};
+    in.nb = CellStateA<A>{0, 0, 0, 0, 0};
+    in.has_nb = ref.nb >= 0;
+    if (in.has_nb) {
+        const Vec4<double> b = ldg4(x + 4 * (size_t)ref.nb);
+        in.nb = CellStateA<A>{b.x, b.y, b.z, b.w, m.zbc[ref.nb]};
+    }
+    in.code = (int8_t)(ref.meta & META_CODE);
+    in.own_first = ref.meta & META_OWN_FIRST;
+    in.cosj = g[0]; in.sinj = g[1]; in.side = g[2];
+    const double fb[4] = {fb0, fb1, fb2, fb1};
+    Adj5 go{0, 0, 0, 0, 0}, gn{0, 0, 0, 0, 0};
+    slot_rev(in, p, [&]() { return boundary_of(m, c, p.jt); }, fb, go, gn, m.err);
+    st_rec(so, go);
+    st_rec(sno, gn);
+}
+
+// The linearisation of one slot's fluxes at the state before the step: all of
+// the reverse that does not depend on the adjoint, so that it can be formed
+// ahead of it.  The slot sums use F1 and F3 only as F1 + F3, so a slot has
+// three adjoint inputs fb0, fb1 (= that of F3) and fb2.
+//   LIN_OSHER: subcritical flow across the edge, Osher's case with one piece,
+//     3 or 5 (k1 = 1, k2 = 2 or 3): fo = (ha ua, ha ua^2, ha ua vt,
+//     4.905 ha^2) with ua = (FIL + FIR) / 2, ha = d^2 / 39.24,
+//     d = (FIL - FIR) / 2 and vt the tangent of the upstream side; both
+//     pieces have the same derivative (osher_rev);
+//   LIN_EDGE: boundary slots (KLAS 1, 4, 10): nine coefficients of the own
+//     cell's adjoints; the fixed points' derivatives are carried forward
+//     along the iterations instead of being reversed through stored iterates;
+//   LIN_ZERO: both cells dry, no contribution;
+//   LIN_GENERAL: everything else (general_slot).
+enum : int { LIN_ZERO = 0, LIN_OSHER = 1, LIN_EDGE = 2, LIN_GENERAL = 3 };
+struct SlotLin {
+    int kind;
+    bool mir, p3, thin, deep, zside, wet;   // LIN_OSHER: route, piece, qr1 clamped, qr0 > HM1, Z_R > ZBC_R, H_R > HM1
+    double c[11];
+};
+
+__device__ __forceinline__ void linearise_osher(const CellStateA<A> &L, const CellStateA<A> &R, double cs, double sn,
+                                                bool mir, const StepParams &p, SlotLin &s) {
+    s.kind = LIN_GENERAL;
+    const double clL = A::sqrt(A::mul(A::c(9.81), L.h));
+    const OsherIn<double> oi = osher_inputs<A>(L, R, cs, sn, clL, mir, p);
+    const double cr = A::sqrt(A::mul(A::c(9.81), oi.qr[0]));
+    const double fir = A::sub(oi.qr[1], A::mul(A::c(2.0), cr));
+    const double ua = A::mul(A::add(oi.fil, fir), A::c(0.5));
+    const double ca = A::fabs(A::mul(A::sub(oi.fil, fir), A::c(0.25)));
+    if (!(oi.ql[1] < clL && oi.qr[1] >= -cr && ua >= -ca && ua < ca)) return;
+    s.kind = LIN_OSHER;
+    s.mir = mir;
+    s.p3 = ua >= 0.0;
+    s.thin = oi.hcR <= p.hm2 || oi.qr[0] <= p.hm2;
+    const double zR = A::lmax(R.zbc, R.z);
+    s.deep = A::depth(zR, L.zbc) > p.hm1;
+    s.zside = R.z > R.zbc;
+    s.wet = R.h > p.hm1;
+    const double d = oi.fil - ua, ha = d * d * (1.0 / 39.24);
+    const double q = oi.hcR / oi.qr[0];
+    s.c[0] = ua;
+    s.c[1] = ha;
+    s.c[2] = s.p3 ? oi.ql[2] : oi.qr[2];
+    s.c[3] = d * (2.0 / 39.24);
+    s.c[4] = 9.81 / clL;
+    s.c[5] = 9.81 / cr;
+    s.c[6] = oi.ur;
+    s.c[7] = oi.hcR;
+    s.c[8] = oi.ratio;
+    s.c[9] = q < 1.5 ? 1.0 / oi.qr[0] : 0.0;          // d ratio / d hcR
+    // mirrored: FLUX3 = 4.905 hc3^2, hc3 = sqrt(fo3 / 4.905) + ZBC_L - ZBC_R = ha + ... where positive
+    s.c[10] = fmax(ha + L.zbc - R.zbc, 0.0);
+}
+
+// go, gn from the slot's adjoint inputs (LIN_OSHER); osher_route_rev's steps
+__device__ __forceinline__ void apply_osher(const SlotLin &s, double cs, double sn, double fb0, double fb1, double fb2,
+                                            Adj5 &go, Adj5 &gn) {
+    const double ua = s.c[0], ha = s.c[1], vt = s.c[2], ur = s.c[6], hcR = s.c[7], ratio = s.c[8], iq = s.c[9];
+    if (s.mir) { cs = -cs; sn = -sn; }
+    const double f0 = s.mir ? -fb0 : fb0;
+    const double hc3b = s.mir ? fb1 * 9.81 * s.c[10] : 0.0;
+    const double hab = ua * (f0 + fb1 * ua + fb2 * vt) + (s.mir ? hc3b : fb1 * 9.81 * ha);
+    const double uab = ha * (f0 + 2.0 * fb1 * ua + fb2 * vt);
+    const double vtb = fb2 * ha * ua;
+    const double db = hab * s.c[3];
+    const double filb = 0.5 * (uab + db), firb = 0.5 * (uab - db);
+    const double t = fb1 * 0.5 * ur;
+    double ratiob = -t * hcR * ur, hcRb = t * (1.0 - ratio) * ur, urb = 2.0 * t * (1.0 - ratio) * hcR;
+    if (!s.thin) { urb += firb * ratio; ratiob += firb * ur; }
+    hcRb += ratiob * iq;
+    const double qr0b = -firb * s.c[5] - ratiob * iq * iq * hcR;
+    const double ql2b = s.p3 ? vtb : 0.0, qr2b = s.p3 ? 0.0 : vtb;
+    Adj5 l{filb * s.c[4], filb * cs - ql2b * sn, filb * sn + ql2b * cs, 0.0, hc3b};
+    Adj5 r{s.wet ? hcRb : 0.0, urb * cs - qr2b * sn, urb * sn + qr2b * cs, 0.0, -hc3b};
+    if (s.deep) {
+        if (s.zside) r.z = qr0b;
+        else r.b += qr0b;
+        l.b -= qr0b;
+    }
+    go = s.mir ? r : l;
+    gn = s.mir ? l : r;
+}
+
+// Boundary slots: the own cell's adjoints {h, ql1, ql2, b} per unit of fb0,
+// fb1 and fb2 (functors.cu:204-232, :371-392, :513-568).
+__device__ __forceinline__ void linearise_edge(const SlotInA<A> &in, double ql1, double ql2, double cl,
+                                               const BoundaryInA<A> &b, const StepParams &p, SlotLin &s) {
+    const double h = in.own.h;
+    for (int i = 0; i < 9; i++) s.c[i] = 0.0;
+    double *H = s.c, *Q = s.c + 3;            // fb0, fb1 (F1 and F3), fb2 -> h; -> ql1
+    double &T = s.c[6], *B = s.c + 7;         // fb2 -> ql2; fb0, fb1 -> b
+    s.kind = LIN_EDGE;
+    if (ql1 > cl && h < p.hm2) {              // supercritical (variant H, functors.cu:517)
+        H[0] = ql1; H[1] = ql1 * ql1 + 9.81 * h; H[2] = ql1 * ql2;
+        Q[0] = h; Q[1] = 2.0 * h * ql1; Q[2] = h * ql2;
+        T = h * ql1;
+        return;
+    }
+    if (in.code == CODE_K4) {
+        H[1] = 9.81 * h;
+    } else if (in.code == CODE_K10) {
+        double f0 = -A::madd(b.dqt, A::c((double)p.kt), b.qt, M_K10);
+        f0 = A::div(f0, in.side);
+        const double fil = A::add(ql1, A::mul(A::c(2.0), cl));
+        // inflow_depth with d hb / d FIL (tf) and d hb / d H (th) carried along
+        double hb0 = h, hb = 0.0, tf0 = 0.0, th0 = 1.0, tf = 0.0, th = 0.0;
+        for (int k = 1; k <= 20; k++) {
+            const double r = A::div(f0, hb0);
+            const double w = A::sub(fil, r);
+            hb = A::divk(A::mul(w, w), 39.24);
+            const double w2 = w * (2.0 / 39.24), e = w2 * r / hb0;
+            tf = w2 + e * tf0;
+            th = e * th0;
+            if (A::fabs(A::sub(hb0, hb)) <= A::c(0.005)) break;
+            hb0 = A::add(A::mul(hb0, A::c(0.5)), A::mul(hb, A::c(0.5)));
+            tf0 = 0.5 * (tf0 + tf);
+            th0 = 0.5 * (th0 + th);
+        }
+        const double k1 = 9.81 * hb - (hb <= 1.0 ? 0.0 : f0 * f0 / (hb * hb));   // d(F1 + F3) / d hb
+        H[1] = k1 * (th + tf * 9.81 / cl);
+        Q[1] = k1 * tf;
+    } else {                                  // KLAS 1
+        const double lev = A::lmadd(b.dzt, A::lc((double)p.jt), b.zt, M_K1);
+        const double d = A::lsub(lev, in.own.zbc);
+        const double hb1 = A::fmax(d, A::c(p.hm2));
+        const double sh = A::sqrt(h), shb = A::sqrt(hb1), ihb = 1.0 / hb1, dsh = 0.5 * ihb * shb;
+        const double fial = A::madd(A::c(6.264), sh, ql1, M_FIAL1);
+        // invariant_iter with d urb / d ql1 (tq, FIAL included), / d FIAL (tl) and / d hb1 (tb) carried along
+        double ur0 = ql1, urb = ql1, tq = 1.0, tl = 0.0, tb = 0.0;
+        for (int k = 1; k <= 30; k++) {
+            const double fiar = A::madd(A::c(-6.264), shb, urb, M_FIAR1);
+            const double dsum = A::add(fial, fiar), ddif = A::sub(fial, fiar);
+            urb = A::divk(A::div(A::mul(A::mul(dsum, ddif), ddif), hb1), 313.92);
+            const double sc = ihb * (1.0 / 313.92), es = ddif * ddif * sc, ed = 2.0 * dsum * ddif * sc;
+            const double el = es + ed, er = es - ed;   // per FIAL, per FIAR
+            tl = el + er * tl;
+            tq = er * tq;
+            tb = er * (tb - 6.264 * dsh) - urb * ihb;
+            if (A::fabs(A::sub(urb, ur0)) <= A::c(0.0001)) break;
+            ur0 = urb;
+        }
+        const double u0 = hb1, u1 = 2.0 * hb1 * urb;             // d F0, d F1 per urb
+        const double h0 = urb, h1 = urb * urb + 9.81 * hb1;      // d F0, d(F1 + F3) per hb1
+        const double dh = tl * 6.264 * 0.5 / sh, dq = tq + tl;
+        H[0] = u0 * dh; H[1] = u1 * dh;
+        Q[0] = u0 * dq; Q[1] = u1 * dq;
+        if (d > p.hm2) { B[0] = -(h0 + u0 * tb); B[1] = -(h1 + u1 * tb); }
+        if (ql1 > 0.0) {                      // FLUX2 = h ql1 ql2
+            H[2] = ql1 * ql2;
+            Q[2] = h * ql2;
+            T = h * ql1;
+        }
+    }
+}
+
+// slot_rev's choice of branch at the state before the step, and the slot's
+// linearisation where it has one of its own.
+__device__ __forceinline__ void linearise_slot(const SlotInA<A> &in, const DevMesh<A> &m, int c, const StepParams &p,
+                                               SlotLin &s) {
+    const double h1 = in.own.h, b1 = in.own.zbc;
+    if (code_is_bounda(in.code)) {
+        const double ql1 = A::dot(in.own.u, in.cosj, in.own.v, in.sinj, M_QL1);
+        const double ql2 = A::dot(in.own.v, in.cosj, -in.own.u, in.sinj, M_QL2);
+        linearise_edge(in, ql1, ql2, A::sqrt(A::mul(A::c(9.81), h1)), boundary_of(m, c, p.jt), p, s);
+        return;
+    }
+    const double zi = A::lmax(in.own.z, A::ladd(b1, A::lc(p.hm1)));
+    double hc = 0, bc = 0, zc = 0;
+    if (in.has_nb) {
+        hc = A::fmax(in.nb.h, A::c(p.hm1));
+        bc = in.nb.zbc;
+        zc = A::lmax(bc, in.nb.z);
+    }
+    s.kind = h1 <= p.hm1 && hc <= p.hm1 ? LIN_ZERO : LIN_GENERAL;
+    if (s.kind == LIN_ZERO || zi <= bc || zc <= b1 || h1 <= p.hm2 || hc <= p.hm2 || !in.has_nb || in.code != CODE_ZERO)
+        return;
+    const bool mir = !in.own_first;
+    linearise_osher(mir ? in.nb : in.own, mir ? in.own : in.nb, mir ? -in.cosj : in.cosj, mir ? -in.sinj : in.sinj, mir,
+                    p, s);
+}
+
+// One reverse step t.  x: the state before the step; xn: the state after it.
+// The adjoint of the state after the step is gathered first from step t + 1's
+// contributions (`first`: it is the seed a.lam instead), with the loss term of
+// row `obs_row` when step t + 1 ends on an observation.
+//
+// A CTA takes a run of cells: one thread per real slot, and a last warp with
+// one lane per cell.  Ahead of the dependency wait the slot threads linearise
+// their fluxes at x (which the recomputation finished before this segment's
+// first reverse step began) and the cell lanes load their update coefficients.
+// After it the slot threads copy the contributions into shared memory
+// (cp.async), the cell lanes sum them and reverse the cell update, and the
+// slot threads apply their linearisation.  So the chain from step to step is
+// the copy, the sums and about forty multiply-adds.
 //
 // coef: the step's update coefficients (written with the recomputed step).
 //
@@ -534,116 +786,177 @@ __device__ __forceinline__ UpdateCoef ld_coef(const double *p) {
 // |U2| < 15, the only case in which its adjoint passes (at the clamp, xn holds
 // +-15 and the adjoint is cut).
 //
-// Seven CTAs per SM (72 registers, some spilled to L1): the kernel waits on
-// L2 gathers, and more resident warps hide them better than fewer spills do.
-__global__ void __launch_bounds__(128, 7) adj_step_kernel(DevMesh<A> m, AdjMesh a, AdjStepBufs b,
-                                                          const double *__restrict__ x, const double *__restrict__ xn,
-                                                          const double *__restrict__ coef, StepParams p, int first,
-                                                          int obs_row) {
-    // launched with programmatic dependent launch: wait for the previous kernel's results
-    cudaGridDependencySynchronize();
-    cudaTriggerProgrammaticLaunchCompletion();
-    const int gid = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = (gid >> 2) < m.C;
-    const int c = valid ? gid >> 2 : m.C - 1, j = gid & 3;
-    const int lane0 = (int)(threadIdx.x & 31) & ~3;
-    double l[4], zg = 0.0;
-    if (first) {
-        for (int q = 0; q < 4; q++) l[q] = a.lam[4 * (size_t)c + q];
+// Bound by that chain and, at 24,020 cells (751 CTAs, one wave at 6 CTAs per
+// SM), by the linearisation in front of it: 7.2 us per reverse step there and
+// 4.0 us at 6,000 cells.  Four lanes per cell, everything after the wait and
+// the general reverse of every slot (1,376 instructions per warp, 464 bytes of
+// spill loads) took 16-18 us.  5 CTAs per SM: 13.8 against 11.9 us per step of
+// the backward pass, recomputation included; 7 and 8: 12.3 and 12.9 us.
+constexpr int ADJ_CTAS = 6;
+constexpr int REC_CELL = 4 * 2 * ADJ_REC + 2;   // doubles per cell in shared memory, padded off the bank period
+__device__ __forceinline__ void copy16(double *smem, const double *g) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(g) : "memory");
+}
+__global__ void __launch_bounds__(ADJ_THREADS, ADJ_CTAS) adj_step_kernel(const __grid_constant__ DevMesh<A> m, AdjMesh a,
+                                                                   AdjStepBufs b, const double *__restrict__ x,
+                                                                   const double *__restrict__ xn,
+                                                                   const double *__restrict__ coef,
+                                                                   const __grid_constant__ StepParams p, int first,
+                                                                   int obs_row) {
+    __shared__ __align__(16) double rec[REC_CELL * ADJ_CELLS];
+    __shared__ double wb[ADJ_CELLS][3];
+    const int t = threadIdx.x;
+    const int4 d = a.seg[blockIdx.x];
+    if (t < ADJ_SLOTS) {
+        SlotLin lin;
+        lin.kind = LIN_ZERO;
+        double cs = 0.0, sn = 0.0, side = 0.0;
+        int place = 0, mj = -1;
+        const bool on = t < d.w;
+        if (on) {
+            const Vec4<double> g = ldg4(a.sgeo + 4 * (size_t)(d.z + t));
+            const AdjSlot ref = AdjSlot::unpack(g.w);
+            cs = g.x; sn = g.y; side = g.z;
+            place = ref.place;
+            mj = a.mirror4[4 * (size_t)d.x + place];
+            const int c = d.x + (place >> 2);
+            const Vec4<double> o = ldcg4(x + 4 * (size_t)c);
+            SlotInA<A> in;
+            in.own = CellStateA<A>{o.x, o.y, o.z, o.w, __ldcg(m.zbc + c)};
+            in.nb = CellStateA<A>{0, 0, 0, 0, 0};
+            in.has_nb = ref.nb >= 0;
+            if (in.has_nb) {
+                const Vec4<double> q = ldcg4(x + 4 * (size_t)ref.nb);
+                in.nb = CellStateA<A>{q.x, q.y, q.z, q.w, __ldcg(m.zbc + ref.nb)};
+            }
+            in.code = (int8_t)(ref.meta & META_CODE);
+            in.own_first = ref.meta & META_OWN_FIRST;
+            in.cosj = cs; in.sinj = sn; in.side = side;
+            linearise_slot(in, m, c, p, lin);
+        }
+        cudaGridDependencySynchronize();
+        cudaTriggerProgrammaticLaunchCompletion();
+        const size_t s = 4 * (size_t)d.x + place;
+        if (on && !first) {
+            double *r = rec + REC_CELL * (place >> 2) + 2 * ADJ_REC * (place & 3);
+            const double *so = b.so_in + ADJ_REC * s, *sf = b.sn_in + ADJ_REC * (size_t)max(mj, 0);
+#pragma unroll
+            for (int q = 0; q < ADJ_REC; q += 2) {
+                copy16(r + q, so + q);
+                if (mj >= 0) copy16(r + ADJ_REC + q, sf + q);
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            if (mj < 0)
+                for (int q = 0; q < 5; q++) r[ADJ_REC + q] = 0.0;
+        }
+        __syncthreads();
+        __syncthreads();   // wb is complete
+        if (on) {
+            const double whb = wb[place >> 2][0], wub = wb[place >> 2][1], wvb = wb[place >> 2][2];
+            const double slcos = side * cs, slsin = side * sn;
+            const double fb0 = side * whb, fb1 = slcos * wub + slsin * wvb, fb2 = slcos * wvb - slsin * wub;
+            double *so = b.so_out + ADJ_REC * s, *sno = b.sn_out + ADJ_REC * s;
+            if (lin.kind == LIN_GENERAL) {
+                general_slot(m, x, a.sgeo + 4 * (size_t)(d.z + t), d.x + (place >> 2), p, fb0, fb1, fb2, so, sno);
+            } else {
+                Adj5 go{0, 0, 0, 0, 0}, gn{0, 0, 0, 0, 0};
+                if (lin.kind == LIN_OSHER) {
+                    apply_osher(lin, cs, sn, fb0, fb1, fb2, go, gn);
+                } else if (lin.kind == LIN_EDGE) {
+                    const double ql1b = fb0 * lin.c[3] + fb1 * lin.c[4] + fb2 * lin.c[5], ql2b = fb2 * lin.c[6];
+                    go.h = fb0 * lin.c[0] + fb1 * lin.c[1] + fb2 * lin.c[2];
+                    go.u = ql1b * cs - ql2b * sn;
+                    go.v = ql1b * sn + ql2b * cs;
+                    go.b = fb0 * lin.c[7] + fb1 * lin.c[8];
+                }
+                st_rec(so, go);
+                st_rec(sno, gn);
+            }
+        }
     } else {
-        gather4(a, b.dir_in, b.so_in, b.sn_in, c, j, obs_row, l, zg);
-    }
-    const Vec4<double> xc = ldg4(x + 4 * (size_t)c);
-    const double hv = xc.x, uv = xc.y, vv = xc.z;
-    const double zbc = m.zbc[c];
-    double whb = 0.0, wub = 0.0, wvb = 0.0;
-    if (j == 0) {
-        // ---- the update (UpdateCellKernel, functors.cu:717-784, variant H): forward values, then its reverse
-        const double HM1 = p.hm1, HM2 = p.hm2;
-        const double dta = m.dta[c];
-        const Vec4<double> xn4 = ldg4(xn + 4 * (size_t)c);
-        const double h2 = xn4.x, u2 = xn4.y, v2 = xn4.z;
-        double h2b = l[0] + l[3];   // Z2 = H2 + ZBC
-        double hb = 0.0, ub = 0.0, vb = 0.0, fncb = 0.0;
-        if (h2 > HM2) {
-            const UpdateCoef k = ld_coef(coef + UPDATE_COEF * (size_t)c);
-            const double ue = fabs(u2) < 15.0 ? l[1] : 0.0;
-            const double ve = fabs(v2) < 15.0 ? l[2] : 0.0;
-            const double nub = ue * k.ih2, nvb = ve * k.ih2;
-            h2b -= (ue * u2 + ve * v2) * k.ih2;
-            hb += nub * uv + nvb * vv;
-            ub += nub * (hv - k.dtw);
-            vb += nvb * (hv - k.dtw);
-            wub -= nub * dta;
-            wvb -= nvb * dta;
-            const double dtwb = -(nub * uv + nvb * vv);
-            fncb += dtwb * k.d_fnc;
-            hb += dtwb * k.d_h;
-            ub += dtwb * k.d_s * uv;
-            vb += dtwb * k.d_s * vv;
-        } else if (h2 > HM1) {
-            if (fabs(uv) < K::VMIN) ub += l[1];
-            if (fabs(vv) < K::VMIN) vb += l[2];
+        const int i = t - ADJ_SLOTS, c = d.x + i;
+        const bool on = i < d.y;
+        Vec4<double> xc{0, 0, 0, 0}, x2{0, 0, 0, 0};
+        UpdateCoef k{0, 0, 0, 0, 0};
+        double dta = 0.0;
+        unsigned mask = 0;
+        int gauge = -1;
+        if (on) {
+            xc = ldcg4(x + 4 * (size_t)c);
+            x2 = ldcg4(xn + 4 * (size_t)c);
+            if (x2.x > p.hm2) {
+                const Vec4<double> q = ldcg4(coef + UPDATE_COEF * (size_t)c);
+                k = {q.x, q.y, q.z, q.w, __ldcg(coef + UPDATE_COEF * (size_t)c + 4)};
+            }
+            dta = m.dta[c];
+            mask = m.cmask[c];
+            if (obs_row >= 0) gauge = a.gauge_of[c];
         }
-        if (h2 > HM1) { hb += h2b; whb -= h2b * dta; }
-        if (valid) {
+        cudaGridDependencySynchronize();
+        cudaTriggerProgrammaticLaunchCompletion();
+        Vec4<double> l{0, 0, 0, 0};
+        double res = 0.0;
+        if (on) {
+            l = ldg4((first ? a.lam : b.dir_in) + 4 * (size_t)c);
+            if (!first && gauge >= 0) res = 2.0 * a.res[(size_t)obs_row * a.ng + gauge];
+        }
+        __syncthreads();
+        double zg = 0.0, hb = 0.0, ub = 0.0, vb = 0.0, fncb = 0.0, whb = 0.0, wub = 0.0, wvb = 0.0;
+        if (on) {
+            if (!first) {
+                // per slot (own + facing), slots 0 and 1, 2 and 3, then the two sums
+                double part[4][5];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    if (mask & (1u << j)) {
+                        double f[5];
+                        ld_rec(rec + REC_CELL * i + 2 * ADJ_REC * j, part[j]);
+                        ld_rec(rec + REC_CELL * i + 2 * ADJ_REC * j + ADJ_REC, f);
+#pragma unroll
+                        for (int q = 0; q < 5; q++) part[j][q] += f[q];
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 5; q++) part[j][q] = 0.0;
+                    }
+                }
+                double sum[5];
+#pragma unroll
+                for (int q = 0; q < 5; q++) sum[q] = (part[0][q] + part[1][q]) + (part[2][q] + part[3][q]);
+                l.x += sum[0]; l.y += sum[1]; l.z += sum[2]; l.w += sum[3];
+                zg = sum[4];
+                l.x += res;
+            }
+            // the update (UpdateCellKernel, functors.cu:717-784, variant H), reversed
+            double h2b = l.x + l.w;   // Z2 = H2 + ZBC
+            const double u = xc.y, v = xc.z, h2 = x2.x, u2 = x2.y, v2 = x2.z;
+            if (h2 > p.hm2) {
+                const double ue = fabs(u2) < 15.0 ? l.y : 0.0;
+                const double ve = fabs(v2) < 15.0 ? l.z : 0.0;
+                const double nub = ue * k.ih2, nvb = ve * k.ih2;
+                h2b -= (ue * u2 + ve * v2) * k.ih2;
+                const double dtwb = -(nub * u + nvb * v);
+                hb = dtwb * k.d_h - dtwb;
+                ub = nub * (xc.x - k.dtw) + dtwb * k.d_s * u;
+                vb = nvb * (xc.x - k.dtw) + dtwb * k.d_s * v;
+                wub = -nub * dta;
+                wvb = -nvb * dta;
+                fncb = dtwb * k.d_fnc;
+            } else if (h2 > p.hm1) {
+                if (fabs(u) < K::VMIN) ub = l.y;
+                if (fabs(v) < K::VMIN) vb = l.z;
+            }
+            if (h2 > p.hm1) { hb += h2b; whb = -h2b * dta; }
+            wb[i][0] = whb; wb[i][1] = wub; wb[i][2] = wvb;
+        }
+        __syncthreads();
+        if (on) {
             stg4(b.dir_out + 4 * (size_t)c, hb, ub, vb, 0.0);
-            a.fnc_g[c] += fncb;
-            a.zbc_g[c] += l[3] + zg;
+            // one writer per cell and step, the steps in order
+            atomicAdd(a.fnc_g + c, fncb);
+            atomicAdd(a.zbc_g + c, l.w + zg);
         }
     }
-    whb = __shfl_sync(0xffffffffu, whb, lane0);
-    wub = __shfl_sync(0xffffffffu, wub, lane0);
-    wvb = __shfl_sync(0xffffffffu, wvb, lane0);
-    if (!valid) return;
-    // ---- lane j: slot 4c+j
-    const size_t s = 4 * (size_t)c + j;
-    double *so = b.so_out + ADJ_REC * s, *sno = b.sn_out + ADJ_REC * s;
-    const uint8_t meta = a.meta4[s];
-    if (meta == 0xFF) {
-        st_rec(so, Adj5{0, 0, 0, 0, 0});
-        st_rec(sno, Adj5{0, 0, 0, 0, 0});
-        return;
-    }
-    const double cs = a.cs4[s], sn = a.sn4[s], side = a.side4[s];
-    const double slcos = side * cs, slsin = side * sn;
-    double fb[4];
-    fb[0] = side * whb;
-    fb[1] = slcos * wub + slsin * wvb;
-    fb[2] = -slsin * wub + slcos * wvb;
-    fb[3] = fb[1];
-    SlotInA<A> in;
-    in.own = CellStateA<A>{hv, uv, vv, xc.w, zbc};
-    in.code = (int8_t)(meta & META_CODE);
-    in.own_first = meta & META_OWN_FIRST;
-    in.has_nb = meta & META_HAS_NB;
-    const int nb = a.nbr4[s];
-    if (in.has_nb) {
-        const Vec4<double> xn4 = ldg4(x + 4 * (size_t)nb);
-        in.nb = CellStateA<A>{xn4.x, xn4.y, xn4.z, xn4.w, m.zbc[nb]};
-    }
-    else
-        in.nb = CellStateA<A>{0, 0, 0, 0, 0};
-    in.cosj = cs; in.sinj = sn; in.side = side;
-    auto fetch = [&]() {
-        BoundaryInA<A> bi;
-        const int row = m.bcell[c];
-        if (row >= 0) {
-            const size_t q = (size_t)p.jt * m.nb + row;
-            bi.qt = m.bqt[q]; bi.dqt = m.bdqt[q]; bi.zt = m.bzt[q]; bi.dzt = m.bdzt[q];
-            bi.top = m.btop[row]; bi.nhq1 = m.bnhq1[row];
-            bi.zw = m.bzw + (size_t)row * m.nhq; bi.qw = m.bqw + (size_t)row * m.nhq;
-        } else {
-            bi.qt = bi.dqt = 0.0; bi.zt = bi.dzt = bi.top = 0.0; bi.nhq1 = 0;
-            bi.zw = m.bzw + (size_t)m.nb * m.nhq; bi.qw = m.bqw + (size_t)m.nb * m.nhq;
-        }
-        bi.nhq = m.nhq;
-        return bi;
-    };
-    Adj5 go{0, 0, 0, 0, 0}, gn{0, 0, 0, 0, 0};
-    slot_rev(in, p, fetch, fb, go, gn, m.err);
-    st_rec(so, go);
-    st_rec(sno, gn);
 }
 
 // The adjoint of x_0 from step 0's contributions, into a.lam, with their bed terms.
@@ -747,8 +1060,8 @@ struct hb_adjoint {
     double *d_terms = nullptr;              // [4C][4] slot terms of the step being recomputed
     double *d_coef[2] = {nullptr, nullptr}; // [k][C][UPDATE_COEF] update coefficients of a segment
     int recorded_seg = -1;                  // segment whose states the forward left in d_seg (-1: none)
-    cudaStream_t recompute = nullptr;        // the recomputation, ahead of the reverse steps (highest priority)
-    cudaStream_t reverse = nullptr;          // the reverse steps (lowest priority)
+    cudaStream_t recompute = nullptr;        // the recomputation, ahead of the reverse steps
+    cudaStream_t reverse = nullptr;          // the reverse steps
     cudaEvent_t ev_recomputed[2] = {nullptr, nullptr}, ev_reversed[2] = {nullptr, nullptr};
     double *d_gd = nullptr;                 // [nobs][ng] gauge depths of the forward
     double *d_obs = nullptr;                // [nobs][ng]
@@ -832,10 +1145,9 @@ extern "C" int hb_adjoint_create(hb_handle *h, const int32_t *gauges, int32_t ng
             seen[gauges[i]] = 1;
         }
     }
-    // per-slot geometry, codes and facing slots (device order); codes without a reverse are rejected
-    std::vector<double> cs4(4 * (size_t)C, 0.0), sn4(4 * (size_t)C, 0.0), side4(4 * (size_t)C, 0.0);
+    // per slot its record and facing slot (device order); codes without a reverse are rejected
     std::vector<int32_t> nbr4(4 * (size_t)C, -1), mirror4(4 * (size_t)C, -1);
-    std::vector<uint8_t> meta4(4 * (size_t)C, 0xFF);
+    std::vector<int32_t> record(4 * (size_t)C, -1);   // r, or -2 - r for the other slot of pair r; -1 = no real slot
     auto a = new hb_adjoint();
     a->h = h; a->C = C; a->T = nsteps; a->k = checkpoint_every; a->obs_every = obs_every; a->ng = ngauges;
     a->nobs = nsteps / obs_every;
@@ -854,12 +1166,11 @@ extern "C" int hb_adjoint_create(hb_handle *h, const int32_t *gauges, int32_t ng
         const int code = rmeta[r] & hb::META_CODE;
         if (code != hb::CODE_ZERO && code != hb::CODE_K4 && code != hb::CODE_K10 && code != hb::CODE_K1)
             return fail(hb::set_error(HB_E_INVALID, "hb_adjoint_create: boundary code %d has no reverse here (KLAS 0, 1, 4, 10 only)", code));
-        const double *g = &rgeo[4 * (size_t)r];
-        cs4[ix.z] = g[0]; sn4[ix.z] = g[1]; side4[ix.z] = g[2]; nbr4[ix.z] = ix.y; meta4[ix.z] = rmeta[r];
+        nbr4[ix.z] = ix.y;
+        record[ix.z] = r;
         if (ix.w >= 0) {
-            // the other slot of a mirror pair: reversed normal, neighbour a, not the lower-numbered side
-            cs4[ix.w] = -g[0]; sn4[ix.w] = -g[1]; side4[ix.w] = g[2]; nbr4[ix.w] = ix.x;
-            meta4[ix.w] = (uint8_t)(hb::CODE_ZERO | hb::META_HAS_NB);
+            nbr4[ix.w] = ix.x;
+            record[ix.w] = -2 - r;
         }
     }
     // The gather of cell c reads the neighbours' slots that face c through
@@ -870,10 +1181,10 @@ extern "C" int hb_adjoint_create(hb_handle *h, const int32_t *gauges, int32_t ng
         for (int j = 0; j < 4; j++) {
             const size_t s = 4 * (size_t)c + j;
             const int nb = nbr4[s];
-            if (meta4[s] == 0xFF || nb < 0) continue;
+            if (record[s] == -1 || nb < 0) continue;
             for (int q = 0; q < 4; q++) {
                 const size_t t = 4 * (size_t)nb + q;
-                if (nbr4[t] == c && meta4[t] != 0xFF && !claimed[t]) { mirror4[s] = (int32_t)t; claimed[t] = 1; break; }
+                if (nbr4[t] == c && record[t] != -1 && !claimed[t]) { mirror4[s] = (int32_t)t; claimed[t] = 1; break; }
             }
             if (mirror4[s] < 0) return fail(hb::set_error(HB_E_BADMESH, "hb_adjoint_create: cell %d slot %d has no facing slot", c, j));
         }
@@ -887,19 +1198,45 @@ extern "C" int hb_adjoint_create(hb_handle *h, const int32_t *gauges, int32_t ng
     hb::adj::AdjMesh &am = a->am;
     double *dp;
     int32_t *ip;
-    uint8_t *up;
-    if ((st = adj_upload(a, &dp, cs4)) != HB_OK) return fail(st);
-    am.cs4 = dp;
-    if ((st = adj_upload(a, &dp, sn4)) != HB_OK) return fail(st);
-    am.sn4 = dp;
-    if ((st = adj_upload(a, &dp, side4)) != HB_OK) return fail(st);
-    am.side4 = dp;
-    if ((st = adj_upload(a, &ip, nbr4)) != HB_OK) return fail(st);
-    am.nbr4 = ip;
+    // the reverse step's CTAs and their slots
+    std::vector<double> sgeo;
+    sgeo.reserve(16 * (size_t)C);
+    std::vector<int4> seg;
+    int4 cur = make_int4(0, 0, 0, 0);
+    for (int c = 0; c < C; c++) {
+        int n = 0;
+        for (int j = 0; j < 4; j++) n += record[4 * (size_t)c + j] != -1;
+        if (cur.w + n > hb::adj::ADJ_SLOTS || cur.y == hb::adj::ADJ_CELLS) {
+            seg.push_back(cur);
+            cur = make_int4(c, 0, cur.z + cur.w, 0);
+        }
+        for (int j = 0; j < 4; j++) {
+            const int q = record[4 * (size_t)c + j];
+            if (q == -1) continue;
+            const bool other = q < 0;
+            const int r = other ? -2 - q : q;
+            // the other slot of a mirror pair: reversed normal, neighbour a, not the lower-numbered side
+            const double *g = &rgeo[4 * (size_t)r];
+            const uint64_t w = hb::adj::AdjSlot::pack(nbr4[4 * (size_t)c + j], 4 * cur.y + j,
+                                                      other ? (uint8_t)(hb::CODE_ZERO | hb::META_HAS_NB) : rmeta[r]);
+            double word;
+            memcpy(&word, &w, sizeof word);
+            sgeo.insert(sgeo.end(), {other ? -g[0] : g[0], other ? -g[1] : g[1], g[2], word});
+        }
+        cur.y++;
+        cur.w += n;
+    }
+    seg.push_back(cur);
+    if ((st = adj_upload(a, &dp, sgeo)) != HB_OK) return fail(st);
+    am.sgeo = dp;
+    {
+        int4 *cp;
+        if ((st = adj_upload(a, &cp, seg)) != HB_OK) return fail(st);
+        am.seg = cp;
+        am.nseg = (int)seg.size();
+    }
     if ((st = adj_upload(a, &ip, mirror4)) != HB_OK) return fail(st);
     am.mirror4 = ip;
-    if ((st = adj_upload(a, &up, meta4)) != HB_OK) return fail(st);
-    am.meta4 = up;
     if ((st = adj_upload(a, &ip, gauge_of)) != HB_OK) return fail(st);
     am.gauge_of = ip;
     if ((st = adj_upload(a, &a->d_gcell, a->gauges_dev)) != HB_OK) return fail(st);
@@ -926,10 +1263,8 @@ extern "C" int hb_adjoint_create(hb_handle *h, const int32_t *gauges, int32_t ng
             cudaEventCreateWithFlags(&a->ev_reversed[q], cudaEventDisableTiming) != cudaSuccess)
             return fail(hb::set_error(HB_E_CUDA, "hb_adjoint_create: cudaEventCreate failed"));
     }
-    int least = 0, greatest = 0;
-    if (cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess ||
-        cudaStreamCreateWithPriority(&a->recompute, cudaStreamNonBlocking, greatest) != cudaSuccess ||
-        cudaStreamCreateWithPriority(&a->reverse, cudaStreamNonBlocking, least) != cudaSuccess)
+    if (cudaStreamCreateWithFlags(&a->recompute, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&a->reverse, cudaStreamNonBlocking) != cudaSuccess)
         return fail(hb::set_error(HB_E_CUDA, "hb_adjoint_create: cudaStreamCreate failed"));
     if ((st = adj_alloc(a, &a->d_gd, (size_t)std::max(a->nobs, 1) * ngauges)) != HB_OK) return fail(st);
     if ((st = adj_alloc(a, &a->d_obs, (size_t)std::max(a->nobs, 1) * ngauges)) != HB_OK) return fail(st);
@@ -1159,8 +1494,8 @@ int enqueue_backward(hb_adjoint *a, bool have_last, cudaStream_t st, std::vector
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)((4 * C + 127) / 128));
-    cfg.blockDim = dim3(128);
+    cfg.gridDim = dim3((unsigned)am.nseg);
+    cfg.blockDim = dim3(hb::adj::ADJ_THREADS);
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
@@ -1211,6 +1546,11 @@ int enqueue_backward(hb_adjoint *a, bool have_last, cudaStream_t st, std::vector
             const int row = (t + 1 < a->T && (t + 1) % a->obs_every == 0) ? (t + 1) / a->obs_every - 1 : -1;
             const double *xs = seg_state(sgi, i), *xn = a->d_seg[b] + (size_t)(i + 1) * S4;
             const double *cf = a->d_coef[b] + (size_t)i * hb::UPDATE_COEF * C;
+            // The segment's first reverse step starts only when its recomputation
+            // is complete (an ordinary launch: as a programmatic one it could start
+            // once the last recomputed step had triggered, and it reads that
+            // step's results ahead of its wait).  The later ones start after it.
+            cfg.numAttrs = i == len - 1 ? 0 : 1;
             HB_CUDA_RET(cudaLaunchKernelEx(&cfg, hb::adj::adj_step_kernel, h->m64, am, bufs, xs, xn, cf, p,
                                            (int)(t == a->T - 1), row));
         }
@@ -1230,8 +1570,7 @@ int enqueue_backward(hb_adjoint *a, bool have_last, cudaStream_t st, std::vector
     return HB_OK;
 }
 
-// Captures enqueue_backward on the reverse stream into an executable graph
-// that keeps the recompute stream's higher priority per node.
+// Captures enqueue_backward on the reverse stream into an executable graph.
 int capture_backward(hb_adjoint *a, bool have_last, cudaGraphExec_t *exec) {
     cudaStream_t st = a->reverse;
     std::vector<cudaEvent_t> temp;
@@ -1242,7 +1581,7 @@ int capture_backward(hb_adjoint *a, bool have_last, cudaGraphExec_t *exec) {
     for (cudaEvent_t ev : temp) cudaEventDestroy(ev);
     if (rc != HB_OK) { if (g) cudaGraphDestroy(g); return rc; }
     if (e != cudaSuccess) return hb::set_error(HB_E_CUDA, "adjoint backward capture: %s", cudaGetErrorString(e));
-    const cudaError_t ei = cudaGraphInstantiateWithFlags(exec, g, cudaGraphInstantiateFlagUseNodePriority);
+    const cudaError_t ei = cudaGraphInstantiate(exec, g, 0);
     cudaGraphDestroy(g);
     if (ei != cudaSuccess) {
         *exec = nullptr;
@@ -1258,14 +1597,12 @@ extern "C" int hb_adjoint_backward(hb_adjoint *a, double *grad_n, double *grad_z
     if (!a) return hb::set_error(HB_E_INVALID, "null adjoint");
     if (!a->forward_done) return hb::set_error(HB_E_INVALID, "hb_adjoint_backward: run hb_adjoint_forward first");
     hb_handle *h = a->h;
-    // The reverse steps run on the adjoint's own lowest-priority stream and
-    // the recomputation of the next segment on its highest-priority one, both
-    // joined to the caller's stream.  The recomputation is a chain of small
-    // kernels; given priority, its blocks start as soon as they are ready
-    // instead of queueing behind the reverse grids, which fill the rest of
-    // the GPU (measured: backward 19.4 -> 17.1 ms on the 24K-cell, 1000-step
-    // case; the other way round, 21.1 ms).  The pass is one graph, captured
-    // on first use (per kind of pass) and replayed after: its thousands of
+    // The reverse steps and the recomputation of the next segment run on two
+    // streams of the adjoint's own, joined to the caller's, both of the same
+    // priority: 24,020 cells, checkpoints every 10 steps, 10.2 us per step of
+    // the backward pass; 11.8 us with the recomputation at the higher
+    // priority and 12.0 us the other way round.  The pass is one graph,
+    // captured on first use (per kind of pass) and replayed after: its
     // launches then cost no host time each.
     cudaStream_t user = (cudaStream_t)stream;
     cudaStream_t st = a->reverse;
