@@ -7,16 +7,21 @@
 
 namespace {
 
-// The one-launch step takes single fp64 meshes of at most this many cells (edge
-// layout, default launch shape).  It halves the latencies of a step but
-// computes every edge twice.  us per step on a B200, 40- or 100-step graphs,
-// one launch / two kernels, variant H:
-//   cells      6,675      24,021     60,000      100,000      120,000      140,000
-//   channel   4.3 / 8.4  5.0 / 9.1  8.6 / 12.4  13.7 / 14.6  14.7 / 15.7  17.6 / 17.1
-//   mixed     4.4 / 8.8  5.6 / 9.9  10.4/ 13.6  14.6 / 15.4  16.8 / 17.3  19.0 / 17.9
-//   dam break 5.3*/ 9.5  5.6 / 10.5 8.5 / 15.0  11.6 / 16.1  12.7 / 17.9  15.3 / 19.2
-// (* before the update warp.)  The line lies where channels and mixed meshes cross.
-constexpr int CELLS_MAX = 120000;
+// The one-launch step takes single fp64 meshes whose CTAs are all resident at
+// once (edge layout, default launch shape): about 33,000 triangles on a B200.
+// It halves the latencies of a step but computes every edge twice, and its
+// second wave costs as much as its first.  us per step, 40-step graphs, one
+// launch / two kernels, variant H:
+//   cells      24,021      32,000      40,000      60,000
+//   channel   4.6 / 6.8   4.6 / 7.7   7.7 / 7.7   8.7*/ 8.7
+//   mixed     5.2 / 7.9   7.7*/ 7.7   8.1*/ 8.0  10.1*/ 10.1
+//   dam break 6.7 / 8.8   6.8 / 8.9     -  / 9.1     -  / 11.4
+// (* two waves)
+bool fits_at_once(const hb_handle *h, size_t ctas) {
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->opt.device) != cudaSuccess) return false;
+    return ctas <= (size_t)sms * hb::CELL_CTAS;
+}
 
 template <int VARIANT, bool COEF>
 int launch_cells_t(int ncseg, const hb::DevMesh<hb::F64Exact> &m, int k0, int n, int write_last, cudaStream_t st) {
@@ -44,7 +49,7 @@ bool hb_cells_used(const hb_handle *h) {
 int hb_cells_build(hb_handle *h, const std::vector<int4> &rix, const std::vector<uint8_t> &rmeta,
                    const std::vector<double> &rgeo) {
     if (h->opt.precision != HB_FP64 || h->opt.layout != HB_LAYOUT_EDGE || h->opt.persistent || h->segmented() ||
-        h->C > CELLS_MAX)
+        !fits_at_once(h, (size_t)h->C / hb::CELL_MAX) || rix.size() >= (size_t)hb::SlotRef::MAX_RECORD)
         return HB_OK;
     hb::DevMesh<hb::F64Exact> &m = h->m64;
     const int nrec = (int)rix.size();
@@ -55,9 +60,7 @@ int hb_cells_build(hb_handle *h, const std::vector<int4> &rix, const std::vector
         record[rix[r].z] = r;
         if (rix[r].w >= 0) record[rix[r].w] = -2 - r;
     }
-    // one allocation: the slot records (32-byte aligned), then the CTAs' entries
-    std::vector<double> table;
-    table.reserve(18 * (size_t)h->C + 64);
+    // the CTAs' runs of cells
     std::vector<int4> seg;
     int4 cur = make_int4(0, 0, 0, 0);
     for (int c = 0; c < h->C; c++) {
@@ -67,23 +70,32 @@ int hb_cells_build(hb_handle *h, const std::vector<int4> &rix, const std::vector
             seg.push_back(cur);
             cur = make_int4(c, 0, cur.z + cur.w, 0);
         }
-        for (int j = 0; j < 4; j++) {
-            const int q = record[4 * (size_t)c + j];
-            if (q == -1) continue;
-            const bool other = q < 0;
-            const int r = other ? -2 - q : q;
-            // a pair's other slot: negated normal, same length, not the lower-numbered side
-            const double *g = &rgeo[4 * (size_t)r];
-            const uint64_t w = hb::SlotRef::pack(other ? rix[r].x : rix[r].y, 4 * cur.y + j,
-                                                 other ? (uint8_t)(hb::CODE_ZERO | hb::META_HAS_NB) : rmeta[r], r);
-            double d;
-            memcpy(&d, &w, sizeof d);
-            table.insert(table.end(), {other ? -g[0] : g[0], other ? -g[1] : g[1], g[2], d});
-        }
         cur.y++;
         cur.w += n;
     }
     seg.push_back(cur);
+    if (!fits_at_once(h, seg.size())) return HB_OK;
+    // One allocation: the slot records (32-byte aligned), then the CTAs' entries.
+    // A CTA's boundary slots, the slowest ones, come last, so that they share
+    // as few warps as possible with the others.
+    std::vector<double> table;
+    table.reserve(4 * (size_t)(cur.z + cur.w) + 2 * seg.size());
+    for (const int4 &d : seg)
+        for (int boundary = 0; boundary < 2; boundary++)
+            for (int place = 0; place < 4 * d.y; place++) {
+                const int q = record[4 * (size_t)d.x + place];
+                if (q == -1) continue;
+                const bool other = q < 0;
+                const int r = other ? -2 - q : q;
+                // a pair's other slot: negated normal, same length, not the lower-numbered side
+                const uint8_t meta = other ? (uint8_t)(hb::CODE_ZERO | hb::META_HAS_NB) : rmeta[r];
+                if (boundary != ((meta & hb::META_CODE) != hb::CODE_ZERO)) continue;
+                const double *g = &rgeo[4 * (size_t)r];
+                const uint64_t w = hb::SlotRef::pack(other ? rix[r].x : rix[r].y, place, meta, r);
+                double v;
+                memcpy(&v, &w, sizeof v);
+                table.insert(table.end(), {other ? -g[0] : g[0], other ? -g[1] : g[1], g[2], v});
+            }
     const size_t records = table.size();
     table.resize(records + 2 * seg.size());
     memcpy(table.data() + records, seg.data(), seg.size() * sizeof(int4));

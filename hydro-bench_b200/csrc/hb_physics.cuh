@@ -56,11 +56,14 @@ __host__ __device__ inline bool code_is_bounda(int8_t c) { return c != CODE_ZERO
 // ---------------------------------------------------------------------------
 // arithmetic policies
 // ---------------------------------------------------------------------------
+// `route_modes`: the direct and the mirrored Osher route round some rotations
+// differently (the fusion modes below).
 // Every policy has a `real` type for the flux/state arithmetic and a `level`
 // type for water levels and bed elevations (Z, ZBC, ZT, ZW, crest heights).
 // A depth rebuilt from levels (level minus bed) is formed in `level`
 // precision and then rounded to `real` (depth()).
 struct F64Exact {
+    static constexpr bool route_modes = true;
     using real = double;
     using level = double;
     static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
@@ -80,14 +83,22 @@ struct F64Exact {
     // over/underflow of every quotient here) take __ddiv_rn; one unsigned
     // compare of the high word tells them.
     static __device__ __forceinline__ double divk(double x, double c) {
-        const double y = 1.0 / c;
         const unsigned e = ((unsigned)__double2hiint(x) & 0x7FFFFFFFu) - ((1023u - 900u) << 20);
-        if (e < (1800u << 20)) {
-            const double q = __dmul_rn(x, y);
-            return __fma_rn(__fma_rn(-q, c, x), y, q);
-        }
+        if (e < (1800u << 20)) return divk_raw(x, c);
         return __ddiv_rn(x, c);
     }
+    // divk for an x known to be in that range
+    static __device__ __forceinline__ double divk_raw(double x, double c) {
+        const double y = 1.0 / c;
+        const double q = __dmul_rn(x, y);
+        return __fma_rn(__fma_rn(-q, c, x), y, q);
+    }
+    // x >= 0 is within [2^-200, 2^200)
+    static __device__ __forceinline__ bool quotient_range(double x) {
+        return (unsigned)__double2hiint(x) - ((1023u - 200u) << 20) < (400u << 20);
+    }
+    // x >= 0, for an x that is not -0
+    static __device__ __forceinline__ bool nonnegative(double x) { return __double2hiint(x) >= 0; }
     static __device__ __forceinline__ double fma(double a, double b, double c) { return __fma_rn(a, b, c); }
     static __device__ __forceinline__ double sqrt(double a) { return __dsqrt_rn(a); }
     static __device__ __forceinline__ double pow(double a, double b) { return ::pow(a, b); }
@@ -120,6 +131,7 @@ struct F64Exact {
 };
 
 struct F32Fast {
+    static constexpr bool route_modes = false;
     using real = float;
     using level = float;
     static __device__ __forceinline__ float mul(float a, float b) { return a * b; }
@@ -127,6 +139,9 @@ struct F32Fast {
     static __device__ __forceinline__ float sub(float a, float b) { return a - b; }
     static __device__ __forceinline__ float div(float a, float b) { return a / b; }
     static __device__ __forceinline__ float divk(float x, double c) { return x / (float)c; }
+    static __device__ __forceinline__ float divk_raw(float x, double c) { return x / (float)c; }
+    static __device__ __forceinline__ bool quotient_range(float) { return true; }
+    static __device__ __forceinline__ bool nonnegative(float x) { return x >= 0.f; }
     static __device__ __forceinline__ float fma(float a, float b, float c) { return fmaf(a, b, c); }
     static __device__ __forceinline__ float sqrt(float a) { return sqrtf(a); }
     static __device__ __forceinline__ float pow(float a, float b) { return powf(a, b); }
@@ -239,86 +254,19 @@ struct StepParams {
 // ---------------------------------------------------------------------------
 // Osher approximate Riemann solver, functors.cu:445-511, :570-712
 // ---------------------------------------------------------------------------
-// out += sign * QF(h, u, v) with the reference build's sums (functors.cu:453-497, :505-511)
+// out += QF(h, u, v) (or -=, `neg`) with the reference build's sums
+// (functors.cu:453-497, :505-511)
 template <class A>
-__device__ __forceinline__ void qf_acc(typename A::real out[4], typename A::real h, typename A::real u,
-                                       typename A::real v, int sign) {
+__device__ __forceinline__ void qf_acc(typename A::real out[4], bool neg, typename A::real h, typename A::real u,
+                                       typename A::real v) {
     using R = typename A::real;
-    R f0 = A::mul(h, u);
-    R sh = sign > 0 ? h : -h;
-    R sf0 = sign > 0 ? f0 : -f0;
-    out[0] = A::madd(sh, u, out[0], M_ACC0);
+    const R f0 = A::mul(h, u);
+    const R sf0 = neg ? -f0 : f0;
+    const R h4 = A::mul(A::c(4.905), h);
+    out[0] = A::madd(neg ? -h : h, u, out[0], M_ACC0);
     out[1] = A::madd(sf0, u, out[1], M_ACC123);
     out[2] = A::madd(sf0, v, out[2], M_ACC123);
-    R h4 = A::mul(A::c(4.905), h);
-    out[3] = A::madd(sign > 0 ? h4 : -h4, h, out[3], M_ACC123);
-}
-
-// Per-piece record of one Osher evaluation, for re-summing FLUX2 with another
-// tangential velocity: f0[i] = h*u of piece i (pieces 1, 2, 3, 5, 6, 7 in that
-// order; 1-3 carry QL's tangent, 5-7 QR's), act/neg bit i = added / subtracted.
-template <class R>
-struct OsherTrace {
-    R f0[6];
-    unsigned act, neg;
-    __device__ __forceinline__ void set(int i, R v) { f0[i] = v; }
-    __device__ __forceinline__ R get(int i) const { return f0[i]; }
-};
-// The same record with the products kept in a store the caller provides
-// (TS: set(i, v) / get(i)), e.g. shared memory: they are read back only for
-// the rare re-summed FLUX2, so they need not occupy registers across the rest
-// of the evaluation.
-template <class TS>
-struct OsherTraceIn {
-    TS *ts;
-    unsigned act, neg;
-    template <class R> __device__ __forceinline__ void set(int i, R v) { ts->set(i, v); }
-    __device__ __forceinline__ auto get(int i) const { return ts->get(i); }
-};
-
-// out += QF(h, u, v) (or -=, `neg`) when `on`, with the reference build's sums
-// (functors.cu:453-497, :505-511); `out` is untouched otherwise.
-template <class A, class TR>
-__device__ __forceinline__ void qf_acc_if(typename A::real out[4], bool on, bool neg, typename A::real h,
-                                          typename A::real u, typename A::real v, TR *tr, int piece) {
-    using R = typename A::real;
-    R f0 = A::mul(h, u);
-    R sh = neg ? -h : h;
-    R sf0 = neg ? -f0 : f0;
-    R h4 = A::mul(A::c(4.905), h);
-    R o0 = A::madd(sh, u, out[0], M_ACC0);
-    R o1 = A::madd(sf0, u, out[1], M_ACC123);
-    R o2 = A::madd(sf0, v, out[2], M_ACC123);
-    R o3 = A::madd(neg ? -h4 : h4, h, out[3], M_ACC123);
-    if (on) { out[0] = o0; out[1] = o1; out[2] = o2; out[3] = o3; }
-    if constexpr (!std::is_same<TR, void>::value) {
-        tr->set(piece, f0);
-        tr->act |= (on ? 1u : 0u) << piece;
-        tr->neg |= (neg ? 1u : 0u) << piece;
-    }
-}
-
-// A piece that is not taken: traced as inactive (osher_f2 skips it).
-template <class A, class TR>
-__device__ __forceinline__ void qf_skip(TR *tr, int piece) {
-    if constexpr (!std::is_same<TR, void>::value) tr->set(piece, typename A::real(0));
-}
-
-// FLUX2 of a traced Osher evaluation re-summed with tangents ql2 / qr2, in the
-// same order and with the same fused sums as qf_acc_if.
-template <class A, class TR>
-__device__ __forceinline__ typename A::real osher_f2(const TR &tr, typename A::real ql2, typename A::real qr2) {
-    using R = typename A::real;
-    R acc = R(0);
-#pragma unroll
-    for (int i = 0; i < 6; i++) {
-        const R v = i < 3 ? ql2 : qr2;
-        const R f0 = tr.get(i);
-        const R sf0 = ((tr.neg >> i) & 1u) ? -f0 : f0;
-        const R o2 = A::madd(sf0, v, acc, M_ACC123);
-        if ((tr.act >> i) & 1u) acc = o2;
-    }
-    return acc;
+    out[3] = A::madd(neg ? -h4 : h4, h, out[3], M_ACC123);
 }
 
 // OSHER(pos, H_pre, QL, QR, FIL, FLR_OSHER), functors.cu:570-712, with the
@@ -335,12 +283,11 @@ __device__ __forceinline__ typename A::real osher_f2(const TR &tr, typename A::r
 // with one are formed only by the lanes that take them.
 // Piece 3 updates FIL and piece 5 updates FIR (QS<3>, QS<5>); no case has
 // both, and piece 6 sees the FIR that piece 5 left.
-template <class A, class TR = void>
+template <class A>
 __device__ __forceinline__ void osher(typename A::real cl, const typename A::real ql[3],
                                       const typename A::real qr[3], typename A::real fil,
-                                      typename A::real out[4], TR *tr = nullptr) {
+                                      typename A::real out[4]) {
     using R = typename A::real;
-    if constexpr (!std::is_same<TR, void>::value) { tr->act = 0; tr->neg = 0; }
     R cr = A::sqrt(A::mul(A::c(9.81), qr[0]));
     R fir = A::sub(qr[1], A::mul(A::c(2.0), cr));
     R ua = A::mul(A::add(fil, fir), A::c(0.5));
@@ -370,52 +317,50 @@ __device__ __forceinline__ void osher(typename A::real cl, const typename A::rea
     // and 7 (supercritical flow out of a side) are rare, so a warp usually
     // skips them altogether.
     // piece 1: QF(QL)
-    if (p1) qf_acc_if<A>(out, true, false, ql[0], ql[1], ql[2], tr, 0);
-    else qf_skip<A>(tr, 0);
+    if (p1) qf_acc<A>(out, false, ql[0], ql[1], ql[2]);
     // piece 2: US = FIL/3, HS = US^2/9.81
     if (p2) {
-        R us = A::divk(fil, 3.0);
-        R hs = A::divk(A::mul(us, us), 9.81);
-        qf_acc_if<A>(out, true, n2, hs, us, ql[2], tr, 1);
-    } else {
-        qf_skip<A>(tr, 1);
+        const R us = A::divk(fil, 3.0);
+        qf_acc<A>(out, n2, A::divk(A::mul(us, us), 9.81), us, ql[2]);
     }
     // pieces 3 and 5 share UA = (FIL + FIR)/2 and the same arithmetic on
     // their own inputs (FIL - UA with QL's tangent, FIR - UA with QR's); no
     // case takes both, so one code path forms whichever is taken and a warp
     // whose lanes take different ones runs it once
-    const R ua35 = A::mul(A::add(fil, fir), A::c(0.5));
-    const R fir5 = A::sub(fir, ua35);
+    const R fir5 = A::sub(fir, ua);
     if (p3 || p5) {
-        const R d = p3 ? A::sub(fil, ua35) : fir5;
-        const R ha = A::divk(A::mul(d, d), 39.24);
-        const R vt = p3 ? ql[2] : qr[2];
-        const R f0 = A::mul(ha, ua35);
-        out[0] = A::madd(ha, ua35, out[0], M_ACC0);
-        out[1] = A::madd(f0, ua35, out[1], M_ACC123);
-        out[2] = A::madd(f0, vt, out[2], M_ACC123);
-        out[3] = A::madd(A::mul(A::c(4.905), ha), ha, out[3], M_ACC123);
-        if constexpr (!std::is_same<TR, void>::value) {
-            tr->set(2, p3 ? f0 : R(0));
-            tr->set(3, p5 ? f0 : R(0));
-            tr->act |= (p3 ? 4u : 0u) | (p5 ? 8u : 0u);
-        }
-    } else {
-        qf_skip<A>(tr, 2);
-        qf_skip<A>(tr, 3);
+        const R d = p3 ? A::sub(fil, ua) : fir5;
+        qf_acc<A>(out, false, A::divk(A::mul(d, d), 39.24), ua, p3 ? ql[2] : qr[2]);
     }
     // piece 6: US = FIR/3 with FIR as piece 5 left it
     if (p6) {
-        R f6 = p5 ? fir5 : fir;
-        R us = A::divk(f6, 3.0);
-        R hs = A::divk(A::mul(us, us), 9.81);
-        qf_acc_if<A>(out, true, n6, hs, us, qr[2], tr, 4);
-    } else {
-        qf_skip<A>(tr, 4);
+        const R us = A::divk(p5 ? fir5 : fir, 3.0);
+        qf_acc<A>(out, n6, A::divk(A::mul(us, us), 9.81), us, qr[2]);
     }
     // piece 7: QF(QR)
-    if (p7) qf_acc_if<A>(out, true, false, qr[0], qr[1], qr[2], tr, 5);
-    else qf_skip<A>(tr, 5);
+    if (p7) qf_acc<A>(out, false, qr[0], qr[1], qr[2]);
+}
+
+// The case of subcritical flow across the edge (K1 = 1, K2 = 2 or 3), which
+// adds piece 3 or piece 5 alone: osher()'s result for it, from `cr` =
+// sqrt(9.81*QR[0]).  False (and no result) in any other case, at UA = -CA, and
+// where CA leaves the range in which the policy's quotients by a constant need
+// no checks (quotient_range): with CA in it, D = +-2 CA, HA and FLUX3 are in
+// divk_raw's range too.
+template <class A>
+__device__ __forceinline__ bool osher_subcritical(typename A::real cl, typename A::real cr, typename A::real ql1,
+                                                  typename A::real ql2, typename A::real qr1, typename A::real qr2,
+                                                  typename A::real fil, typename A::real out[4]) {
+    using R = typename A::real;
+    const R fir = A::sub(qr1, A::mul(A::c(2.0), cr));
+    const R ua = A::mul(A::add(fil, fir), A::c(0.5));
+    const R ca = A::fabs(A::mul(A::sub(fil, fir), A::c(0.25)));
+    const bool p3 = A::nonnegative(ua);   // FIL + FIR is never -0
+    const R d = A::sub(p3 ? fil : fir, ua);
+    const R ha = A::divk_raw(A::mul(d, d), 39.24);
+    out[0] = out[1] = out[2] = out[3] = R(0);
+    qf_acc<A>(out, false, ha, ua, p3 ? ql2 : qr2);
+    return ql1 < cl && qr1 >= -cr && A::fabs(ua) < ca && A::quotient_range(ca);
 }
 
 // ---------------------------------------------------------------------------

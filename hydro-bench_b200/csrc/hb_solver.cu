@@ -342,7 +342,14 @@ int append_scenario(const hb_mesh_desc *md, int scn, const hb_options &opt, hb::
                                    sb < 0 ? -1 : (int)(4 * (size_t)c0 + sb)));
         hm.rmeta.push_back(mt);
         hm.rgeo.push_back((R)md->cosf[so]); hm.rgeo.push_back((R)md->sinf[so]);
-        hm.rgeo.push_back((R)md->side[so]); hm.rgeo.push_back(R(0));
+        hm.rgeo.push_back((R)md->side[so]);
+        R slots = R(0);
+        if constexpr (std::is_same<R, double>::value) {
+            const int4 ix = hm.rix.back();
+            const unsigned long long w = hb::pack_slots(ix.z, ix.y, ix.w);
+            std::memcpy(&slots, &w, sizeof slots);
+        }
+        hm.rgeo.push_back(slots);
     };
     sc.slot_index.assign(S, -1);
     sc.npairs = 0;
@@ -563,12 +570,12 @@ int build_device_mesh(hb_handle *h, const hb_mesh_desc *mds, int n, hb::DevMesh<
     {
         std::vector<hb::TileDesc> tiles;
         m.max_tile_cells = 1;
-        m.max_tile_pairs = 1;
+        m.max_tile_queue = 1;
         for (const auto &sc : h->scn)
             for (const auto &td : sc.tiles) {
                 tiles.push_back(td);
                 m.max_tile_cells = std::max(m.max_tile_cells, td.cells);
-                m.max_tile_pairs = std::max(m.max_tile_pairs, td.npairs);
+                m.max_tile_queue = std::max(m.max_tile_queue, 2 * td.npairs + td.nsingles);
             }
         m.ntiles = (int)tiles.size();
         hb::TileDesc *tp;
@@ -636,12 +643,12 @@ int launch_steps_t(hb_handle *h, hb::DevMesh<A> m, int n, cudaStream_t st) {
     int rc;
     using namespace hb;
     switch (h->launch_config) {
-    case 0: rc = go(flux_kernel<A, VARIANT, 128, 7, SEG>, 128, update_kernel<A, VARIANT, 8, SEG>); break;
+    case 0: rc = go(flux_kernel<A, VARIANT, 128, 7, SEG>, 128, update_kernel<A, VARIANT, 6, SEG>); break;
     case 1: rc = go(flux_kernel<A, VARIANT, 128, 6, SEG>, 128, update_kernel<A, VARIANT, 8, SEG>); break;
     case 2: rc = go(flux_kernel<A, VARIANT, 128, 8, SEG>, 128, update_kernel<A, VARIANT, 8, SEG>); break;
     case 3: rc = go(flux_kernel<A, VARIANT, 256, 3, SEG>, 256, update_kernel<A, VARIANT, 6, SEG>); break;
     case 4: rc = go(flux_kernel<A, VARIANT, 256, 4, SEG>, 256, update_kernel<A, VARIANT, 8, SEG>); break;
-    case 5: rc = go(flux_kernel<A, VARIANT, 128, 7, SEG>, 128, update_kernel<A, VARIANT, 6, SEG>); break;
+    case 5: rc = go(flux_kernel<A, VARIANT, 128, 7, SEG>, 128, update_kernel<A, VARIANT, 8, SEG>); break;
     case 6: rc = go(flux_kernel<A, VARIANT, 256, 2, SEG>, 256, update_kernel<A, VARIANT, 6, SEG>); break;
     case 7: rc = go(flux_kernel<A, VARIANT, 64, 12, SEG>, 64, update_kernel<A, VARIANT, 8, SEG>); break;
     case 14: rc = go(flux_kernel<A, VARIANT, 128, 6, SEG>, 128, update_kernel<A, VARIANT, 6, SEG>); break;
@@ -778,7 +785,7 @@ int hb_forward_step_into(hb_handle *h, long long t0, int k, const double *in, do
     cfg.numAttrs = 1;
     cfg.gridDim = dim3((unsigned)((m.nrecords + 127) / 128));
     cfg.blockDim = dim3(128);
-    HB_CUDA_RET(cudaLaunchKernelEx(&cfg, hb::flux_kernel<hb::F64Exact, 0, 128, 6, false, false>, m, k, write_flux));
+    HB_CUDA_RET(cudaLaunchKernelEx(&cfg, hb::flux_kernel<hb::F64Exact, 0, 128, 7, false>, m, k, write_flux));
     cfg.gridDim = dim3((unsigned)((m.C + hb::UPDATE_THREADS - 1) / hb::UPDATE_THREADS));
     cfg.blockDim = dim3(hb::UPDATE_THREADS);
     HB_CUDA_RET(cudaLaunchKernelEx(&cfg, hb::update_kernel<hb::F64Exact, 0, 6, false, true>, m, k, write_flux));

@@ -25,8 +25,8 @@ enum : uint8_t { META_CODE = 0x0F, META_OWN_FIRST = 0x10, META_HAS_NB = 0x20 };
 enum Layout : int { LAYOUT_EDGE = HB_LAYOUT_EDGE, LAYOUT_TILE = HB_LAYOUT_TILE };
 struct LaunchConfig { int layout, threads, min_blocks, update_min_blocks; };
 constexpr LaunchConfig LAUNCH_CONFIGS[] = {
-    {LAYOUT_EDGE, 128, 7, 8}, {LAYOUT_EDGE, 128, 6, 8}, {LAYOUT_EDGE, 128, 8, 8}, {LAYOUT_EDGE, 256, 3, 6},
-    {LAYOUT_EDGE, 256, 4, 8}, {LAYOUT_EDGE, 128, 7, 6}, {LAYOUT_EDGE, 256, 2, 6}, {LAYOUT_EDGE, 64, 12, 8},
+    {LAYOUT_EDGE, 128, 7, 6}, {LAYOUT_EDGE, 128, 6, 8}, {LAYOUT_EDGE, 128, 8, 8}, {LAYOUT_EDGE, 256, 3, 6},
+    {LAYOUT_EDGE, 256, 4, 8}, {LAYOUT_EDGE, 128, 7, 8}, {LAYOUT_EDGE, 256, 2, 6}, {LAYOUT_EDGE, 64, 12, 8},
     {LAYOUT_TILE, 256, 3, 0}, {LAYOUT_TILE, 256, 2, 0}, {LAYOUT_TILE, 128, 6, 0}, {LAYOUT_TILE, 128, 4, 0},
     {LAYOUT_TILE, 512, 1, 0}, {LAYOUT_TILE, 256, 4, 0},
     {LAYOUT_EDGE, 128, 6, 6}, {LAYOUT_EDGE, 128, 6, 9}, {LAYOUT_EDGE, 128, 7, 9}, {LAYOUT_TILE, 128, 8, 0},
@@ -87,7 +87,7 @@ struct DevMesh {
     const int4 *rix;           // {a, b, sa, sb}: cell of the slot, its neighbour (-1 = none),
                                // slot 4*a+j, and for a pair the slot of b (-1 otherwise)
     uint8_t *rmeta;            // code | own_first | has_nb of slot a (code changes on breach)
-    const R *rgeo;             // [nrecords][4] {COSF, SINF, SIDE, 0} of slot a
+    const R *rgeo;             // [nrecords][4] {COSF, SINF, SIDE, x} of slot a; x: fp64 pack_slots, else 0
     const R *sgeo;             // [real slots][4] {COSF, SINF, SIDE, SlotRef::pack} (cell_kernel; else null)
     const int4 *cseg;          // cell_kernel CTAs {first cell, cells, first slot record, slot records}
     R *f0, *f1, *f2, *f3;      // [4C] fluxes of the last step, index 4*cell + j
@@ -114,26 +114,39 @@ struct DevMesh {
     int rev_flux, rev_update;
     // tile layout
     const TileDesc *tiles;     // [ntiles]
-    int ntiles, max_tile_cells, max_tile_pairs;
+    int ntiles, max_tile_cells, max_tile_queue;   // the largest tile's cells and queue entries (2 per pair, 1 per single)
 };
 
-struct StepIndex { int par, kt, jt; long long step; };
+// One step: the state buffer it reads, its number, and its scenario's table
+// intervals.
+struct StepIndex { int par, per_day, ndays; long long step; };
 
 // EARLY: read ahead of the dependency wait, so from L2 (a line that an earlier
 // launch left in L1 may be old).
 template <bool EARLY = false, class A>
 __device__ __forceinline__ StepIndex step_index(const DevMesh<A> &m, int k, int per_day, int ndays) {
     const long long step = (EARLY ? __ldcg(m.step_ctr) : *m.step_ctr) + k;
-    StepIndex si;
-    si.step = step;
-    si.par = (int)(step & 1);
-    si.jt = (int)(step / per_day);
-    si.kt = 1 + (int)(step % per_day);
-    if (si.jt >= ndays) {   // beyond the boundary tables: never read past them
-        if (threadIdx.x == 0) atomicOr(m.err, ERRBIT_TABLE_RANGE);
-        si.jt = ndays - 1;
+    if (threadIdx.x == 0 && step >= (long long)per_day * ndays) atomicOr(m.err, ERRBIT_TABLE_RANGE);
+    return {(int)(step & 1), per_day, ndays, step};
+}
+
+// The step's day and step within it, for the slots that read boundary tables:
+// the division (by a value known at run time) is left to them, since it costs
+// about as much as a fifth of a cell's whole update.  Beyond the tables (which
+// step_index reports) the last interval, so that they are never read past.
+__device__ __forceinline__ StepParams with_time(StepParams p, const StepIndex &si) {
+    int day, in_day;
+    if (si.step <= 0xFFFFFFFFll) {
+        const unsigned s = (unsigned)si.step, q = s / (unsigned)si.per_day;
+        day = (int)q;
+        in_day = (int)(s - q * (unsigned)si.per_day);
+    } else {
+        day = (int)(si.step / si.per_day);
+        in_day = (int)(si.step % si.per_day);
     }
-    return si;
+    p.jt = day >= si.ndays ? si.ndays - 1 : day;
+    p.kt = 1 + in_day;
+    return p;
 }
 
 template <class R> struct Vec4 { R x, y, z, w; };
@@ -209,11 +222,12 @@ __device__ __forceinline__ void store_flux(const DevMesh<A> &m, int s, const typ
 
 // One slot on its own: flux_slot with its boundary tables (functors.cu:47-202).
 // single_core takes the slot's cell a (device order, for its table row), its
-// slot sa, both cells' states and the record's code byte and geometry.
+// slot sa, both cells' states and the record's code byte and geometry; for a
+// boundary code p has the step's time (with_time).
 template <class A, int VARIANT, class T>
 __device__ __forceinline__ void single_core(const DevMesh<A> &m, int r, int a, int sa, const CellStateA<A> &own,
                                             const CellStateA<A> &nb, uint8_t meta, const Vec4<typename A::real> &g,
-                                            const StepIndex &si, const StepParams &p, int write_flux, const T &tout) {
+                                            const StepParams &p, int write_flux, const T &tout) {
     using R = typename A::real;
     using L = typename A::level;
     SlotInA<A> in;
@@ -227,7 +241,7 @@ __device__ __forceinline__ void single_core(const DevMesh<A> &m, int r, int a, i
         BoundaryInA<A> bi;
         const int row = m.bcell[a];
         if (row >= 0) {
-            const size_t q = (size_t)si.jt * m.nb + row;
+            const size_t q = (size_t)p.jt * m.nb + row;
             bi.qt = m.bqt[q]; bi.dqt = m.bdqt[q]; bi.zt = m.bzt[q]; bi.dzt = m.bdzt[q];
             bi.top = m.btop[row]; bi.nhq1 = m.bnhq1[row];
             bi.zw = m.bzw + (size_t)row * m.nhq; bi.qw = m.bqw + (size_t)row * m.nhq;
@@ -253,255 +267,254 @@ __device__ __forceinline__ void single_core(const DevMesh<A> &m, int r, int a, i
     if (o.undefined) atomicOr(m.err, ERRBIT_UNDEFINED);
 }
 
+// A record's geometry, cells and slots.  fp64 records are one 256-bit load:
+// the fourth value of rgeo holds both slots (pack_slots: 4a + j in the low
+// word, 4b + j in the high one; a single's neighbour without a slot of its own
+// as 4b, none as all ones), and rix is not read by the step.
+__host__ __device__ inline unsigned long long pack_slots(int sa, int b, int sb) {
+    return (unsigned long long)(unsigned)(sb >= 0 ? sb : b < 0 ? -1 : 4 * b) << 32 | (unsigned)sa;
+}
+template <class A>
+struct Record {
+    Vec4<typename A::real> g;
+    int a, b, sa, sb;
+};
+template <class A>
+__device__ __forceinline__ Record<A> load_record(const DevMesh<A> &m, int r) {
+    Record<A> q;
+    q.g = ldg4(m.rgeo + 4 * (size_t)r);
+    if constexpr (std::is_same<typename A::real, double>::value) {
+        const unsigned long long w = (unsigned long long)__double_as_longlong(q.g.w);
+        q.sa = (int)(unsigned)w;
+        q.sb = (int)(unsigned)(w >> 32);
+        q.a = q.sa >> 2;
+        q.b = q.sb >> 2;
+    } else {
+        const int4 ix = m.rix[r];
+        q.a = ix.x; q.b = ix.y; q.sa = ix.z; q.sb = ix.w;
+    }
+    return q;
+}
+
+// One side of record r on its own: a single record's slot, or slot a
+// (item = 2r) or b (item = 2r + 1) of a pair, computed as the reference
+// computes every slot.
 template <class A, int VARIANT, class T>
-__device__ __forceinline__ void single_record(const DevMesh<A> &m, int r, const StepIndex &si,
-                                              const StepParams &p, int write_flux, const T &tout) {
-    using R = typename A::real;
-    using L = typename A::level;
-    const int4 ix = m.rix[r];
-    const Vec4<R> g = ldg4(m.rgeo + 4 * (size_t)r);
-    const uint8_t meta = m.rmeta[r];
-    const CellStateA<A> own = load_cell(m, si.par, ix.x);
-    const CellStateA<A> nb =
-        (meta & META_HAS_NB) ? load_cell(m, si.par, ix.y) : CellStateA<A>{R(0), R(0), R(0), L(0), L(0)};
-    single_core<A, VARIANT>(m, r, ix.x, ix.z, own, nb, meta, g, si, p, write_flux, tout);
-}
-
-// The mirrored Osher of a pair computed on its own (when its inputs differ
-// from the direct route's in the normal velocity); mirror_core takes the
-// pair's cells a (direct side) and b, its geometry and b's slot sb.
-template <class A, class T>
-__device__ __forceinline__ void mirror_core(const DevMesh<A> &m, const CellStateA<A> &A_, const CellStateA<A> &B_,
-                                            const Vec4<typename A::real> &g, int sb, const StepParams &p,
-                                            int write_flux, const T &tout) {
-    using R = typename A::real;
-    const R cs = g.x, sn = g.y;
-    const R clA = A::sqrt(A::mul(A::c(9.81), A_.h));
-    const OsherIn<R> oi = osher_inputs<A>(A_, B_, cs, sn, clA, true, p);
-    R fo[4], fb[4];
-    osher<A>(oi.cl, oi.ql, oi.qr, oi.fil, fo);
-    fb[0] = -fo[0];
-    fb[1] = osher_f1<A>(fo[1], oi.ratio, oi.hcR, oi.ur);
-    fb[2] = fo[2];
-    fb[3] = mirror_f3<A>(fo[3], A_.zbc, B_.zbc);
-    if (write_flux) store_flux(m, sb, fb);
-    store_terms<A>(tout, sb, fb, g.z, -cs, -sn);
-}
-
-template <class A, class T>
-__device__ __forceinline__ void pair_mirror(const DevMesh<A> &m, int r, const StepIndex &si,
+__device__ __forceinline__ void side_record(const DevMesh<A> &m, int item, const StepIndex &si,
                                             const StepParams &p, int write_flux, const T &tout) {
     using R = typename A::real;
-    const int4 ix = m.rix[r];
-    const Vec4<R> g = ldg4(m.rgeo + 4 * (size_t)r);
-    const CellStateA<A> A_ = load_cell(m, si.par, ix.x), B_ = load_cell(m, si.par, ix.y);
-    mirror_core<A>(m, A_, B_, g, ix.w, p, write_flux, tout);
+    using L = typename A::level;
+    const int r = item >> 1;
+    const bool other = item & 1;
+    const Record<A> q = load_record(m, r);
+    Vec4<R> g = q.g;
+    uint8_t meta = m.rmeta[r];
+    int c = q.a, n = q.b, s = q.sa;
+    if (other) {   // negated normal, not the lower-numbered side
+        c = q.b; n = q.a; s = q.sb;
+        g.x = -g.x; g.y = -g.y;
+        meta &= (uint8_t)~META_OWN_FIRST;
+    }
+    const CellStateA<A> own = load_cell(m, si.par, c);
+    const CellStateA<A> nb =
+        (meta & META_HAS_NB) ? load_cell(m, si.par, n) : CellStateA<A>{R(0), R(0), R(0), L(0), L(0)};
+    const bool timed = code_is_bounda((int8_t)(meta & META_CODE));
+    single_core<A, VARIANT>(m, r, c, s, own, nb, meta, g, timed ? with_time(p, si) : p, write_flux, tout);
 }
 
-template <class R>
-__device__ __forceinline__ bool same_bits(R a, R b) {
-    if constexpr (sizeof(R) == 8) return __double_as_longlong((double)a) == __double_as_longlong((double)b);
-    else return __float_as_int((float)a) == __float_as_int((float)b);
-}
-
-// One mirror-pair record.  It evaluates both slots' branch chains
-// (functors.cu:98-150) and, when both reach Osher, runs it once: the direct
-// route at a and the mirrored route at b have the same cells, normal and
-// inputs except two rotations that the reference build rounds differently.
-// When those agree bit for bit the two Osher evaluations are identical, and
-// the b side's FLUX2 is re-summed with its own tangent if only that differs;
-// otherwise the pair goes to the CTA's queue, whose mirrored Osher
-// evaluations run together after the main pass (pair_mirror).
-// pair_core takes both cells' states, the geometry of a's slot and the two
-// slots sa, sb; a pair whose mirrored Osher must run on its own is queued as
-// record r.  tslot stores the Osher trace and the tangents of a re-summed
-// FLUX2 (TRACE_VALUES values): SmemTrace, the thread's slot in shared memory
-// (the edge-layout kernels, whose registers are scarce), or RegTrace
-// (registers: the tile kernel, whose shared memory is).
-constexpr int TRACE_VALUES = 16;
-template <class R>
-struct SmemTrace {   // values at p[i * stride]
-    R *p;
-    int stride;
-    __device__ __forceinline__ void set(int i, R v) { p[i * stride] = v; }
-    __device__ __forceinline__ R get(int i) const { return p[i * stride]; }
-    // a value kept out of registers across a stretch of code: the volatile
-    // access makes the compiler read it back instead of holding it
-    __device__ __forceinline__ void park(int i, R v) { *(volatile R *)(p + i * stride) = v; }
-    __device__ __forceinline__ R unpark(int i) const { return *(volatile R *)(p + i * stride); }
-};
-template <class R>
-struct RegTrace {
-    R v[TRACE_VALUES];
-    __device__ __forceinline__ void set(int i, R x) { v[i] = x; }
-    __device__ __forceinline__ R get(int i) const { return v[i]; }
-    __device__ __forceinline__ void park(int i, R x) { v[i] = x; }
-    __device__ __forceinline__ R unpark(int i) const { return v[i]; }
-};
-
-template <class A, int VARIANT, class T, class TS>
-__device__ __forceinline__ void pair_core(const DevMesh<A> &m, int r, const CellStateA<A> &A_,
-                                          const CellStateA<A> &B_, const Vec4<typename A::real> &g, int sa, int sb,
-                                          const StepParams &p, int write_flux, const T &tout, int *queue, int *qn,
-                                          TS &tslot) {
+// One mirror-pair record: both sides' fluxes where both cells are deep and
+// the flow across the edge is subcritical (or both are dry), the bulk of any
+// mesh.  The two routes (functors.cu:151-200) have the same cells, normal and
+// inputs except two rotations that the reference build rounds differently
+// (policies with route_modes), so they share the square roots, the depth ratio
+// and their quotients, and each runs osher_subcritical from its own FIR.
+// Every other pair puts its two sides into the CTA's queue, which runs after
+// the main pass (side_record).  So the main pass holds neither the powers of
+// the one-sided branches nor Osher's other pieces.
+//
+// Bound by the gathers' latency and by issue.  207,234 cells, flux kernel, warp
+// instructions per launch: both branch chains, Osher in full and a queue of
+// mirrored evaluations 7.47 M; this form 4.0 M, and 3.0 M after its comparisons
+// were cut to those below.  Step 22.2 -> 15.9 -> 14.4 us, 2M-cell dam break
+// 181 -> 153 -> 148 us; with one-load records and their loads ahead of the
+// dependency wait 14.0 and 146 us.
+template <class A, class T>
+__device__ __forceinline__ void pair_record(const DevMesh<A> &m, int r, const Record<A> &q, const StepIndex &si,
+                                            const StepParams &p, int write_flux, const T &tout, int *queue, int *qn) {
     using R = typename A::real;
-    const int4 ix = make_int4(0, 0, sa, sb);
-    const R cs = g.x, sn = g.y;
-    const R clA = A::sqrt(A::mul(A::c(9.81), A_.h));
-    auto nofetch = []() { return BoundaryInA<A>{}; };
-    SlotInA<A> ia, ib;
-    ia.own = A_; ia.nb = B_; ia.has_nb = true; ia.own_first = true; ia.code = CODE_ZERO;
-    ia.cosj = cs; ia.sinj = sn; ia.side = g.z;
-    ib.own = B_; ib.nb = A_; ib.has_nb = true; ib.own_first = false; ib.code = CODE_ZERO;
-    ib.cosj = -cs; ib.sinj = -sn; ib.side = ia.side;
-    // each side's branch chain; a side whose fluxes are final is written at once
-    int ra_, rb_;
-    {
-        SlotOut<R> oa;
-        ra_ = flux_chain<A, VARIANT>(ia, clA, p, nofetch, oa);   // 0 or 1 (direct)
-        if (!ra_) {
-            if (write_flux) store_flux(m, ix.z, oa.f);
-            store_terms<A>(tout, ix.z, oa.f, g.z, cs, sn);
+    using L = typename A::level;
+    const CellStateA<A> a = load_cell(m, si.par, q.a), b = load_cell(m, si.par, q.b);
+    const R cs = q.g.x, sn = q.g.y, side = q.g.z;
+    // Deep enough for both branch chains (functors.cu:98-150) to reach Osher and
+    // for its inputs (osher_inputs) to take none of their bounds: both depths
+    // and QR[0] above HM1 and HM2 (so max(H, HM1) = H and QR[1] is not the
+    // thin-water value), the right level above its bed (so max(ZBC, Z) = Z),
+    // and each side's level above the other's bed (of which QR[0] > 0 is one).
+    const R HMX = A::c(fmax(p.hm1, p.hm2));
+    const R qr0 = A::depth(b.z, a.zbc);
+    if (a.h > HMX && b.h > HMX && qr0 > HMX && a.z > b.zbc && b.z >= b.zbc) {
+        const R cl = A::sqrt(A::mul(A::c(9.81), a.h)), cr = A::sqrt(A::mul(A::c(9.81), qr0));
+        const R ratio = A::fmin(A::div(b.h, qr0), A::c(1.5));
+        const R ql1 = A::dot(a.u, cs, a.v, sn, M_QL1), ql2 = A::dot(a.v, cs, -a.u, sn, M_QL2);
+        const R qr2 = A::dot(b.v, cs, -b.u, sn, M_QR2);
+        const R fil = A::add(ql1, A::mul(A::c(2.0), cl));
+        const R ur = A::dot(b.u, cs, b.v, sn, M_UR);
+        R fa[4], fb[4];
+        bool ok = osher_subcritical<A>(cl, cr, ql1, ql2, A::mul(ur, ratio), qr2, fil, fa);
+        R urm = ur;
+        if constexpr (A::route_modes) {
+            urm = A::dot(b.u, cs, b.v, sn, M_UR1);
+            ok &= osher_subcritical<A>(cl, cr, ql1, A::dot(a.v, cs, -a.u, sn, M_QL2M), A::mul(urm, ratio), qr2, fil, fb);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; i++) fb[i] = fa[i];
         }
+        if (ok) {
+            fa[1] = osher_f1<A>(fa[1], ratio, b.h, ur);
+            if (write_flux) store_flux(m, q.sa, fa);
+            store_terms<A>(tout, q.sa, fa, side, cs, sn);
+            fb[0] = -fb[0];
+            fb[1] = osher_f1<A>(fb[1], ratio, b.h, urm);
+            // mirror_f3
+            const L za = A::ladd(A::lvl(A::sqrt(A::divk_raw(fb[3], 4.905))), a.zbc);
+            const R hc3 = za > b.zbc ? A::depth(za, b.zbc) : R(0);
+            fb[3] = A::mul(A::mul(A::c(4.905), hc3), hc3);
+            if (write_flux) store_flux(m, q.sb, fb);
+            store_terms<A>(tout, q.sb, fb, side, -cs, -sn);
+            return;
+        }
+    } else if (a.h <= A::c(p.hm1) && b.h <= A::c(p.hm1)) {   // both dry (functors.cu:98-105)
+        const R f[4] = {R(0), R(0), R(0), R(0)};
+        if (write_flux) { store_flux(m, q.sa, f); store_flux(m, q.sb, f); }
+        store_terms<A>(tout, q.sa, f, side, cs, sn);
+        store_terms<A>(tout, q.sb, f, side, -cs, -sn);
+        return;
     }
-    {
-        SlotOut<R> ob;
-        rb_ = flux_chain<A, VARIANT>(ib, R(0), p, nofetch, ob);  // 0 or 2 (mirrored)
-        if (!rb_) {
-            if (write_flux) store_flux(m, ix.w, ob.f);
-            store_terms<A>(tout, ix.w, ob.f, g.z, -cs, -sn);
-        }
-    }
-    if (ra_ | rb_) {
-        // the two routes' inputs differ only in QL2, UR and so QR1 (osher_inputs)
-        const OsherIn<R> oi = osher_inputs<A>(A_, B_, cs, sn, clA, ra_ == 0, p);
-        // Everything the epilogues take besides Osher's result is formed first
-        // (same operations, same bits), so that few values stay live across
-        // Osher: FLUX1's correction of each side, whether b's mirrored Osher
-        // equals this one (QR1 agrees), and whether b's FLUX2 must be re-summed
-        // with its own tangent (only QL2 differs; the tangents and the
-        // per-piece products then wait in shared memory).
-        const R ur_m = ra_ ? A::dot(B_.u, cs, B_.v, sn, M_UR1) : oi.ur;
-        R qr1_m = A::mul(ur_m, oi.ratio);
-        if (oi.hcR <= A::c(p.hm2) || oi.qr[0] <= A::c(p.hm2)) qr1_m = A::copysign(A::c(K::VMIN), ur_m);
-        const bool b_same = rb_ && (!ra_ || same_bits(oi.qr[1], qr1_m));
-        const R ql2_m = ra_ ? A::dot(A_.v, cs, -A_.u, sn, M_QL2M) : oi.ql[2];
-        const bool b_resum = b_same && ra_ && !same_bits(oi.ql[2], ql2_m);
-        if (b_resum) { tslot.set(6, ql2_m); tslot.set(7, oi.qr[2]); }
-        // the epilogues' other inputs wait across Osher in the trace store too
-        // (read back afterwards rather than held in registers)
-        tslot.park(8, osher_f1_term<A>(oi.ratio, oi.hcR, oi.ur));   // FLUX1 term of side a
-        tslot.park(9, osher_f1_term<A>(oi.ratio, oi.hcR, ur_m));    // FLUX1 term of side b
-        tslot.park(10, cs);
-        tslot.park(11, sn);
-        tslot.park(12, g.z);
-        using L = typename A::level;
-        L zbcA = A_.zbc, zbcB = B_.zbc;
-        if constexpr (std::is_same<L, R>::value) { tslot.park(13, zbcA); tslot.park(14, zbcB); }
-        // the two slot indices wait in the trace store too (fp64: one 64-bit slot)
-        int psa = ix.z, psb = ix.w;
-        if constexpr (sizeof(R) == 8)
-            tslot.park(15, __longlong_as_double((long long)(((unsigned long long)(unsigned)psb << 32) | (unsigned)psa)));
-        R fo[4];
-        OsherTraceIn<TS> tr{&tslot, 0u, 0u};
-        osher<A>(oi.cl, oi.ql, oi.qr, oi.fil, fo, &tr);
-        const R pcs = tslot.unpark(10), psn = tslot.unpark(11), pside = tslot.unpark(12);
-        if constexpr (std::is_same<L, R>::value) { zbcA = tslot.unpark(13); zbcB = tslot.unpark(14); }
-        if constexpr (sizeof(R) == 8) {
-            const unsigned long long w = (unsigned long long)__double_as_longlong((double)tslot.unpark(15));
-            psa = (int)(unsigned)(w & 0xFFFFFFFFull);
-            psb = (int)(unsigned)(w >> 32);
-        }
-        if (ra_) {
-            R f[4];
-            f[0] = fo[0];
-            f[1] = A::add(fo[1], tslot.unpark(8));
-            f[2] = fo[2];
-            f[3] = fo[3];
-            if (write_flux) store_flux(m, psa, f);
-            store_terms<A>(tout, psa, f, pside, pcs, psn);
-        }
-        if (b_same) {
-            R f[4];
-            f[0] = -fo[0];
-            f[1] = A::add(fo[1], tslot.unpark(9));
-            f[2] = b_resum ? osher_f2<A>(tr, tslot.get(6), tslot.get(7)) : fo[2];
-            f[3] = mirror_f3<A>(fo[3], zbcA, zbcB);
-            if (write_flux) store_flux(m, psb, f);
-            store_terms<A>(tout, psb, f, pside, -pcs, -psn);
-        } else if (rb_) {
-            queue[atomicAdd(qn, 1)] = r;
-        }
-    }
+    const int i = atomicAdd(qn, 2);
+    queue[i] = 2 * r;
+    queue[i + 1] = 2 * r + 1;
 }
 
-template <class A, int VARIANT, class T, class TS>
-__device__ __forceinline__ void pair_record(const DevMesh<A> &m, int r, const StepIndex &si, const StepParams &p,
-                                            int write_flux, const T &tout, int *queue, int *qn, TS &tslot) {
+// One side of such an edge on its own (cell_kernel): pair_record's common case
+// for the slot of `own` that faces `nb`, by the direct or the mirrored route.
+// False, and no result, in any other case.
+template <class A>
+__device__ __forceinline__ bool slot_common(const CellStateA<A> &own, const CellStateA<A> &nb, bool own_first,
+                                            typename A::real cosj, typename A::real sinj, const StepParams &p,
+                                            typename A::real f[4]) {
     using R = typename A::real;
-    const int4 ix = m.rix[r];
-    const Vec4<R> g = ldg4(m.rgeo + 4 * (size_t)r);
-    const CellStateA<A> A_ = load_cell(m, si.par, ix.x), B_ = load_cell(m, si.par, ix.y);
-    pair_core<A, VARIANT>(m, r, A_, B_, g, ix.z, ix.w, p, write_flux, tout, queue, qn, tslot);
+    using L = typename A::level;
+    const CellStateA<A> &a = own_first ? own : nb, &b = own_first ? nb : own;
+    const R cs = own_first ? cosj : -cosj, sn = own_first ? sinj : -sinj;
+    const R HMX = A::c(fmax(p.hm1, p.hm2));
+    const R qr0 = A::depth(b.z, a.zbc);
+    if (!(a.h > HMX && b.h > HMX && qr0 > HMX && a.z > b.zbc && b.z >= b.zbc)) {
+        f[0] = f[1] = f[2] = f[3] = R(0);
+        return a.h <= A::c(p.hm1) && b.h <= A::c(p.hm1);   // both dry
+    }
+    const R cl = A::sqrt(A::mul(A::c(9.81), a.h)), cr = A::sqrt(A::mul(A::c(9.81), qr0));
+    const R ratio = A::fmin(A::div(b.h, qr0), A::c(1.5));
+    const R ql1 = A::dot(a.u, cs, a.v, sn, M_QL1);
+    const R ql2 = own_first ? A::dot(a.v, cs, -a.u, sn, M_QL2) : A::dot(a.v, cs, -a.u, sn, M_QL2M);
+    const R ur = own_first ? A::dot(b.u, cs, b.v, sn, M_UR) : A::dot(b.u, cs, b.v, sn, M_UR1);
+    const R qr2 = A::dot(b.v, cs, -b.u, sn, M_QR2);
+    const R fil = A::add(ql1, A::mul(A::c(2.0), cl));
+    if (!osher_subcritical<A>(cl, cr, ql1, ql2, A::mul(ur, ratio), qr2, fil, f)) return false;
+    f[1] = osher_f1<A>(f[1], ratio, b.h, ur);
+    if (!own_first) {
+        f[0] = -f[0];
+        const L za = A::ladd(A::lvl(A::sqrt(A::divk_raw(f[3], 4.905))), a.zbc);
+        const R hc3 = za > b.zbc ? A::depth(za, b.zbc) : R(0);
+        f[3] = A::mul(A::mul(A::c(4.905), hc3), hc3);
+    }
+    return true;
 }
 
 // Flux of every record of one step.  Single mesh (SEG = false): records
 // [0, npairs) are mirror pairs and the rest single slots, one per thread.
 // Batch (SEG = true): CTA b takes the scenario and record range of fseg[b].
-// SMEM_TRACE: the Osher trace in shared memory (fewer registers, more shared
-// memory per CTA) or in registers.
-template <class A, int VARIANT, int THREADS, int MINB, bool SEG, bool SMEM_TRACE = true>
+// Singles go through the queue as well, so side_record's code is there once.
+template <class A, int VARIANT, int THREADS, int MINB, bool SEG>
 __global__ void __launch_bounds__(THREADS, MINB) flux_kernel(DevMesh<A> m, int k, int write_flux) {
-    using R = typename A::real;
-    __shared__ int queue[THREADS];
+    __shared__ int queue[2 * THREADS];
     __shared__ int qn;
-    __shared__ R trace[SMEM_TRACE ? TRACE_VALUES * THREADS : 1];
-    auto tslot = [&]() {
-        if constexpr (SMEM_TRACE) return SmemTrace<R>{trace + threadIdx.x, THREADS};
-        else return RegTrace<R>{};
-    }();
     if (threadIdx.x == 0) qn = 0;
     int r;
     bool valid, pair;
     StepIndex si;
     StepParams p;
+    Record<A> q{};
+    // constant tables: read before the dependency wait
     if constexpr (SEG) {
-        const int4 d = m.fseg[blockIdx.x];   // constant tables: read before the dependency wait
+        const int4 d = m.fseg[blockIdx.x];
         const ScnParams sp = m.scn[d.x];
-        cudaGridDependencySynchronize();
-        cudaTriggerProgrammaticLaunchCompletion();
-        si = step_index(m, k, sp.per_day, sp.ndays);
-        p = StepParams{sp.hm1, sp.hm2, sp.jl, sp.dt, si.kt, si.jt};
         r = d.y + (int)threadIdx.x;
         valid = (int)threadIdx.x < d.z;
         pair = d.w != 0;
-    } else {
+        if (valid && pair) q = load_record(m, r);
         cudaGridDependencySynchronize();
         cudaTriggerProgrammaticLaunchCompletion();
-        si = step_index(m, k, m.per_day, m.ndays);
-        p = StepParams{m.hm1, m.hm2, m.jl, m.dt, si.kt, si.jt};
+        si = step_index(m, k, sp.per_day, sp.ndays);
+        p = StepParams{sp.hm1, sp.hm2, sp.jl, sp.dt, 1, 0};
+    } else {
         r = (m.rev_flux ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x) * THREADS + threadIdx.x;
         valid = r < m.nrecords;
         pair = r < m.npairs;
+        if (pair) q = load_record(m, r);
+        cudaGridDependencySynchronize();
+        cudaTriggerProgrammaticLaunchCompletion();
+        si = step_index(m, k, m.per_day, m.ndays);
+        p = StepParams{m.hm1, m.hm2, m.jl, m.dt, 1, 0};
     }
     __syncthreads();
     const Terms<typename A::real> tout{m.slotw, 0};
     if (valid) {
-        if (pair) pair_record<A, VARIANT>(m, r, si, p, write_flux, tout, queue, &qn, tslot);
-        else single_record<A, VARIANT>(m, r, si, p, write_flux, tout);
+        if (pair) pair_record<A>(m, r, q, si, p, write_flux, tout, queue, &qn);
+        else queue[atomicAdd(&qn, 1)] = 2 * r;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < qn; i += THREADS) pair_mirror<A>(m, queue[i], si, p, write_flux, tout);
+    for (int i = threadIdx.x; i < qn; i += THREADS) side_record<A, VARIANT>(m, queue[i], si, p, write_flux, tout);
+}
+
+// The fluxes of a cell's zero-length slot: the cell's state, no neighbour, zero
+// geometry, code 0.  The two-kernel step calls it out of line: it is rarely
+// needed, and its powers would take the cell kernel's registers.
+template <class R> struct ZeroSlot { R f[4]; };
+template <class A, int VARIANT>
+__device__ __forceinline__ ZeroSlot<typename A::real> zero_slot(const CellStateA<A> &st, const StepParams &p,
+                                                                int write_flux) {
+    using R = typename A::real;
+    using L = typename A::level;
+    SlotInA<A> in;
+    in.own = st;
+    in.nb = {R(0), R(0), R(0), L(0), L(0)};
+    in.has_nb = false; in.own_first = false; in.code = CODE_ZERO;
+    in.cosj = R(0); in.sinj = R(0); in.side = R(0);
+    auto nofetch = []() { return BoundaryInA<A>{}; };
+    SlotOut<R> o;
+    if (write_flux) flux_slot<A, VARIANT, decltype(nofetch), false>(in, A::sqrt(A::mul(A::c(9.81), st.h)), p, nofetch, o);
+    else flux_chain<A, VARIANT, decltype(nofetch), true>(in, R(0), p, nofetch, o);
+    return {{o.f[0], o.f[1], o.f[2], o.f[3]}};
+}
+template <class A, int VARIANT>
+__device__ __noinline__ ZeroSlot<typename A::real> zero_slot_call(const CellStateA<A> st, const StepParams p,
+                                                                  int write_flux) {
+    return zero_slot<A, VARIANT>(st, p, write_flux);
 }
 
 // Sums and update of one cell (UpdateCellKernel, functors.cu:717-784).  The
 // zero-length fourth slot of a triangle is evaluated here, without pow
 // (flux_slot's ZERO_LEN) unless fluxes are written out, and only where its
 // zero addends can change the sums.
-// SMEM_TERMS: `terms` is in shared memory (tile layout), else global.
+// TERMS: where `terms` is and when it is read.
 // update_core takes the cell's state and constants `in`, and two functions
 // that give its DT/AREA and its friction: a caller that formed them while it
 // waited for the terms returns them, others compute them where they are used.
+enum : int {
+    TERMS_GLOBAL = 0,      // edge layout: global memory, all read up front
+    TERMS_SMEM = 1,        // tile layout: shared memory, all read up front
+    TERMS_SMEM_LATE = 2    // cell_kernel: shared memory, each read where it is added (24 registers fewer)
+};
 template <class A>
 struct CellIn {
     Vec4<typename A::real> raw;         // the stored state record
@@ -509,38 +522,43 @@ struct CellIn {
     unsigned mask;
     typename A::real fnc, dta, sidex;   // dta: DT/AREA (variant H) or AREA (variant F)
 };
-template <class A, int VARIANT>
-__device__ __forceinline__ CellIn<A> load_cell_in(const DevMesh<A> &m, int par, int c) {
+// EARLY: ahead of the dependency wait; ZBC and FNC, which the adjoint's
+// parameters change between sequences, then come from L2.
+template <class A, int VARIANT, bool EARLY = false>
+__device__ __forceinline__ CellIn<A> load_cell_constants(const DevMesh<A> &m, int c) {
     using R = typename A::real;
     CellIn<A> in;
-    in.raw = ldg4(m.S[par] + 4 * (size_t)c);
-    in.zbc = m.zbc[c];
+    in.zbc = EARLY ? __ldcg(m.zbc + c) : m.zbc[c];
     in.mask = m.cmask[c];
-    in.fnc = m.fnc[c];
+    in.fnc = EARLY ? __ldcg(m.fnc + c) : m.fnc[c];
     in.dta = m.dta[c];
     in.sidex = VARIANT == 1 ? m.sidex[c] : R(0);
     return in;
 }
 
-template <class A, int VARIANT, bool COEF, bool SMEM_TERMS, class DtaOf, class FrictionOf>
+template <class A, int VARIANT, bool COEF, int TERMS, class DtaOf, class FrictionOf>
 __device__ __forceinline__ void update_core(const DevMesh<A> &m, int c, const CellIn<A> &cin, const StepIndex &si,
                                             const StepParams &p, int write_flux, const typename A::real *terms,
                                             const DtaOf &dta_of, const FrictionOf &friction_of) {
     using R = typename A::real;
     using L = typename A::level;
+    constexpr bool SMEM_TERMS = TERMS != TERMS_GLOBAL;
     const Vec4<R> raw = cin.raw;
     const unsigned mask = cin.mask;
     CellStateA<A> st;
     st.h = raw.x; st.u = raw.y; st.v = raw.z; st.zbc = cin.zbc;
     if constexpr (is_split<A>::value) st.z = split_level<A>(raw.x, raw.w, st.zbc);
     else st.z = raw.w;
-    // only the real slots' terms are read (a triangle's zero-length fourth
-    // slot is evaluated below and has none)
+    // A triangle's zero-length fourth slot is evaluated below and has no terms,
+    // so they are not read.  Any other slot's place is read without asking
+    // whether it is a real one (only a real slot's terms are used).
+    auto terms_of = [&](int j) { return SMEM_TERMS ? ld4(terms + 4 * j) : ldg4(terms + 4 * j); };
     Vec4<R> t[4];
+    if constexpr (TERMS != TERMS_SMEM_LATE) {
 #pragma unroll
-    for (int j = 0; j < 4; j++)
-        t[j] = !(mask & (1u << j)) ? Vec4<R>{R(0), R(0), R(0), R(0)}
-                                   : (SMEM_TERMS ? ld4(terms + 4 * j) : ldg4(terms + 4 * j));
+        for (int j = 0; j < 3; j++) t[j] = terms_of(j);
+        if (mask & 8u) t[3] = terms_of(3);
+    }
     // The slot sums in slot order j = 0..3.  A zero-length slot (a
     // triangle's fourth) adds SIDE*F0 = 0*F0 to WH and 0*(...) to WU and WV.
     // For a finite state (h > 0) its fluxes are finite, so each addend is a
@@ -560,6 +578,7 @@ __device__ __forceinline__ void update_core(const DevMesh<A> &m, int c, const Ce
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         if (mask & (1u << j)) {
+            if constexpr (TERMS == TERMS_SMEM_LATE) t[j] = terms_of(j);
             // F0 and SIDE for WH; the WU/WV increments were formed by the flux kernel
             wh = A::madd(t[j].w, t[j].x, wh, M_WH);
             wu = A::add(wu, t[j].y);
@@ -569,26 +588,18 @@ __device__ __forceinline__ void update_core(const DevMesh<A> &m, int c, const Ce
         }
     }
     if (need_zero) {
-        SlotInA<A> in;
-        in.own = st;
-        in.nb = {R(0), R(0), R(0), L(0), L(0)};
-        in.has_nb = false; in.own_first = false; in.code = CODE_ZERO;
-        in.cosj = R(0); in.sinj = R(0); in.side = R(0);
-        auto nofetch = []() { return BoundaryInA<A>{}; };
-        SlotOut<R> o;
+        const ZeroSlot<R> o =
+            SMEM_TERMS ? zero_slot<A, VARIANT>(st, p, write_flux) : zero_slot_call<A, VARIANT>(st, p, write_flux);
         if (write_flux) {
-            flux_slot<A, VARIANT, decltype(nofetch), false>(in, A::sqrt(A::mul(A::c(9.81), st.h)), p, nofetch, o);
 #pragma unroll
             for (int j = 0; j < 4; j++)
                 if (!(mask & (1u << j))) store_flux(m, 4 * c + j, o.f);
-        } else {
-            flux_chain<A, VARIANT, decltype(nofetch), true>(in, R(0), p, nofetch, o);
         }
         wh = R(0); wu = R(0); wv = R(0);
 #pragma unroll 1
         for (int j = 0; j < 4; j++) {
             if (mask & (1u << j)) {
-                const Vec4<R> tj = SMEM_TERMS ? ld4(terms + 4 * j) : ldg4(terms + 4 * j);
+                const Vec4<R> tj = terms_of(j);
                 wh = A::madd(tj.w, tj.x, wh, M_WH);
                 wu = A::add(wu, tj.y);
                 wv = A::add(wv, tj.z);
@@ -609,7 +620,8 @@ __device__ __forceinline__ void update_core(const DevMesh<A> &m, int c, const Ce
     else stg4(m.S[np] + 4 * (size_t)c, o.h, o.u, o.v, o.z);
     // W enters no step: only the last one of a sequence leaves it
     if (write_flux) m.W[c] = speed<A>(o.u, o.v);
-    if (!(isfinite((double)o.h) && isfinite((double)o.u) && isfinite((double)o.v))) atomicOr(m.err, ERRBIT_NONFINITE);
+    // (U and V are always finite: each is the smaller of its size and a bound)
+    if (!isfinite((double)o.h)) atomicOr(m.err, ERRBIT_NONFINITE);
     if constexpr (std::is_same<A, F64Exact>::value) {
         if (m.ckpt != nullptr) {
             const long long t1 = si.step + 1;
@@ -624,41 +636,53 @@ __device__ __forceinline__ void update_core(const DevMesh<A> &m, int c, const Ce
     }
 }
 
-template <class A, int VARIANT, bool COEF = false, bool SMEM_TERMS = false>
-__device__ __forceinline__ void update_one(const DevMesh<A> &m, int c, const StepIndex &si, const StepParams &p,
-                                           int write_flux, const typename A::real *terms) {
-    const CellIn<A> in = load_cell_in<A, VARIANT>(m, si.par, c);
-    update_core<A, VARIANT, COEF, SMEM_TERMS>(
+// The update of cell c from its constants `in` (load_cell_constants).
+template <class A, int VARIANT, bool COEF = false, int TERMS = TERMS_GLOBAL>
+__device__ __forceinline__ void update_one(const DevMesh<A> &m, int c, CellIn<A> in, const StepIndex &si,
+                                           const StepParams &p, int write_flux, const typename A::real *terms) {
+    in.raw = ldg4(m.S[si.par] + 4 * (size_t)c);
+    update_core<A, VARIANT, COEF, TERMS>(
         m, c, in, si, p, write_flux, terms,
         [&]() { return cell_dta<A, VARIANT>(in.raw.x, in.raw.y, in.dta, in.sidex, p); },
         [&]() { return cell_friction<A>(in.raw.x, in.raw.y, in.raw.z, in.fnc, p); });
 }
 
-// Every cell of one step.  Single mesh: a grid-stride loop over the cells.
-// Batch: CTA b takes the scenario and cell range of useg[b].  COEF: also the
-// update coefficients of the wet cells into m.ucoef.
+// Every cell of one step, one per thread.  Batch: CTA b takes the scenario and
+// cell range of useg[b].  COEF: also the update coefficients of the wet cells
+// into m.ucoef.
+//
+// Bound by issue (3.1 M warp instructions at 207,234 cells, half of them fp64
+// chains: a power, a square root and three quotients per cell) and by the tail:
+// 1,620 CTAs are 1.37 waves of 8 per SM and 1.82 of 6, and the step takes
+// 14.1 us with the first, 13.7 us with the second.  The constants' early loads:
+// 14.5 -> 14.1 us (8 per SM).
 template <class A, int VARIANT, int UMINB, bool SEG, bool COEF = false>
 __global__ void __launch_bounds__(UPDATE_THREADS, UMINB) update_kernel(DevMesh<A> m, int k, int write_flux) {
     // batches: the flux segments run forward, so the cells run reversed
     const bool rev = SEG ? m.rev_update != 0 : m.rev_flux == 0;
     const int blk = rev ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
+    int c, per_day, ndays;
+    bool on;
+    StepParams p;
     if constexpr (SEG) {
         const int4 d = m.useg[blk];
         const ScnParams sp = m.scn[d.x];
-        cudaGridDependencySynchronize();
-        cudaTriggerProgrammaticLaunchCompletion();
-        const StepIndex si = step_index(m, k, sp.per_day, sp.ndays);
-        const StepParams p{sp.hm1, sp.hm2, sp.jl, sp.dt, si.kt, si.jt};
-        const int c = d.y + (int)threadIdx.x;
-        if ((int)threadIdx.x < d.z) update_one<A, VARIANT, COEF>(m, c, si, p, write_flux, m.slotw + 16 * (size_t)c);
+        c = d.y + (int)threadIdx.x;
+        on = (int)threadIdx.x < d.z;
+        per_day = sp.per_day; ndays = sp.ndays;
+        p = StepParams{sp.hm1, sp.hm2, sp.jl, sp.dt, 1, 0};
     } else {
-        cudaGridDependencySynchronize();
-        cudaTriggerProgrammaticLaunchCompletion();
-        const StepIndex si = step_index(m, k, m.per_day, m.ndays);
-        const StepParams p{m.hm1, m.hm2, m.jl, m.dt, si.kt, si.jt};
-        for (int c = blk * UPDATE_THREADS + threadIdx.x; c < m.C; c += gridDim.x * UPDATE_THREADS)
-            update_one<A, VARIANT, COEF>(m, c, si, p, write_flux, m.slotw + 16 * (size_t)c);
+        c = blk * UPDATE_THREADS + (int)threadIdx.x;
+        on = c < m.C;
+        per_day = m.per_day; ndays = m.ndays;
+        p = StepParams{m.hm1, m.hm2, m.jl, m.dt, 1, 0};
     }
+    CellIn<A> in{};
+    if (on) in = load_cell_constants<A, VARIANT, true>(m, c);
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+    const StepIndex si = step_index(m, k, per_day, ndays);
+    if (on) update_one<A, VARIANT, COEF>(m, c, in, si, p, write_flux, m.slotw + 16 * (size_t)c);
 }
 
 // What a slot of cell_kernel needs besides its geometry, packed into the
@@ -694,12 +718,14 @@ struct SlotRef {
 // Same operations per slot and per cell, so the same bits as the two-kernel
 // step.  COEF as in update_kernel.
 //
-// Bound by that chain: of a 4.3 us step at 6,675 cells about 1.3 us is the
+// Bound by that chain: of a 3.9 us step at 6,675 cells about 1.3 us is the
 // launch and the state's way through L2, the rest dependent fp64 operations.
 // What shortened it there: one launch 8.4 -> 5.1 us; the update warp's early
-// work and the step index read ahead of the wait 5.1 -> 4.3 us.  96 slots per
-// CTA are 32 triangles, one update warp; 7 CTAs per SM hold 32,000 cells at
-// once (5.0 us; 7.0 us at 6 per SM).
+// work and the step index read ahead of the wait 5.1 -> 4.3 us; the common
+// case ahead of the general one (slot_common) 4.4 -> 3.9 us (it costs where
+// many warps hold both: a developed dam break at 24,021 cells 5.7 -> 6.7 us).
+// 96 slots per CTA are 32 triangles, one update warp; 7 CTAs per SM hold
+// 33,000 cells at once.
 constexpr int CELL_SLOTS = 96, CELL_MAX = 32, CELL_THREADS = CELL_SLOTS + CELL_MAX;
 constexpr int CELL_TERMS = 18;   // values per cell in shared memory: 4 slots x 4, padded off the bank period
 constexpr int CELL_CTAS = 7;     // CTAs per SM asked of the compiler
@@ -728,11 +754,16 @@ __global__ void __launch_bounds__(CELL_THREADS, CELL_CTAS) cell_kernel(DevMesh<A
             zb = __ldcg(m.zbc + d.x + (ref.place >> 2));
             if (ref.nb >= 0) zbn = __ldcg(m.zbc + ref.nb);
         }
+        StepParams p{m.hm1, m.hm2, m.jl, m.dt, 1, 0};
+        const bool timed = code_is_bounda((int8_t)(ref.meta & META_CODE));
+        if (k > 0 && timed) p = with_time(p, si);
         cudaGridDependencySynchronize();
         cudaTriggerProgrammaticLaunchCompletion();
-        if (k == 0) si = step_index(m, k, m.per_day, m.ndays);
+        if (k == 0) {
+            si = step_index(m, k, m.per_day, m.ndays);
+            if (timed) p = with_time(p, si);
+        }
         if (t < d.w) {
-            const StepParams p{m.hm1, m.hm2, m.jl, m.dt, si.kt, si.jt};
             const R *S = m.S[si.par];
             const int c = d.x + (ref.place >> 2), sa = 4 * d.x + ref.place;
             const Vec4<R> a = ldg4(S + 4 * (size_t)c);
@@ -744,25 +775,26 @@ __global__ void __launch_bounds__(CELL_THREADS, CELL_CTAS) cell_kernel(DevMesh<A
             uint8_t meta = ref.meta;
             if ((meta & META_CODE) == CODE_K7) meta = m.rmeta[ref.record];   // breached since?
             const Terms<R, true> tout{terms + CELL_TERMS * (ref.place >> 2) + 4 * (ref.place & 3), sa};
-            single_core<A, VARIANT>(m, ref.record, c, sa, CellStateA<A>{a.x, a.y, a.z, a.w, zb}, nb, meta, g, si, p,
-                                    write_flux, tout);
+            const CellStateA<A> own{a.x, a.y, a.z, a.w, zb};
+            R f[4];
+            if ((meta & META_CODE) == CODE_ZERO && (meta & META_HAS_NB) &&
+                slot_common<A>(own, nb, meta & META_OWN_FIRST, g.x, g.y, p, f)) {
+                if (write_flux) store_flux(m, sa, f);
+                store_terms<A>(tout, sa, f, g.z, g.x, g.y);
+            } else {
+                single_core<A, VARIANT>(m, ref.record, c, sa, own, nb, meta, g, p, write_flux, tout);
+            }
         }
         __syncthreads();
     } else {
         const int i = t - CELL_SLOTS, c = d.x + i;
         const bool on = i < d.y;
         CellIn<A> in{};
-        if (on) {
-            in.zbc = __ldcg(m.zbc + c);
-            in.mask = m.cmask[c];
-            in.fnc = __ldcg(m.fnc + c);
-            in.dta = m.dta[c];
-            in.sidex = VARIANT == 1 ? m.sidex[c] : R(0);
-        }
+        if (on) in = load_cell_constants<A, VARIANT, true>(m, c);
         cudaGridDependencySynchronize();
         cudaTriggerProgrammaticLaunchCompletion();
         if (k == 0) si = step_index(m, k, m.per_day, m.ndays);
-        const StepParams p{m.hm1, m.hm2, m.jl, m.dt, si.kt, si.jt};
+        const StepParams p{m.hm1, m.hm2, m.jl, m.dt, 1, 0};
         // a cell that is shallow now rarely needs its friction: it is formed late if it does
         Friction<R> f{R(0), R(0), R(0)};
         R dta = R(0);
@@ -776,7 +808,7 @@ __global__ void __launch_bounds__(CELL_THREADS, CELL_CTAS) cell_kernel(DevMesh<A
         }
         __syncthreads();
         if (on)
-            update_core<A, VARIANT, COEF, true>(m, c, in, si, p, write_flux, terms + CELL_TERMS * i,
+            update_core<A, VARIANT, COEF, TERMS_SMEM_LATE>(m, c, in, si, p, write_flux, terms + CELL_TERMS * i,
                                                 [&]() { return dta; },
                                                 [&]() { return ready ? f : friction(); });
     }
@@ -801,20 +833,20 @@ __global__ void __launch_bounds__(THREADS, MINB) tile_kernel(DevMesh<A> m, int k
     cudaGridDependencySynchronize();
     cudaTriggerProgrammaticLaunchCompletion();
     const StepIndex si = step_index(m, k, sp.per_day, sp.ndays);
-    const StepParams p{sp.hm1, sp.hm2, sp.jl, sp.dt, si.kt, si.jt};
+    const StepParams p{sp.hm1, sp.hm2, sp.jl, sp.dt, 1, 0};
     const Terms<R, true> tout{terms, 4 * td.cell0};
     __syncthreads();
     const int nrec = td.npairs + td.nsingles;
     for (int i = threadIdx.x; i < nrec; i += THREADS) {
-        RegTrace<R> tslot;
-        if (i < td.npairs) pair_record<A, VARIANT>(m, td.rec0 + i, si, p, write_flux, tout, queue, &qn, tslot);
-        else single_record<A, VARIANT>(m, td.rec0 + i, si, p, write_flux, tout);
+        if (i < td.npairs) pair_record<A>(m, td.rec0 + i, load_record(m, td.rec0 + i), si, p, write_flux, tout, queue, &qn);
+        else queue[atomicAdd(&qn, 1)] = 2 * (td.rec0 + i);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < qn; i += THREADS) pair_mirror<A>(m, queue[i], si, p, write_flux, tout);
+    for (int i = threadIdx.x; i < qn; i += THREADS) side_record<A, VARIANT>(m, queue[i], si, p, write_flux, tout);
     __syncthreads();
     for (int c = threadIdx.x; c < td.cells; c += THREADS)
-        update_one<A, VARIANT, false, true>(m, td.cell0 + c, si, p, write_flux, terms + 16 * c);
+        update_one<A, VARIANT, false, TERMS_SMEM>(m, td.cell0 + c, load_cell_constants<A, VARIANT>(m, td.cell0 + c), si, p,
+                                            write_flux, terms + 16 * c);
 }
 
 // ---------------------------------------------------------------------------
@@ -887,22 +919,20 @@ template <class A, int VARIANT, int THREADS, int MINB, bool SEG>
 __global__ void __launch_bounds__(THREADS, MINB)
     persistent_kernel(DevMesh<A> m, int n, int nflux, int ncell, unsigned *bar, unsigned phantom,
                       unsigned long long limit_ns) {
-    // The mirrored-Osher queue collects the pairs of several chunks and is run
-    // when it could not take another chunk's worth, and at the end of the flux
-    // phase: one block barrier per chunk instead of three.  Every queued pair
-    // is run before the grid barrier, as flux_kernel runs it before it ends.
+    // The queue of sides collects those of several chunks and is run when it
+    // could not take another chunk's worth, and at the end of the flux phase:
+    // one block barrier per chunk instead of three.  Every queued side is run
+    // before the grid barrier, as flux_kernel runs it before it ends.
     constexpr int QCAP = 4 * THREADS;
     __shared__ int queue[QCAP];
     __shared__ int qn;
-    __shared__ typename A::real trace[TRACE_VALUES * THREADS];
-    SmemTrace<typename A::real> tslot{trace + threadIdx.x, THREADS};
     const Terms<typename A::real> tout{m.slotw, 0};
     unsigned arrivals = 0;
     if (threadIdx.x == 0) qn = 0;
     __syncthreads();
     auto run_queue = [&](const StepIndex &si, const StepParams &p, int wf) {   // all threads; empties the queue
         const int nq = qn;
-        for (int i = threadIdx.x; i < nq; i += THREADS) pair_mirror<A>(m, queue[i], si, p, wf, tout);
+        for (int i = threadIdx.x; i < nq; i += THREADS) side_record<A, VARIANT>(m, queue[i], si, p, wf, tout);
         __syncthreads();
         if (threadIdx.x == 0) qn = 0;
         __syncthreads();
@@ -913,7 +943,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
         StepParams p0{};
         if constexpr (!SEG) {
             si0 = step_index(m, k, m.per_day, m.ndays);
-            p0 = StepParams{m.hm1, m.hm2, m.jl, m.dt, si0.kt, si0.jt};
+            p0 = StepParams{m.hm1, m.hm2, m.jl, m.dt, 1, 0};
         }
         for (int b = blockIdx.x; b < nflux; b += gridDim.x) {
             int r0, cnt;
@@ -924,7 +954,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
                 const int4 d = m.fseg[b];
                 const ScnParams sp = m.scn[d.x];
                 si = step_index(m, k, sp.per_day, sp.ndays);
-                p = StepParams{sp.hm1, sp.hm2, sp.jl, sp.dt, si.kt, si.jt};
+                p = StepParams{sp.hm1, sp.hm2, sp.jl, sp.dt, 1, 0};
                 r0 = d.y;
                 cnt = d.z;
                 seg_pairs = d.w != 0;
@@ -935,13 +965,13 @@ __global__ void __launch_bounds__(THREADS, MINB)
             if ((int)threadIdx.x < cnt) {
                 const int r = r0 + (int)threadIdx.x;
                 const bool pair = SEG ? seg_pairs : r < m.npairs;
-                if (pair) pair_record<A, VARIANT>(m, r, si, p, wf, tout, queue, &qn, tslot);
-                else single_record<A, VARIANT>(m, r, si, p, wf, tout);
+                if (pair) pair_record<A>(m, r, load_record(m, r), si, p, wf, tout, queue, &qn);
+                else queue[atomicAdd(&qn, 1)] = 2 * r;
             }
             __syncthreads();   // the queue's count is complete
-            // a batch chunk's pairs have their scenario's parameters: its queue
+            // a batch chunk's sides have their scenario's parameters: its queue
             // runs at once; a single mesh's when another chunk might not fit
-            if (SEG || qn > QCAP - THREADS) run_queue(si, p, wf);
+            if (SEG || qn > QCAP - 2 * THREADS) run_queue(si, p, wf);
         }
         if constexpr (!SEG) run_queue(si0, p0, wf);
         arrivals += gridDim.x;
@@ -954,17 +984,18 @@ __global__ void __launch_bounds__(THREADS, MINB)
                 const int4 d = m.useg[b];
                 const ScnParams sp = m.scn[d.x];
                 si = step_index(m, k, sp.per_day, sp.ndays);
-                p = StepParams{sp.hm1, sp.hm2, sp.jl, sp.dt, si.kt, si.jt};
+                p = StepParams{sp.hm1, sp.hm2, sp.jl, sp.dt, 1, 0};
                 c0 = d.y;
                 cnt = d.z;
             } else {
                 si = step_index(m, k, m.per_day, m.ndays);
-                p = StepParams{m.hm1, m.hm2, m.jl, m.dt, si.kt, si.jt};
+                p = StepParams{m.hm1, m.hm2, m.jl, m.dt, 1, 0};
                 c0 = b * UPDATE_THREADS;
                 cnt = min(UPDATE_THREADS, m.C - c0);
             }
             for (int i = threadIdx.x; i < cnt; i += THREADS)
-                update_one<A, VARIANT>(m, c0 + i, si, p, wf, m.slotw + 16 * (size_t)(c0 + i));
+                update_one<A, VARIANT>(m, c0 + i, load_cell_constants<A, VARIANT>(m, c0 + i), si, p, wf,
+                                       m.slotw + 16 * (size_t)(c0 + i));
         }
         if (k + 1 < n) {
             arrivals += gridDim.x;

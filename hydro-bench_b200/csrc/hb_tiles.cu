@@ -8,8 +8,8 @@
 
 namespace {
 
-size_t tile_smem_bytes(int max_cells, int max_pairs, size_t real_size) {
-    return 16 * real_size * (size_t)max_cells + sizeof(int) * (size_t)max_pairs;
+size_t tile_smem_bytes(int max_cells, int max_queue, size_t real_size) {
+    return 16 * real_size * (size_t)max_cells + sizeof(int) * (size_t)max_queue;
 }
 
 // Calls f(kernel, threads) with the tile kernel of a tile-layout launch shape.
@@ -39,7 +39,7 @@ int launch_tiles_t(hb_handle *h, hb::DevMesh<A> m, int n, cudaStream_t st) {
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cfg.dynamicSmemBytes = tile_smem_bytes(m.max_tile_cells, m.max_tile_pairs, sizeof(typename A::real));
+    cfg.dynamicSmemBytes = tile_smem_bytes(m.max_tile_cells, m.max_tile_queue, sizeof(typename A::real));
     const int rc = with_tile_kernel<A, VARIANT>(h->launch_config, [&](auto kernel, int threads) -> int {
         cfg.blockDim = dim3(threads);
         for (int k = 0; k < n; k++) HB_CUDA_RET(cudaLaunchKernelEx(&cfg, kernel, m, k, (int)(k == n - 1)));
@@ -53,7 +53,7 @@ int launch_tiles_t(hb_handle *h, hb::DevMesh<A> m, int n, cudaStream_t st) {
 // largest tile needs (beyond the 48 KB default).
 template <class A, int VARIANT>
 int set_tile_smem(const hb::DevMesh<A> &m) {
-    const size_t bytes = tile_smem_bytes(m.max_tile_cells, m.max_tile_pairs, sizeof(typename A::real));
+    const size_t bytes = tile_smem_bytes(m.max_tile_cells, m.max_tile_queue, sizeof(typename A::real));
     for (int c = 0; c < hb::N_LAUNCH_CONFIGS; c++) {
         if (hb::LAUNCH_CONFIGS[c].layout != hb::LAYOUT_TILE) continue;
         const int rc = with_tile_kernel<A, VARIANT>(c, [&](auto kernel, int) -> int {
@@ -77,12 +77,12 @@ int hb_tiles_launch(hb_handle *h, int n, cudaStream_t st) {
 
 int hb_tiles_resident(hb_handle *h, int config, int tile_cells, int *per_sm) {
     const bool f = h->opt.variant == HB_VARIANT_F;
-    // shared memory of a tile of up to 5/4 tile_cells cells, with as many
-    // mirror pairs as its slots could form (an upper bound)
+    // shared memory of a tile of up to 5/4 tile_cells cells, with every slot
+    // of its triangles in the queue
     const int cells = 5 * tile_cells / 4 + 1;
     return h->with_mesh([&](auto &m) -> int {
         using A = typename std::remove_reference<decltype(m)>::type::Policy;
-        const size_t bytes = tile_smem_bytes(cells, 2 * cells, sizeof(typename A::real));
+        const size_t bytes = tile_smem_bytes(cells, 3 * cells, sizeof(typename A::real));
         auto query = [&](auto kernel, int threads) -> int {
             HB_CUDA_RET(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
             HB_CUDA_RET(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, threads, bytes));

@@ -46,7 +46,7 @@ typedef enum { HB_VARIANT_H = 0, HB_VARIANT_F = 1 } hb_variant;
 typedef enum { HB_FP64 = 0, HB_FP32 = 1, HB_SPLIT = 2 } hb_precision;
 /* HB_LAYOUT_EDGE: two kernels per step, one thread per flux record then one
  * per cell, with the slots' terms of the cell sums passed through device
- * memory (single fp64 meshes of up to 120,000 cells at the default launch
+ * memory (single fp64 meshes of up to about 33,000 cells at the default launch
  * shape: one kernel, each slot computed from its own side).  HB_LAYOUT_TILE:
  * one kernel per step; the cells are grouped into
  * compact tiles of about tile_cells cells, and one CTA computes every flux of
