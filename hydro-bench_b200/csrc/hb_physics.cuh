@@ -138,9 +138,22 @@ struct F32Fast {
     static __device__ __forceinline__ float add(float a, float b) { return a + b; }
     static __device__ __forceinline__ float sub(float a, float b) { return a - b; }
     static __device__ __forceinline__ float div(float a, float b) { return a / b; }
-    static __device__ __forceinline__ float divk(float x, double c) { return x / (float)c; }
-    static __device__ __forceinline__ float divk_raw(float x, double c) { return x / (float)c; }
-    static __device__ __forceinline__ bool quotient_range(float) { return true; }
+    // as F64Exact::divk: e <= 2^-25 for every constant here, and every fp32
+    // significand gives the rounded quotient (checked one by one)
+    static __device__ __forceinline__ float divk(float x, double c) {
+        const unsigned e = ((unsigned)__float_as_int(x) & 0x7FFFFFFFu) - ((127u - 60u) << 23);
+        if (e < (120u << 23)) return divk_raw(x, c);
+        return x / (float)c;
+    }
+    static __device__ __forceinline__ float divk_raw(float x, double c) {
+        const float cf = (float)c, y = 1.0f / cf;
+        const float q = __fmul_rn(x, y);
+        return __fmaf_rn(__fmaf_rn(-q, cf, x), y, q);
+    }
+    // x >= 0 is within [2^-15, 2^15)
+    static __device__ __forceinline__ bool quotient_range(float x) {
+        return (unsigned)__float_as_int(x) - ((127u - 15u) << 23) < (30u << 23);
+    }
     static __device__ __forceinline__ bool nonnegative(float x) { return x >= 0.f; }
     static __device__ __forceinline__ float fma(float a, float b, float c) { return fmaf(a, b, c); }
     static __device__ __forceinline__ float sqrt(float a) { return sqrtf(a); }

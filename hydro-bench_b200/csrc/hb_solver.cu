@@ -575,7 +575,7 @@ int build_device_mesh(hb_handle *h, const hb_mesh_desc *mds, int n, hb::DevMesh<
             for (const auto &td : sc.tiles) {
                 tiles.push_back(td);
                 m.max_tile_cells = std::max(m.max_tile_cells, td.cells);
-                m.max_tile_queue = std::max(m.max_tile_queue, 2 * td.npairs + td.nsingles);
+                m.max_tile_queue = std::max(m.max_tile_queue, 2 * td.npairs);
             }
         m.ntiles = (int)tiles.size();
         hb::TileDesc *tp;
@@ -730,13 +730,14 @@ int enqueue_steps(hb_handle *h, int n, cudaStream_t st) {
     });
 }
 
-int default_config(int layout) {
-    return layout == HB_LAYOUT_TILE ? hb::DEFAULT_TILE_CONFIG : hb::DEFAULT_EDGE_CONFIG;
+int default_config(int layout, int precision) {
+    if (layout != HB_LAYOUT_TILE) return hb::DEFAULT_EDGE_CONFIG;
+    return precision == HB_FP64 ? hb::DEFAULT_TILE_CONFIG_FP64 : hb::DEFAULT_TILE_CONFIG;
 }
 
 // launch shape index of tile_config (0 = the layout's default), or -1
-int config_for(int layout, int tile_config) {
-    if (tile_config == 0) return default_config(layout);
+int config_for(int layout, int precision, int tile_config) {
+    if (tile_config == 0) return default_config(layout, precision);
     if (tile_config < 0 || tile_config > hb::N_LAUNCH_CONFIGS) return -1;
     return hb::LAUNCH_CONFIGS[tile_config - 1].layout == layout ? tile_config - 1 : -1;
 }
@@ -831,11 +832,11 @@ extern "C" int hb_create_batch(const hb_mesh_desc *meshes, int32_t n, const hb_o
         return hb::set_error(HB_E_INVALID, "hb_create: layout %d", opt.layout);
     if (opt.tile_cells < 0 || opt.tile_cells > 1024)   // 5/4 x 1024 fp64 cells: 160 KB of shared memory
         return hb::set_error(HB_E_INVALID, "hb_create: tile_cells %d outside 0..1024", opt.tile_cells);
-    if (config_for(opt.layout, opt.tile_config) < 0)
+    if (config_for(opt.layout, opt.precision, opt.tile_config) < 0)
         return hb::set_error(HB_E_INVALID, "hb_create: tile_config %d is no shape of layout %d", opt.tile_config, opt.layout);
     if (opt.persistent != 0 && opt.persistent != 1)
         return hb::set_error(HB_E_INVALID, "hb_create: persistent %d", opt.persistent);
-    if (opt.persistent && (opt.layout != HB_LAYOUT_EDGE || config_for(opt.layout, opt.tile_config) != hb::DEFAULT_EDGE_CONFIG))
+    if (opt.persistent && (opt.layout != HB_LAYOUT_EDGE || config_for(opt.layout, opt.precision, opt.tile_config) != hb::DEFAULT_EDGE_CONFIG))
         return hb::set_error(HB_E_INVALID, "hb_create: a persistent handle takes the edge layout's default launch shape");
     long long total = 0;
     for (int s = 0; s < n; s++) total += std::max(meshes[s].cells, 0);
@@ -843,7 +844,7 @@ extern "C" int hb_create_batch(const hb_mesh_desc *meshes, int32_t n, const hb_o
     HB_CUDA_RET(cudaSetDevice(opt.device));
     auto h = new hb_handle();
     h->opt = opt;
-    h->launch_config = config_for(opt.layout, opt.tile_config);
+    h->launch_config = config_for(opt.layout, opt.precision, opt.tile_config);
     h->tile_cells = opt.tile_cells > 0 ? opt.tile_cells : 256;
     if (opt.layout == HB_LAYOUT_TILE && opt.tile_cells == 0 && opt.precision != HB_FP64) {
         // balanced default (fp32 state): about 512 cells per tile, adjusted so
@@ -1174,7 +1175,7 @@ extern "C" int hb_get_permutation_at(hb_handle *h, int32_t s, int32_t *perm) {
 
 extern "C" int hb_set_tile_config(hb_handle *h, int32_t tile_config) {
     if (!h) return hb::set_error(HB_E_INVALID, "null handle");
-    const int c = config_for(h->opt.layout, tile_config);
+    const int c = config_for(h->opt.layout, h->opt.precision, tile_config);
     if (c < 0) return hb::set_error(HB_E_INVALID, "tile_config %d is no shape of this handle's layout", tile_config);
     if (h->opt.persistent && c != hb::DEFAULT_EDGE_CONFIG)
         return hb::set_error(HB_E_INVALID, "a persistent handle keeps the default launch shape");

@@ -33,7 +33,13 @@ constexpr LaunchConfig LAUNCH_CONFIGS[] = {
     {LAYOUT_TILE, 256, 5, 0}};
 constexpr int N_LAUNCH_CONFIGS = sizeof(LAUNCH_CONFIGS) / sizeof(LAUNCH_CONFIGS[0]);
 constexpr int DEFAULT_EDGE_CONFIG = 0;
-constexpr int DEFAULT_TILE_CONFIG = 8;
+// Tile layout, fp32 and split: 256 threads, 4 CTAs per SM (64 registers, no
+// spills).  us per step against 3 per SM, each with its own balanced tiles:
+// split 207,234 cells 9.3 / 9.8, 500,001-cell dam break 21.4 / 23.5, 1,000,000
+// cells 43.0 / 49.2, 64 scenarios of 3.8 M cells 147 / 174; fp32 120,000 cells
+// 6.9 / 7.3; it loses on about 60,000 cells (5.75 / 5.60).  fp64, whose tile
+// kernel spills below 80 registers: 20.2 at 3 per SM, 22.6 at 4 (207,234).
+constexpr int DEFAULT_TILE_CONFIG = 13, DEFAULT_TILE_CONFIG_FP64 = 8;
 constexpr int UPDATE_THREADS = 128;
 
 // One tile of the tile layout: a compact group of cells, contiguous in the
@@ -114,7 +120,7 @@ struct DevMesh {
     int rev_flux, rev_update;
     // tile layout
     const TileDesc *tiles;     // [ntiles]
-    int ntiles, max_tile_cells, max_tile_queue;   // the largest tile's cells and queue entries (2 per pair, 1 per single)
+    int ntiles, max_tile_cells, max_tile_queue;   // the largest tile's cells and queue entries (2 per pair)
 };
 
 // One step: the state buffer it reads, its number, and its scenario's table
@@ -820,6 +826,18 @@ __global__ void __launch_bounds__(CELL_THREADS, CELL_CTAS) cell_kernel(DevMesh<A
 // single records, computed by each tile for its own slot as the reference
 // computes every slot; the state of the neighbour across is read from global
 // memory, where the previous step (the previous launch) left it.
+//
+// The next pair's record is loaded while one is computed; the first one, the
+// step index and the first cell's constants are loaded ahead of what they
+// would wait behind.
+//
+// A 207,234-cell mesh is one wave of 443 CTAs, three to an SM, bound by issue
+// (half of the cycles) and the latencies of its phases.  us per step, split
+// precision, 207,234-cell channel / 500,001-cell dam break, and fp32, 61,003
+// mixed cells: 13.0 / 29.3 / 7.0 before pair_record's common case, 10.4 / 24.8 /
+// 5.8 with it, 10.0 / 23.5 / 5.8 with the next record's load, 9.8 / 23.5 / 5.6
+// with the early loads.  Chunks of 32 pairs drawn from a counter: 10.6 / 25.4 /
+// 5.8.
 template <class A, int VARIANT, int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) tile_kernel(DevMesh<A> m, int k, int write_flux) {
     using R = typename A::real;
@@ -830,23 +848,34 @@ __global__ void __launch_bounds__(THREADS, MINB) tile_kernel(DevMesh<A> m, int k
     const TileDesc td = m.tiles[blockIdx.x];   // constant tables: read before the dependency wait
     const ScnParams sp = m.scn[td.scn];
     if (threadIdx.x == 0) qn = 0;
+    Record<A> next{};
+    if ((int)threadIdx.x < td.npairs) next = load_record(m, td.rec0 + threadIdx.x);
+    StepIndex si;
+    if (k > 0) si = step_index<true>(m, k, sp.per_day, sp.ndays);   // as cell_kernel
     cudaGridDependencySynchronize();
     cudaTriggerProgrammaticLaunchCompletion();
-    const StepIndex si = step_index(m, k, sp.per_day, sp.ndays);
+    if (k == 0) si = step_index(m, k, sp.per_day, sp.ndays);
     const StepParams p{sp.hm1, sp.hm2, sp.jl, sp.dt, 1, 0};
     const Terms<R, true> tout{terms, 4 * td.cell0};
     __syncthreads();
-    const int nrec = td.npairs + td.nsingles;
-    for (int i = threadIdx.x; i < nrec; i += THREADS) {
-        if (i < td.npairs) pair_record<A>(m, td.rec0 + i, load_record(m, td.rec0 + i), si, p, write_flux, tout, queue, &qn);
-        else queue[atomicAdd(&qn, 1)] = 2 * (td.rec0 + i);
+    for (int i = threadIdx.x; i < td.npairs; i += THREADS) {
+        const Record<A> q = next;
+        if (i + THREADS < td.npairs) next = load_record(m, td.rec0 + i + THREADS);
+        pair_record<A>(m, td.rec0 + i, q, si, p, write_flux, tout, queue, &qn);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < qn; i += THREADS) side_record<A, VARIANT>(m, queue[i], si, p, write_flux, tout);
+    // the singles and the queued sides
+    const int sides = td.nsingles + qn;
+    for (int j = threadIdx.x; j < sides; j += THREADS)
+        side_record<A, VARIANT>(m, j < td.nsingles ? 2 * (td.rec0 + td.npairs + j) : queue[j - td.nsingles], si, p,
+                                write_flux, tout);
+    CellIn<A> in{};
+    if ((int)threadIdx.x < td.cells) in = load_cell_constants<A, VARIANT>(m, td.cell0 + threadIdx.x);
     __syncthreads();
-    for (int c = threadIdx.x; c < td.cells; c += THREADS)
-        update_one<A, VARIANT, false, TERMS_SMEM>(m, td.cell0 + c, load_cell_constants<A, VARIANT>(m, td.cell0 + c), si, p,
-                                            write_flux, terms + 16 * c);
+    for (int c = threadIdx.x; c < td.cells; c += THREADS) {
+        if (c != (int)threadIdx.x) in = load_cell_constants<A, VARIANT>(m, td.cell0 + c);
+        update_one<A, VARIANT, false, TERMS_SMEM>(m, td.cell0 + c, in, si, p, write_flux, terms + 16 * c);
+    }
 }
 
 // ---------------------------------------------------------------------------
