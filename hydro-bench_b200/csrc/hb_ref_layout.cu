@@ -1,7 +1,7 @@
 // hb_ref_layout.cu -- CalculateFlux / UpdateCell over the caller's own arrays
 // in the reference layout (functors.cu:787-818).  One thread per slot for the
-// flux, one per cell for the update, like the reference; the arithmetic is the
-// shared physics of hb_physics.cuh.
+// flux (sorted within the block by what a slot needs), one per cell for the
+// update; the arithmetic is the shared physics of hb_physics.cuh.
 #include "hb_common.cuh"
 #include "hb_physics.cuh"
 #include "hydrob200_refview.h"
@@ -17,11 +17,10 @@ struct RefView<double> { using type = hb_ref_mesh_view; };
 template <>
 struct RefView<float> { using type = hb_ref_mesh_view_f32; };
 
+// One slot in general, CalculateFluxKernel's body (functors.cu:47-202).
 template <class A, int VARIANT>
-__global__ void __launch_bounds__(256) ref_flux_kernel(typename RefView<typename A::real>::type m, int kt, int jt) {
+__device__ __forceinline__ void ref_slot(const typename RefView<typename A::real>::type &m, int idx, int kt, int jt) {
     using R = typename A::real;
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= 4 * m.CELL) return;
     const int pos = idx >> 2;
     const auto &c = m.cells;
     const auto &sd = m.sides;
@@ -59,35 +58,146 @@ __global__ void __launch_bounds__(256) ref_flux_kernel(typename RefView<typename
     if (o.mask & 8) sd.FLUX3[idx] = o.f[3];
 }
 
-template <class A, int VARIANT>
-__global__ void __launch_bounds__(256) ref_update_kernel(typename RefView<typename A::real>::type m) {
+// A slot without neighbour and code 0, as a rule a triangle's zero-length
+// fourth slot: the branch the chain takes for a wet cell above a bed at or
+// above zero (ZC = 0 <= ZBC, functors.cu:112-117), or the dry one.  False, and
+// no result, in any other case.
+template <class A>
+__device__ __forceinline__ bool closed_common(const CellStateA<A> &own, typename A::real cs, typename A::real sn,
+                                              const StepParams &p, typename A::real f[4]) {
     using R = typename A::real;
-    const int pos = blockIdx.x * blockDim.x + threadIdx.x;
+    f[0] = f[1] = f[2] = f[3] = R(0);
+    if (own.h <= A::c(p.hm1)) return p.hm1 >= 0.0;   // both depths at most HM1: no neighbour counts as 0
+    if (!(own.z > R(0) && R(0) <= own.zbc)) return false;
+    const R ql1 = A::dot(own.u, cs, own.v, sn, M_QL1), ql2 = A::dot(own.v, cs, -own.u, sn, M_QL2);
+    f[0] = A::mul(A::c(K::C1), A::pow(own.h, A::c(1.5)));
+    const R ha = A::mul(own.h, A::fabs(ql1));
+    f[1] = A::mul(ha, ql1);
+    f[2] = A::mul(ha, ql2);
+    return true;
+}
+
+// One slot per thread, sorted within the block: the interior slots with code 0
+// to the front threads, those without neighbour (a quarter of a triangle mesh's
+// slots, one in every group of four lanes, whose flux takes a power) to the
+// last ones, so that a warp runs one of the two common cases (slot_common,
+// closed_common).  The others, and the slots that are in no common case, go to
+// the block's queue and run the general path together at the end.
+//
+// Bound by the gathers' latency and by issue.  207,234 triangles, flux kernel
+// alone: every slot through the whole chain in place 36 us and more, the common
+// case in place and the rest in the queue 35.5 us (11.4 M warp instructions),
+// sorted 26.4 us (9.6 M); the pair of calls 42.6 -> 29.5 us.
+constexpr int REF_THREADS = 128;
+template <class A, int VARIANT>
+__global__ void __launch_bounds__(REF_THREADS, 7) ref_flux_kernel(const __grid_constant__
+                                                               typename RefView<typename A::real>::type m,
+                                                               int kt, int jt) {
+    using R = typename A::real;
+    __shared__ int2 list[REF_THREADS];   // {slot - the block's first, neighbour}
+    __shared__ int queue[REF_THREADS];
+    __shared__ int qn, nopen, nclosed;
+    const int t = threadIdx.x;
+    if (t == 0) qn = nopen = nclosed = 0;
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+    __syncthreads();
+    const int base = blockIdx.x * REF_THREADS;
+    const auto &c = m.cells;
+    const auto &sd = m.sides;
+    if ((long long)base + t < 4LL * m.CELL) {
+        const int nc = (int)(sd.NAC[base + t] - R(1));
+        if (sd.KLAS[base + t] != R(0)) queue[atomicAdd(&qn, 1)] = base + t;
+        else if (nc != -1) list[atomicAdd(&nopen, 1)] = make_int2(t, nc);
+        else list[REF_THREADS - 1 - atomicAdd(&nclosed, 1)] = make_int2(t, -1);
+    }
+    __syncthreads();
+    const bool open = t < nopen;
+    if (open || t >= REF_THREADS - nclosed) {
+        const int2 e = list[t];
+        const int idx = base + e.x, pos = idx >> 2;
+        const CellState<R> own{c.H[pos], c.U[pos], c.V[pos], c.Z[pos], c.ZBC[pos]};
+        const StepParams p{(double)m.HM1, (double)m.HM2, (double)m.JL, (double)m.DT, kt, jt};
+        R f[4];
+        bool done;
+        if (open) {
+            const int nc = e.y;
+            const CellState<R> nb{c.H[nc], c.U[nc], c.V[nc], c.Z[nc], c.ZBC[nc]};
+            done = slot_common<A>(own, nb, pos < nc, sd.COSF[idx], sd.SINF[idx], p, f);
+        } else {
+            done = closed_common<A>(own, sd.COSF[idx], sd.SINF[idx], p, f);
+        }
+        if (done) {
+            sd.FLUX0[idx] = f[0]; sd.FLUX1[idx] = f[1]; sd.FLUX2[idx] = f[2]; sd.FLUX3[idx] = f[3];
+        } else {
+            queue[atomicAdd(&qn, 1)] = idx;
+        }
+    }
+    __syncthreads();
+    for (int q = t; q < qn; q += REF_THREADS) ref_slot<A, VARIANT>(m, queue[q], kt, jt);
+}
+
+// The four values of a cell in a slot array: one vector load where every slot
+// array is aligned to it (VEC, the launch's check), four loads otherwise.
+template <bool VEC>
+__device__ __forceinline__ void ld_slots(const double *p, double v[4]) {
+    if constexpr (VEC) {
+        asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                     : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p) : "memory");
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = p[j];
+    }
+}
+template <bool VEC>
+__device__ __forceinline__ void ld_slots(const float *p, float v[4]) {
+    if constexpr (VEC) {
+        const float4 q = *reinterpret_cast<const float4 *>(p);
+        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = p[j];
+    }
+}
+
+template <class A, int VARIANT, bool VEC>
+__global__ void __launch_bounds__(REF_THREADS, 6) ref_update_kernel(typename RefView<typename A::real>::type m) {
+    using R = typename A::real;
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+    const int pos = blockIdx.x * REF_THREADS + threadIdx.x;
     if (pos >= m.CELL) return;
     const auto &c = m.cells;
     const auto &sd = m.sides;
-    R wh = R(0), wu = R(0), wv = R(0);
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const int s = 4 * pos + j;
-        wsum_add<A>(wh, wu, wv, sd.FLUX0[s], sd.FLUX1[s], sd.FLUX2[s], sd.FLUX3[s], sd.SIDE[s], sd.SLCOS[s], sd.SLSIN[s]);
-    }
+    const size_t s = 4 * (size_t)pos;
     CellUpdateIn<R> ci;
     ci.h = c.H[pos]; ci.u = c.U[pos]; ci.v = c.V[pos]; ci.zbc = c.ZBC[pos]; ci.fnc = c.FNC[pos];
     ci.hlo = R(0);
+    const R area = c.AREA[pos];
+    R f0[4], f1[4], f2[4], f3[4], side[4], slcos[4], slsin[4];
+    ld_slots<VEC>(sd.FLUX0 + s, f0);
+    ld_slots<VEC>(sd.SIDE + s, side);
+    ld_slots<VEC>(sd.FLUX1 + s, f1);
+    ld_slots<VEC>(sd.FLUX3 + s, f3);
+    ld_slots<VEC>(sd.FLUX2 + s, f2);
+    ld_slots<VEC>(sd.SLCOS + s, slcos);
+    ld_slots<VEC>(sd.SLSIN + s, slsin);
+    R wh = R(0), wu = R(0), wv = R(0);
+#pragma unroll
+    for (int j = 0; j < 4; j++) wsum_add<A>(wh, wu, wv, f0[j], f1[j], f2[j], f3[j], side[j], slcos[j], slsin[j]);
     R dta, sidex = R(0);
     if (VARIANT == 1) {
         // SIDEX: triangle inradius or smaller mid-width of a quad (v0 functors.cu:752-763)
-        const R s0 = sd.SIDE[4 * pos], s1 = sd.SIDE[4 * pos + 1], s2 = sd.SIDE[4 * pos + 2], s3 = sd.SIDE[4 * pos + 3];
+        const R s0 = side[0], s1 = side[1], s2 = side[2], s3 = side[3];
         if (s3 > R(0)) {
             sidex = A::fmin(A::mul(A::c(0.5), A::add(s0, s2)), A::mul(A::c(0.5), A::add(s1, s3)));
         } else {
             R ss = A::mul(A::c(0.5), A::add(A::add(s0, s1), s2));
             sidex = A::sqrt(A::div(A::mul(A::mul(A::sub(ss, s0), A::sub(ss, s1)), A::sub(ss, s2)), ss));
         }
-        dta = c.AREA[pos];
+        dta = area;
     } else {
-        dta = A::div(A::c((double)m.DT), c.AREA[pos]);
+        dta = A::div(A::c((double)m.DT), area);
     }
     StepParams p{(double)m.HM1, (double)m.HM2, (double)m.JL, (double)m.DT, 0, 0};
     dta = cell_dta<A, VARIANT>(ci.h, ci.u, dta, sidex, p);
@@ -96,30 +206,45 @@ __global__ void __launch_bounds__(256) ref_update_kernel(typename RefView<typena
     c.H[pos] = o.h; c.U[pos] = o.u; c.V[pos] = o.v; c.Z[pos] = o.z; c.W[pos] = speed<A>(o.u, o.v);
 }
 
+// Launched with programmatic dependent launch: both kernels wait for their
+// predecessor's results before they touch the caller's arrays.
+template <class... P, class... Args>
+static int ref_launch(void (*kernel)(P...), long long threads, void *stream, Args... args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)((threads + REF_THREADS - 1) / REF_THREADS));
+    cfg.blockDim = dim3(REF_THREADS);
+    cfg.stream = (cudaStream_t)stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    HB_CUDA_RET(cudaLaunchKernelEx(&cfg, kernel, args...));
+    return HB_OK;
+}
+
 template <class A, class View>
 static int launch_flux(const View *m, int kt, int jt, int variant, void *stream) {
     if (!m || m->CELL < 0) return set_error(HB_E_INVALID, "hb_ref_calculate_flux: bad mesh view");
     if (m->CELL == 0) return HB_OK;
     if (jt < 0 || jt >= m->NDAYS) return set_error(HB_E_INVALID, "hb_ref_calculate_flux: jt=%d outside [0,%d)", jt, m->NDAYS);
-    const long long n = 4LL * m->CELL;
-    const int blocks = (int)((n + 255) / 256);
-    cudaStream_t st = (cudaStream_t)stream;
-    if (variant == HB_VARIANT_F) ref_flux_kernel<A, 1><<<blocks, 256, 0, st>>>(*m, kt, jt);
-    else ref_flux_kernel<A, 0><<<blocks, 256, 0, st>>>(*m, kt, jt);
-    HB_CUDA_RET(cudaGetLastError());
-    return HB_OK;
+    return ref_launch(variant == HB_VARIANT_F ? ref_flux_kernel<A, 1> : ref_flux_kernel<A, 0>, 4LL * m->CELL, stream, *m,
+                      kt, jt);
 }
 
 template <class A, class View>
 static int launch_update(const View *m, int variant, void *stream) {
     if (!m || m->CELL < 0) return set_error(HB_E_INVALID, "hb_ref_update_cell: bad mesh view");
     if (m->CELL == 0) return HB_OK;
-    const int blocks = (m->CELL + 255) / 256;
-    cudaStream_t st = (cudaStream_t)stream;
-    if (variant == HB_VARIANT_F) ref_update_kernel<A, 1><<<blocks, 256, 0, st>>>(*m);
-    else ref_update_kernel<A, 0><<<blocks, 256, 0, st>>>(*m);
-    HB_CUDA_RET(cudaGetLastError());
-    return HB_OK;
+    using R = typename A::real;
+    const auto &s = m->sides;
+    const void *slots[] = {s.FLUX0, s.FLUX1, s.FLUX2, s.FLUX3, s.SIDE, s.SLCOS, s.SLSIN};
+    bool vec = true;
+    for (const void *q : slots) vec = vec && (uintptr_t)q % (4 * sizeof(R)) == 0;
+    const bool f = variant == HB_VARIANT_F;
+    auto kernel = f ? (vec ? ref_update_kernel<A, 1, true> : ref_update_kernel<A, 1, false>)
+                    : (vec ? ref_update_kernel<A, 0, true> : ref_update_kernel<A, 0, false>);
+    return ref_launch(kernel, m->CELL, stream, *m);
 }
 
 }  // namespace hb

@@ -401,41 +401,6 @@ __device__ __forceinline__ void pair_record(const DevMesh<A> &m, int r, const Re
     queue[i + 1] = 2 * r + 1;
 }
 
-// One side of such an edge on its own (cell_kernel): pair_record's common case
-// for the slot of `own` that faces `nb`, by the direct or the mirrored route.
-// False, and no result, in any other case.
-template <class A>
-__device__ __forceinline__ bool slot_common(const CellStateA<A> &own, const CellStateA<A> &nb, bool own_first,
-                                            typename A::real cosj, typename A::real sinj, const StepParams &p,
-                                            typename A::real f[4]) {
-    using R = typename A::real;
-    using L = typename A::level;
-    const CellStateA<A> &a = own_first ? own : nb, &b = own_first ? nb : own;
-    const R cs = own_first ? cosj : -cosj, sn = own_first ? sinj : -sinj;
-    const R HMX = A::c(fmax(p.hm1, p.hm2));
-    const R qr0 = A::depth(b.z, a.zbc);
-    if (!(a.h > HMX && b.h > HMX && qr0 > HMX && a.z > b.zbc && b.z >= b.zbc)) {
-        f[0] = f[1] = f[2] = f[3] = R(0);
-        return a.h <= A::c(p.hm1) && b.h <= A::c(p.hm1);   // both dry
-    }
-    const R cl = A::sqrt(A::mul(A::c(9.81), a.h)), cr = A::sqrt(A::mul(A::c(9.81), qr0));
-    const R ratio = A::fmin(A::div(b.h, qr0), A::c(1.5));
-    const R ql1 = A::dot(a.u, cs, a.v, sn, M_QL1);
-    const R ql2 = own_first ? A::dot(a.v, cs, -a.u, sn, M_QL2) : A::dot(a.v, cs, -a.u, sn, M_QL2M);
-    const R ur = own_first ? A::dot(b.u, cs, b.v, sn, M_UR) : A::dot(b.u, cs, b.v, sn, M_UR1);
-    const R qr2 = A::dot(b.v, cs, -b.u, sn, M_QR2);
-    const R fil = A::add(ql1, A::mul(A::c(2.0), cl));
-    if (!osher_subcritical<A>(cl, cr, ql1, ql2, A::mul(ur, ratio), qr2, fil, f)) return false;
-    f[1] = osher_f1<A>(f[1], ratio, b.h, ur);
-    if (!own_first) {
-        f[0] = -f[0];
-        const L za = A::ladd(A::lvl(A::sqrt(A::divk_raw(f[3], 4.905))), a.zbc);
-        const R hc3 = za > b.zbc ? A::depth(za, b.zbc) : R(0);
-        f[3] = A::mul(A::mul(A::c(4.905), hc3), hc3);
-    }
-    return true;
-}
-
 // Flux of every record of one step.  Single mesh (SEG = false): records
 // [0, npairs) are mirror pairs and the rest single slots, one per thread.
 // Batch (SEG = true): CTA b takes the scenario and record range of fseg[b].
