@@ -599,71 +599,67 @@ __device__ __noinline__ void general_slot(const DevMesh<A> &m, const double *x, 
 enum : int { LIN_ZERO = 0, LIN_OSHER = 1, LIN_EDGE = 2, LIN_GENERAL = 3 };
 struct SlotLin {
     int kind;
-    bool mir, p3, thin, deep, zside, wet;   // LIN_OSHER: route, piece, qr1 clamped, qr0 > HM1, Z_R > ZBC_R, H_R > HM1
+    bool p3;       // LIN_OSHER: piece 3 (else 5)
     double c[11];
 };
 
+// LIN_OSHER where the forward's slot_common takes the edge from the
+// lower-numbered cell L to R (so that none of osher_inputs' bounds is taken),
+// with the right level strictly above its bed; LIN_ZERO where both cells are
+// dry; LIN_GENERAL otherwise.
 __device__ __forceinline__ void linearise_osher(const CellStateA<A> &L, const CellStateA<A> &R, double cs, double sn,
                                                 bool mir, const StepParams &p, SlotLin &s) {
-    s.kind = LIN_GENERAL;
-    const double clL = A::sqrt(A::mul(A::c(9.81), L.h));
-    const OsherIn<double> oi = osher_inputs<A>(L, R, cs, sn, clL, mir, p);
-    const double cr = A::sqrt(A::mul(A::c(9.81), oi.qr[0]));
-    const double fir = A::sub(oi.qr[1], A::mul(A::c(2.0), cr));
-    const double ua = A::mul(A::add(oi.fil, fir), A::c(0.5));
-    const double ca = A::fabs(A::mul(A::sub(oi.fil, fir), A::c(0.25)));
-    if (!(oi.ql[1] < clL && oi.qr[1] >= -cr && ua >= -ca && ua < ca)) return;
+    s.kind = L.h <= p.hm1 && R.h <= p.hm1 ? LIN_ZERO : LIN_GENERAL;
+    const double HMX = fmax(p.hm1, p.hm2);
+    const double qr0 = A::depth(R.z, L.zbc);
+    if (!(L.h > HMX && R.h > HMX && qr0 > HMX && L.z > R.zbc && R.z > R.zbc)) return;
+    const double cl = A::sqrt(A::mul(A::c(9.81), L.h)), cr = A::sqrt(A::mul(A::c(9.81), qr0));
+    const double q = A::div(R.h, qr0), ratio = A::fmin(q, A::c(1.5));
+    const double ql1 = A::dot(L.u, cs, L.v, sn, M_QL1);
+    const double ql2 = mir ? A::dot(L.v, cs, -L.u, sn, M_QL2M) : A::dot(L.v, cs, -L.u, sn, M_QL2);
+    const double ur = mir ? A::dot(R.u, cs, R.v, sn, M_UR1) : A::dot(R.u, cs, R.v, sn, M_UR);
+    const double qr1 = A::mul(ur, ratio), qr2 = A::dot(R.v, cs, -R.u, sn, M_QR2);
+    const double fil = A::add(ql1, A::mul(A::c(2.0), cl)), fir = A::sub(qr1, A::mul(A::c(2.0), cr));
+    const double ua = A::mul(A::add(fil, fir), A::c(0.5));
+    const double ca = A::fabs(A::mul(A::sub(fil, fir), A::c(0.25)));
+    if (!(ql1 < cl && qr1 >= -cr && A::fabs(ua) < ca)) return;
     s.kind = LIN_OSHER;
-    s.mir = mir;
-    s.p3 = ua >= 0.0;
-    s.thin = oi.hcR <= p.hm2 || oi.qr[0] <= p.hm2;
-    const double zR = A::lmax(R.zbc, R.z);
-    s.deep = A::depth(zR, L.zbc) > p.hm1;
-    s.zside = R.z > R.zbc;
-    s.wet = R.h > p.hm1;
-    const double d = oi.fil - ua, ha = d * d * (1.0 / 39.24);
-    const double q = oi.hcR / oi.qr[0];
+    s.p3 = A::nonnegative(ua);
+    const double d = fil - ua, ha = d * d * (1.0 / 39.24);
     s.c[0] = ua;
     s.c[1] = ha;
-    s.c[2] = s.p3 ? oi.ql[2] : oi.qr[2];
+    s.c[2] = s.p3 ? ql2 : qr2;
     s.c[3] = d * (2.0 / 39.24);
-    s.c[4] = 9.81 / clL;
+    s.c[4] = 9.81 / cl;
     s.c[5] = 9.81 / cr;
-    s.c[6] = oi.ur;
-    s.c[7] = oi.hcR;
-    s.c[8] = oi.ratio;
-    s.c[9] = q < 1.5 ? 1.0 / oi.qr[0] : 0.0;          // d ratio / d hcR
+    s.c[6] = ur;
+    s.c[7] = R.h;
+    s.c[8] = ratio;
+    s.c[9] = q < 1.5 ? 1.0 / qr0 : 0.0;          // d ratio / d hcR
     // mirrored: FLUX3 = 4.905 hc3^2, hc3 = sqrt(fo3 / 4.905) + ZBC_L - ZBC_R = ha + ... where positive
     s.c[10] = fmax(ha + L.zbc - R.zbc, 0.0);
 }
 
-// go, gn from the slot's adjoint inputs (LIN_OSHER); osher_route_rev's steps
-__device__ __forceinline__ void apply_osher(const SlotLin &s, double cs, double sn, double fb0, double fb1, double fb2,
-                                            Adj5 &go, Adj5 &gn) {
+// The adjoints l, r of the edge's two cells from the slot's adjoint inputs
+// (LIN_OSHER); osher_route_rev's steps
+__device__ __forceinline__ void apply_osher(const SlotLin &s, bool mir, double cs, double sn, double fb0, double fb1,
+                                            double fb2, Adj5 &l, Adj5 &r) {
     const double ua = s.c[0], ha = s.c[1], vt = s.c[2], ur = s.c[6], hcR = s.c[7], ratio = s.c[8], iq = s.c[9];
-    if (s.mir) { cs = -cs; sn = -sn; }
-    const double f0 = s.mir ? -fb0 : fb0;
-    const double hc3b = s.mir ? fb1 * 9.81 * s.c[10] : 0.0;
-    const double hab = ua * (f0 + fb1 * ua + fb2 * vt) + (s.mir ? hc3b : fb1 * 9.81 * ha);
+    const double f0 = mir ? -fb0 : fb0;
+    const double hc3b = mir ? fb1 * 9.81 * s.c[10] : 0.0;
+    const double hab = ua * (f0 + fb1 * ua + fb2 * vt) + (mir ? hc3b : fb1 * 9.81 * ha);
     const double uab = ha * (f0 + 2.0 * fb1 * ua + fb2 * vt);
     const double vtb = fb2 * ha * ua;
     const double db = hab * s.c[3];
     const double filb = 0.5 * (uab + db), firb = 0.5 * (uab - db);
     const double t = fb1 * 0.5 * ur;
-    double ratiob = -t * hcR * ur, hcRb = t * (1.0 - ratio) * ur, urb = 2.0 * t * (1.0 - ratio) * hcR;
-    if (!s.thin) { urb += firb * ratio; ratiob += firb * ur; }
-    hcRb += ratiob * iq;
+    const double urb = 2.0 * t * (1.0 - ratio) * hcR + firb * ratio;
+    const double ratiob = (firb - t * hcR) * ur;
+    const double hcRb = t * (1.0 - ratio) * ur + ratiob * iq;
     const double qr0b = -firb * s.c[5] - ratiob * iq * iq * hcR;
-    const double ql2b = s.p3 ? vtb : 0.0, qr2b = s.p3 ? 0.0 : vtb;
-    Adj5 l{filb * s.c[4], filb * cs - ql2b * sn, filb * sn + ql2b * cs, 0.0, hc3b};
-    Adj5 r{s.wet ? hcRb : 0.0, urb * cs - qr2b * sn, urb * sn + qr2b * cs, 0.0, -hc3b};
-    if (s.deep) {
-        if (s.zside) r.z = qr0b;
-        else r.b += qr0b;
-        l.b -= qr0b;
-    }
-    go = s.mir ? r : l;
-    gn = s.mir ? l : r;
+    const double ql2b = s.p3 ? vtb : 0.0, qr2b = vtb - ql2b;
+    l = {filb * s.c[4], filb * cs - ql2b * sn, filb * sn + ql2b * cs, 0.0, hc3b - qr0b};
+    r = {hcRb, urb * cs - qr2b * sn, urb * sn + qr2b * cs, qr0b, -hc3b};
 }
 
 // Boundary slots: the own cell's adjoints {h, ql1, ql2, b} per unit of fb0,
@@ -738,32 +734,6 @@ __device__ __forceinline__ void linearise_edge(const SlotInA<A> &in, double ql1,
     }
 }
 
-// slot_rev's choice of branch at the state before the step, and the slot's
-// linearisation where it has one of its own.
-__device__ __forceinline__ void linearise_slot(const SlotInA<A> &in, const DevMesh<A> &m, int c, const StepParams &p,
-                                               SlotLin &s) {
-    const double h1 = in.own.h, b1 = in.own.zbc;
-    if (code_is_bounda(in.code)) {
-        const double ql1 = A::dot(in.own.u, in.cosj, in.own.v, in.sinj, M_QL1);
-        const double ql2 = A::dot(in.own.v, in.cosj, -in.own.u, in.sinj, M_QL2);
-        linearise_edge(in, ql1, ql2, A::sqrt(A::mul(A::c(9.81), h1)), boundary_of(m, c, p.jt), p, s);
-        return;
-    }
-    const double zi = A::lmax(in.own.z, A::ladd(b1, A::lc(p.hm1)));
-    double hc = 0, bc = 0, zc = 0;
-    if (in.has_nb) {
-        hc = A::fmax(in.nb.h, A::c(p.hm1));
-        bc = in.nb.zbc;
-        zc = A::lmax(bc, in.nb.z);
-    }
-    s.kind = h1 <= p.hm1 && hc <= p.hm1 ? LIN_ZERO : LIN_GENERAL;
-    if (s.kind == LIN_ZERO || zi <= bc || zc <= b1 || h1 <= p.hm2 || hc <= p.hm2 || !in.has_nb || in.code != CODE_ZERO)
-        return;
-    const bool mir = !in.own_first;
-    linearise_osher(mir ? in.nb : in.own, mir ? in.own : in.nb, mir ? -in.cosj : in.cosj, mir ? -in.sinj : in.sinj, mir,
-                    p, s);
-}
-
 // One reverse step t.  x: the state before the step; xn: the state after it.
 // The adjoint of the state after the step is gathered first from step t + 1's
 // contributions (`first`: it is the seed a.lam instead), with the loss term of
@@ -813,6 +783,7 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_CTAS) adj_step_kernel(const _
         lin.kind = LIN_ZERO;
         double cs = 0.0, sn = 0.0, side = 0.0;
         int place = 0, mj = -1;
+        bool mir = false;
         const bool on = t < d.w;
         if (on) {
             const Vec4<double> g = ldg4(a.sgeo + 4 * (size_t)(d.z + t));
@@ -821,19 +792,32 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_CTAS) adj_step_kernel(const _
             place = ref.place;
             mj = a.mirror4[4 * (size_t)d.x + place];
             const int c = d.x + (place >> 2);
-            const Vec4<double> o = ldcg4(x + 4 * (size_t)c);
-            SlotInA<A> in;
-            in.own = CellStateA<A>{o.x, o.y, o.z, o.w, __ldcg(m.zbc + c)};
-            in.nb = CellStateA<A>{0, 0, 0, 0, 0};
-            in.has_nb = ref.nb >= 0;
-            if (in.has_nb) {
-                const Vec4<double> q = ldcg4(x + 4 * (size_t)ref.nb);
-                in.nb = CellStateA<A>{q.x, q.y, q.z, q.w, __ldcg(m.zbc + ref.nb)};
+            // the cells in the order of the edge (slot_common): the lower-numbered one first
+            mir = ref.nb >= 0 && !(ref.meta & META_OWN_FIRST);
+            const int cl = mir ? ref.nb : c, cr = mir ? c : ref.nb;
+            const Vec4<double> o = ldcg4(x + 4 * (size_t)cl);
+            const CellStateA<A> L{o.x, o.y, o.z, o.w, __ldcg(m.zbc + cl)};
+            const int8_t code = (int8_t)(ref.meta & META_CODE);
+            if (code_is_bounda(code)) {
+                if (ref.nb >= 0) {
+                    lin.kind = LIN_GENERAL;
+                } else {
+                    SlotInA<A> in;
+                    in.own = L;
+                    in.nb = CellStateA<A>{0, 0, 0, 0, 0};
+                    in.has_nb = in.own_first = false;
+                    in.code = code;
+                    in.cosj = cs; in.sinj = sn; in.side = side;
+                    linearise_edge(in, A::dot(L.u, cs, L.v, sn, M_QL1), A::dot(L.v, cs, -L.u, sn, M_QL2),
+                                   A::sqrt(A::mul(A::c(9.81), L.h)), boundary_of(m, c, p.jt), p, lin);
+                }
+            } else if (cr >= 0) {
+                const Vec4<double> q = ldcg4(x + 4 * (size_t)cr);
+                linearise_osher(L, CellStateA<A>{q.x, q.y, q.z, q.w, __ldcg(m.zbc + cr)}, mir ? -cs : cs, mir ? -sn : sn,
+                                mir, p, lin);
+            } else {
+                lin.kind = LIN_GENERAL;
             }
-            in.code = (int8_t)(ref.meta & META_CODE);
-            in.own_first = ref.meta & META_OWN_FIRST;
-            in.cosj = cs; in.sinj = sn; in.side = side;
-            linearise_slot(in, m, c, p, lin);
         }
         cudaGridDependencySynchronize();
         cudaTriggerProgrammaticLaunchCompletion();
@@ -860,18 +844,18 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_CTAS) adj_step_kernel(const _
             if (lin.kind == LIN_GENERAL) {
                 general_slot(m, x, a.sgeo + 4 * (size_t)(d.z + t), d.x + (place >> 2), p, fb0, fb1, fb2, so, sno);
             } else {
-                Adj5 go{0, 0, 0, 0, 0}, gn{0, 0, 0, 0, 0};
+                Adj5 l{0, 0, 0, 0, 0}, r{0, 0, 0, 0, 0};
                 if (lin.kind == LIN_OSHER) {
-                    apply_osher(lin, cs, sn, fb0, fb1, fb2, go, gn);
+                    apply_osher(lin, mir, mir ? -cs : cs, mir ? -sn : sn, fb0, fb1, fb2, l, r);
                 } else if (lin.kind == LIN_EDGE) {
                     const double ql1b = fb0 * lin.c[3] + fb1 * lin.c[4] + fb2 * lin.c[5], ql2b = fb2 * lin.c[6];
-                    go.h = fb0 * lin.c[0] + fb1 * lin.c[1] + fb2 * lin.c[2];
-                    go.u = ql1b * cs - ql2b * sn;
-                    go.v = ql1b * sn + ql2b * cs;
-                    go.b = fb0 * lin.c[7] + fb1 * lin.c[8];
+                    l.h = fb0 * lin.c[0] + fb1 * lin.c[1] + fb2 * lin.c[2];
+                    l.u = ql1b * cs - ql2b * sn;
+                    l.v = ql1b * sn + ql2b * cs;
+                    l.b = fb0 * lin.c[7] + fb1 * lin.c[8];
                 }
-                st_rec(so, go);
-                st_rec(sno, gn);
+                st_rec(mir ? sno : so, l);   // the slot's own cell is L on the direct route
+                st_rec(mir ? so : sno, r);
             }
         }
     } else {

@@ -794,22 +794,24 @@ __device__ __forceinline__ void flux_slot(const SlotInA<A> &in, typename A::real
     else { o.f[0] = -fo[0]; o.f[3] = mirror_f3<A>(fo[3], in.nb.zbc, in.own.zbc); }
 }
 
-// The common case of an interior slot (code 0) of `own` that faces `nb`, by the
-// direct or the mirrored route: both cells deep and the flow across the edge
-// subcritical, or both dry.  False, and no result, in any other case.  Deep
-// enough: for both sides' branch chains to reach Osher and for its inputs
-// (osher_inputs) to take none of their bounds: both depths and QR[0] above HM1
-// and HM2 (so max(H, HM1) = H and QR[1] is not the thin-water value), the right
-// level above its bed (so max(ZBC, Z) = Z), and each side's level above the
-// other's bed (of which QR[0] > 0 is one).
+// The common case of an interior slot (code 0) across an edge from the
+// lower-numbered cell a to b, by the direct route (the slot of a) or the
+// mirrored one (that of b); (cosj, sinj) is the slot's own normal.  Both cells
+// deep and the flow across the edge subcritical, or both dry; false, and no
+// result, in any other case.  Deep enough: for both sides' branch chains to
+// reach Osher and for its inputs (osher_inputs) to take none of their bounds:
+// both depths and QR[0] above HM1 and HM2 (so max(H, HM1) = H and QR[1] is not
+// the thin-water value), the right level above its bed (so max(ZBC, Z) = Z), and
+// each side's level above the other's bed (of which QR[0] > 0 is one).  The
+// caller loads the cells in this order: selecting their five values instead
+// costs forty selects.
 template <class A>
-__device__ __forceinline__ bool slot_common(const CellStateA<A> &own, const CellStateA<A> &nb, bool own_first,
+__device__ __forceinline__ bool slot_common(const CellStateA<A> &a, const CellStateA<A> &b, bool direct,
                                             typename A::real cosj, typename A::real sinj, const StepParams &p,
                                             typename A::real f[4]) {
     using R = typename A::real;
     using L = typename A::level;
-    const CellStateA<A> &a = own_first ? own : nb, &b = own_first ? nb : own;
-    const R cs = own_first ? cosj : -cosj, sn = own_first ? sinj : -sinj;
+    const R cs = direct ? cosj : -cosj, sn = direct ? sinj : -sinj;
     const R HMX = A::c(fmax(p.hm1, p.hm2));
     const R qr0 = A::depth(b.z, a.zbc);
     if (!(a.h > HMX && b.h > HMX && qr0 > HMX && a.z > b.zbc && b.z >= b.zbc)) {
@@ -819,13 +821,13 @@ __device__ __forceinline__ bool slot_common(const CellStateA<A> &own, const Cell
     const R cl = A::sqrt(A::mul(A::c(9.81), a.h)), cr = A::sqrt(A::mul(A::c(9.81), qr0));
     const R ratio = A::fmin(A::div(b.h, qr0), A::c(1.5));
     const R ql1 = A::dot(a.u, cs, a.v, sn, M_QL1);
-    const R ql2 = own_first ? A::dot(a.v, cs, -a.u, sn, M_QL2) : A::dot(a.v, cs, -a.u, sn, M_QL2M);
-    const R ur = own_first ? A::dot(b.u, cs, b.v, sn, M_UR) : A::dot(b.u, cs, b.v, sn, M_UR1);
+    const R ql2 = direct ? A::dot(a.v, cs, -a.u, sn, M_QL2) : A::dot(a.v, cs, -a.u, sn, M_QL2M);
+    const R ur = direct ? A::dot(b.u, cs, b.v, sn, M_UR) : A::dot(b.u, cs, b.v, sn, M_UR1);
     const R qr2 = A::dot(b.v, cs, -b.u, sn, M_QR2);
     const R fil = A::add(ql1, A::mul(A::c(2.0), cl));
     if (!osher_subcritical<A>(cl, cr, ql1, ql2, A::mul(ur, ratio), qr2, fil, f)) return false;
     f[1] = osher_f1<A>(f[1], ratio, b.h, ur);
-    if (!own_first) {
+    if (!direct) {
         f[0] = -f[0];
         const L za = A::ladd(A::lvl(A::sqrt(A::divk_raw(f[3], 4.905))), a.zbc);
         const R hc3 = za > b.zbc ? A::depth(za, b.zbc) : R(0);

@@ -116,16 +116,16 @@ __global__ void __launch_bounds__(REF_THREADS, 7) ref_flux_kernel(const __grid_c
     if (open || t >= REF_THREADS - nclosed) {
         const int2 e = list[t];
         const int idx = base + e.x, pos = idx >> 2;
-        const CellState<R> own{c.H[pos], c.U[pos], c.V[pos], c.Z[pos], c.ZBC[pos]};
         const StepParams p{(double)m.HM1, (double)m.HM2, (double)m.JL, (double)m.DT, kt, jt};
+        auto cell = [&](int i) { return CellState<R>{c.H[i], c.U[i], c.V[i], c.Z[i], c.ZBC[i]}; };
         R f[4];
         bool done;
         if (open) {
-            const int nc = e.y;
-            const CellState<R> nb{c.H[nc], c.U[nc], c.V[nc], c.Z[nc], c.ZBC[nc]};
-            done = slot_common<A>(own, nb, pos < nc, sd.COSF[idx], sd.SINF[idx], p, f);
+            const bool direct = pos < e.y;
+            const int ca = direct ? pos : e.y, cb = direct ? e.y : pos;
+            done = slot_common<A>(cell(ca), cell(cb), direct, sd.COSF[idx], sd.SINF[idx], p, f);
         } else {
-            done = closed_common<A>(own, sd.COSF[idx], sd.SINF[idx], p, f);
+            done = closed_common<A>(cell(pos), sd.COSF[idx], sd.SINF[idx], p, f);
         }
         if (done) {
             sd.FLUX0[idx] = f[0]; sd.FLUX1[idx] = f[1]; sd.FLUX2[idx] = f[2]; sd.FLUX3[idx] = f[3];

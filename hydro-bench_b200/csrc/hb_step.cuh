@@ -718,12 +718,18 @@ __global__ void __launch_bounds__(CELL_THREADS, CELL_CTAS) cell_kernel(DevMesh<A
         // the adjoint's parameters change between sequences, from L2)
         Vec4<R> g{R(0), R(0), R(0), R(0)};
         SlotRef ref{-1, 0, 0, 0};
-        L zb = L(0), zbn = L(0);
+        L zba = L(0), zbb = L(0);
+        int ca = 0, cb = -1;   // the lower-numbered cell of the edge and the other (slot_common); the slot's own if alone
+        bool direct = true;
         if (t < d.w) {
             g = ldg4(m.sgeo + 4 * (size_t)(d.z + t));
             ref = SlotRef::unpack((unsigned long long)__double_as_longlong((double)g.w));
-            zb = __ldcg(m.zbc + d.x + (ref.place >> 2));
-            if (ref.nb >= 0) zbn = __ldcg(m.zbc + ref.nb);
+            direct = ref.nb < 0 || (ref.meta & META_OWN_FIRST);
+            ca = d.x + (ref.place >> 2);
+            cb = ref.nb;
+            if (!direct) { cb = ca; ca = ref.nb; }
+            zba = __ldcg(m.zbc + ca);
+            if (cb >= 0) zbb = __ldcg(m.zbc + cb);
         }
         StepParams p{m.hm1, m.hm2, m.jl, m.dt, 1, 0};
         const bool timed = code_is_bounda((int8_t)(ref.meta & META_CODE));
@@ -736,24 +742,24 @@ __global__ void __launch_bounds__(CELL_THREADS, CELL_CTAS) cell_kernel(DevMesh<A
         }
         if (t < d.w) {
             const R *S = m.S[si.par];
-            const int c = d.x + (ref.place >> 2), sa = 4 * d.x + ref.place;
-            const Vec4<R> a = ldg4(S + 4 * (size_t)c);
-            CellStateA<A> nb{R(0), R(0), R(0), L(0), L(0)};
-            if (ref.nb >= 0) {
-                const Vec4<R> b = ldg4(S + 4 * (size_t)ref.nb);
-                nb = {b.x, b.y, b.z, b.w, zbn};
+            const int sa = 4 * d.x + ref.place;
+            const Vec4<R> va = ldg4(S + 4 * (size_t)ca);
+            const CellStateA<A> a{va.x, va.y, va.z, va.w, zba};
+            CellStateA<A> b{R(0), R(0), R(0), L(0), L(0)};
+            if (cb >= 0) {
+                const Vec4<R> vb = ldg4(S + 4 * (size_t)cb);
+                b = {vb.x, vb.y, vb.z, vb.w, zbb};
             }
             uint8_t meta = ref.meta;
             if ((meta & META_CODE) == CODE_K7) meta = m.rmeta[ref.record];   // breached since?
             const Terms<R, true> tout{terms + CELL_TERMS * (ref.place >> 2) + 4 * (ref.place & 3), sa};
-            const CellStateA<A> own{a.x, a.y, a.z, a.w, zb};
             R f[4];
-            if ((meta & META_CODE) == CODE_ZERO && (meta & META_HAS_NB) &&
-                slot_common<A>(own, nb, meta & META_OWN_FIRST, g.x, g.y, p, f)) {
+            if ((meta & META_CODE) == CODE_ZERO && cb >= 0 && slot_common<A>(a, b, direct, g.x, g.y, p, f)) {
                 if (write_flux) store_flux(m, sa, f);
                 store_terms<A>(tout, sa, f, g.z, g.x, g.y);
             } else {
-                single_core<A, VARIANT>(m, ref.record, c, sa, own, nb, meta, g, p, write_flux, tout);
+                single_core<A, VARIANT>(m, ref.record, sa >> 2, sa, direct ? a : b, direct ? b : a, meta, g, p,
+                                        write_flux, tout);
             }
         }
         __syncthreads();
