@@ -24,7 +24,8 @@ bool fits_at_once(const hb_handle *h, size_t ctas) {
 }
 
 template <int VARIANT, bool COEF>
-int launch_cells_t(int ncseg, const hb::DevMesh<hb::F64Exact> &m, int k0, int n, int write_last, cudaStream_t st) {
+int launch_cells_t(int ncseg, const hb::DevMesh<hb::F64Exact> &m, int k0, int n, int write_last, int tick,
+                   cudaStream_t st) {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -36,7 +37,7 @@ int launch_cells_t(int ncseg, const hb::DevMesh<hb::F64Exact> &m, int k0, int n,
     cfg.numAttrs = 1;
     for (int k = 0; k < n; k++)
         HB_CUDA_RET(cudaLaunchKernelEx(&cfg, hb::cell_kernel<hb::F64Exact, VARIANT, COEF>, m, k0 + k,
-                                       (int)(write_last && k == n - 1)));
+                                       (int)(write_last && k == n - 1), k == n - 1 ? tick : 0));
     return HB_OK;
 }
 
@@ -108,11 +109,11 @@ int hb_cells_build(hb_handle *h, const std::vector<int4> &rix, const std::vector
     return HB_OK;
 }
 
-int hb_cells_launch(hb_handle *h, const hb::DevMesh<hb::F64Exact> &m, int k0, int n, int write_last, bool coef,
-                    cudaStream_t st) {
+int hb_cells_launch(hb_handle *h, const hb::DevMesh<hb::F64Exact> &m, int k0, int n, int write_last, int tick,
+                    bool coef, cudaStream_t st) {
     if (h->opt.variant == HB_VARIANT_F) {
         if (coef) return hb::set_error(HB_E_INVALID, "update coefficients: variant H only");
-        return launch_cells_t<1, false>(h->ncseg, m, k0, n, write_last, st);
+        return launch_cells_t<1, false>(h->ncseg, m, k0, n, write_last, tick, st);
     }
-    return coef ? launch_cells_t<0, true>(h->ncseg, m, k0, n, write_last, st) : launch_cells_t<0, false>(h->ncseg, m, k0, n, write_last, st);
+    return coef ? launch_cells_t<0, true>(h->ncseg, m, k0, n, write_last, tick, st) : launch_cells_t<0, false>(h->ncseg, m, k0, n, write_last, tick, st);
 }

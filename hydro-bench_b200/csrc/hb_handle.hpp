@@ -64,7 +64,7 @@ struct hb_handle {
     // persistent handles: the grid-barrier words {arrival count, give-up flag}
     // (both zeroed before each launch), the resident CTAs of the cooperative
     // launch (0 = not yet queried), and the barrier wait bound
-    unsigned *d_bar = nullptr;
+    unsigned *d_bar = nullptr;       // a third word behind them is DevMesh::tick
     int persist_blocks = 0;
     unsigned long long barrier_limit_ns = 1000000000ull;
     unsigned barrier_phantom = 0;
@@ -148,8 +148,8 @@ int hb_tiles_resident(hb_handle *h, int config, int tile_cells, int *per_sm);
 bool hb_cells_used(const hb_handle *h);
 int hb_cells_build(hb_handle *h, const std::vector<int4> &rix, const std::vector<uint8_t> &rmeta,
                    const std::vector<double> &rgeo);
-int hb_cells_launch(hb_handle *h, const hb::DevMesh<hb::F64Exact> &m, int k0, int n, int write_last, bool coef,
-                    cudaStream_t st);
+int hb_cells_launch(hb_handle *h, const hb::DevMesh<hb::F64Exact> &m, int k0, int n, int write_last, int tick,
+                    bool coef, cudaStream_t st);
 // One fp64 edge-layout step t0 + k (the device step counter must hold t0)
 // from state `in` to state `out` ([C][4] each), keeping the slots' terms of
 // the cell sums in `terms` ([4C][4]) and the update coefficients of the wet

@@ -545,6 +545,7 @@ int build_device_mesh(hb_handle *h, const hb_mesh_desc *mds, int n, hb::DevMesh<
     m.sidex = sidex;
     m.err = h->d_err;
     m.step_ctr = h->d_ctr;
+    m.tick = h->d_bar + 2;
     // scenario table and segment tables
     std::vector<hb::ScnParams> sp;
     for (const auto &sc : h->scn)
@@ -610,10 +611,7 @@ int launch_tick(hb_handle *h, int n, cudaStream_t st) {
 template <class A, int VARIANT, bool SEG>
 int launch_steps_t(hb_handle *h, hb::DevMesh<A> m, int n, cudaStream_t st) {
     if constexpr (std::is_same<A, hb::F64Exact>::value && !SEG) {
-        if (hb_cells_used(h)) {
-            TRY(hb_cells_launch(h, m, 0, n, 1, false, st));
-            return launch_tick(h, n, st);
-        }
+        if (hb_cells_used(h)) return hb_cells_launch(h, m, 0, n, 1, n, false, st);
     }
     // Programmatic dependent launch: each kernel may start while its predecessor
     // drains and waits in cudaGridDependencySynchronize for its results.
@@ -775,7 +773,7 @@ int hb_forward_step_into(hb_handle *h, long long t0, int k, const double *in, do
     m.S[par ^ 1] = out;
     m.slotw = terms;
     m.ucoef = coef;
-    if (hb_cells_used(h)) return hb_cells_launch(h, m, k, 1, write_flux, true, st);
+    if (hb_cells_used(h)) return hb_cells_launch(h, m, k, 1, write_flux, 0, true, st);
     // programmatic dependent launch, as in the step sequence (launch_steps_t)
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -866,7 +864,7 @@ extern "C" int hb_create_batch(const hb_mesh_desc *meshes, int32_t n, const hb_o
     }
     int st;
     if ((st = dev_alloc(h, &h->d_err, 1)) != HB_OK || (st = dev_alloc(h, &h->d_ctr, 1)) != HB_OK ||
-        (st = dev_alloc(h, &h->d_bar, 2)) != HB_OK) {
+        (st = dev_alloc(h, &h->d_bar, 3)) != HB_OK) {
         delete h;
         return st;
     }
