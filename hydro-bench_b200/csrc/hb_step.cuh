@@ -939,11 +939,14 @@ template <class A, int VARIANT, int THREADS, int MINB, bool SEG>
 __global__ void __launch_bounds__(THREADS, MINB)
     persistent_kernel(DevMesh<A> m, int n, int nflux, int ncell, unsigned *bar, unsigned phantom,
                       unsigned long long limit_ns) {
-    // The queue of sides collects those of several chunks and is run when it
-    // could not take another chunk's worth, and at the end of the flux phase:
-    // one block barrier per chunk instead of three.  Every queued side is run
-    // before the grid barrier, as flux_kernel runs it before it ends.
-    constexpr int QCAP = 4 * THREADS;
+    // The queue of sides collects those of several chunks and is run when the
+    // chunks since could have filled it but for one, and at the end of the flux
+    // phase: one block barrier per chunk instead of three.  The bound is counted
+    // from the chunks' records, the same in every thread: the queue's own count
+    // may already hold the next chunk's sides when a slow thread reads it.
+    // Every queued side is run before the grid barrier, as flux_kernel runs it
+    // before it ends.
+    constexpr int QCAP = 16 * THREADS;
     __shared__ int queue[QCAP];
     __shared__ int qn;
     const Terms<typename A::real> tout{m.slotw, 0};
@@ -965,6 +968,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
             si0 = step_index(m, k, m.per_day, m.ndays);
             p0 = StepParams{m.hm1, m.hm2, m.jl, m.dt, 1, 0};
         }
+        int bound = 0;   // sides that the chunks since the queue was last run may have queued
         for (int b = blockIdx.x; b < nflux; b += gridDim.x) {
             int r0, cnt;
             bool seg_pairs = false;
@@ -991,7 +995,11 @@ __global__ void __launch_bounds__(THREADS, MINB)
             __syncthreads();   // the queue's count is complete
             // a batch chunk's sides have their scenario's parameters: its queue
             // runs at once; a single mesh's when another chunk might not fit
-            if (SEG || qn > QCAP - 2 * THREADS) run_queue(si, p, wf);
+            bound += 2 * cnt;
+            if (SEG || bound > QCAP - 2 * THREADS) {
+                run_queue(si, p, wf);
+                bound = 0;
+            }
         }
         if constexpr (!SEG) run_queue(si0, p0, wf);
         arrivals += gridDim.x;
