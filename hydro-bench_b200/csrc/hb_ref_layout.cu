@@ -58,25 +58,6 @@ __device__ __forceinline__ void ref_slot(const typename RefView<typename A::real
     if (o.mask & 8) sd.FLUX3[idx] = o.f[3];
 }
 
-// A slot without neighbour and code 0, as a rule a triangle's zero-length
-// fourth slot: the branch the chain takes for a wet cell above a bed at or
-// above zero (ZC = 0 <= ZBC, functors.cu:112-117), or the dry one.  False, and
-// no result, in any other case.
-template <class A>
-__device__ __forceinline__ bool closed_common(const CellStateA<A> &own, typename A::real cs, typename A::real sn,
-                                              const StepParams &p, typename A::real f[4]) {
-    using R = typename A::real;
-    f[0] = f[1] = f[2] = f[3] = R(0);
-    if (own.h <= A::c(p.hm1)) return p.hm1 >= 0.0;   // both depths at most HM1: no neighbour counts as 0
-    if (!(own.z > R(0) && R(0) <= own.zbc)) return false;
-    const R ql1 = A::dot(own.u, cs, own.v, sn, M_QL1), ql2 = A::dot(own.v, cs, -own.u, sn, M_QL2);
-    f[0] = A::mul(A::c(K::C1), A::pow(own.h, A::c(1.5)));
-    const R ha = A::mul(own.h, A::fabs(ql1));
-    f[1] = A::mul(ha, ql1);
-    f[2] = A::mul(ha, ql2);
-    return true;
-}
-
 // One slot per thread, sorted within the block: the interior slots with code 0
 // to the front threads, those without neighbour (a quarter of a triangle mesh's
 // slots, one in every group of four lanes, whose flux takes a power) to the

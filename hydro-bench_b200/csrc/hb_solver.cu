@@ -526,8 +526,7 @@ int build_device_mesh(hb_handle *h, const hb_mesh_desc *mds, int n, hb::DevMesh<
     for (int b = 0; b < 2; b++) TRY(dev_alloc(h, &m.S[b], 4 * (size_t)C));
     TRY(dev_alloc(h, &m.slotw, 16 * (size_t)C));
     TRY(dev_alloc(h, &m.W, C));
-    TRY(dev_alloc(h, &m.f0, S)); TRY(dev_alloc(h, &m.f1, S));
-    TRY(dev_alloc(h, &m.f2, S)); TRY(dev_alloc(h, &m.f3, S));
+    TRY(dev_alloc(h, &m.flux, 4 * S));
     R *dta = nullptr, *sidex = nullptr;
     TRY(dev_alloc(h, &dta, C));
     TRY(dev_alloc(h, &sidex, C));
@@ -941,16 +940,17 @@ int get_flux_t(hb_handle *h, int s, hb::DevMesh<A> &m, double *F0, double *F1, d
     const hb::Scenario &sc = h->scn[s];
     const int C = sc.cells;
     const size_t S = 4 * (size_t)C;
-    std::vector<R> buf(S);
+    std::vector<R> buf(4 * S);
     double *dst[4] = {F0, F1, F2, F3};
-    R *src[4] = {m.f0, m.f1, m.f2, m.f3};
     HB_CUDA_RET(cudaDeviceSynchronize());
-    for (int k = 0; k < 4; k++) {
-        if (!dst[k]) continue;
-        HB_CUDA_RET(cudaMemcpy(buf.data(), src[k] + 4 * (size_t)sc.cell0, S * sizeof(R), cudaMemcpyDeviceToHost));
-        for (int i = 0; i < C; i++)
-            for (int j = 0; j < 4; j++) dst[k][4 * (size_t)sc.perm[i] + j] = (double)buf[4 * (size_t)i + j];
-    }
+    HB_CUDA_RET(cudaMemcpy(buf.data(), m.flux + 16 * (size_t)sc.cell0, 4 * S * sizeof(R), cudaMemcpyDeviceToHost));
+    for (int i = 0; i < C; i++)
+        for (int j = 0; j < 4; j++) {
+            const R *f = &buf[4 * (4 * (size_t)i + j)];
+            const size_t so = 4 * (size_t)sc.perm[i] + j;
+            for (int k = 0; k < 4; k++)
+                if (dst[k]) dst[k][so] = (double)f[k];
+        }
     return HB_OK;
 }
 template <class A>
@@ -1208,8 +1208,7 @@ extern "C" int hb_autotune(hb_handle *h, int32_t steps, void *stream, float *ms_
         using R = typename std::remove_reference<decltype(m)>::type::R;
         const size_t C = (size_t)h->C;
         pieces = {{m.S[0], 4 * C * sizeof(R)}, {m.S[1], 4 * C * sizeof(R)}, {m.W, C * sizeof(R)},
-                  {m.f0, 4 * C * sizeof(R)}, {m.f1, 4 * C * sizeof(R)}, {m.f2, 4 * C * sizeof(R)},
-                  {m.f3, 4 * C * sizeof(R)}, {m.rmeta, (size_t)std::max(m.nrecords, 1)},
+                  {m.flux, 16 * C * sizeof(R)}, {m.rmeta, (size_t)std::max(m.nrecords, 1)},
                   {h->d_err, sizeof(uint32_t)}, {h->d_ctr, sizeof(long long)}};
         return HB_OK;
     });
@@ -1317,15 +1316,26 @@ struct CheckpointHeader {
     uint64_t payload;                   // bytes after the header
 };
 
-// the pieces of device memory a resumed run needs, in checkpoint order
+// The pieces of device memory a resumed run needs, in checkpoint order.  The
+// fluxes (`value` > 0, the size of one) are [slot][4] on the device and four
+// arrays in a checkpoint.
+struct CheckpointPiece { void *p; size_t bytes, value; };
 template <class A>
-std::vector<std::pair<void *, size_t>> checkpoint_pieces(hb_handle *h, hb::DevMesh<A> &m) {
+std::vector<CheckpointPiece> checkpoint_pieces(hb_handle *h, hb::DevMesh<A> &m) {
     using R = typename A::real;
     const size_t C = (size_t)h->C;
     const int par = (int)(h->steps_done & 1);
-    return {{m.S[par], 4 * C * sizeof(R)}, {m.W, C * sizeof(R)},       {m.f0, 4 * C * sizeof(R)},
-            {m.f1, 4 * C * sizeof(R)},     {m.f2, 4 * C * sizeof(R)}, {m.f3, 4 * C * sizeof(R)},
-            {m.rmeta, (size_t)m.nrecords}, {h->d_err, sizeof(uint32_t)}};
+    return {{m.S[par], 4 * C * sizeof(R), 0}, {m.W, C * sizeof(R), 0}, {m.flux, 16 * C * sizeof(R), sizeof(R)},
+            {m.rmeta, (size_t)m.nrecords, 0}, {h->d_err, sizeof(uint32_t), 0}};
+}
+// records of four values <-> four arrays of n values
+void records_to_arrays(const char *rec, char *arr, size_t n, size_t value) {
+    for (size_t i = 0; i < n; i++)
+        for (size_t k = 0; k < 4; k++) memcpy(arr + (k * n + i) * value, rec + (4 * i + k) * value, value);
+}
+void arrays_to_records(const char *arr, char *rec, size_t n, size_t value) {
+    for (size_t i = 0; i < n; i++)
+        for (size_t k = 0; k < 4; k++) memcpy(rec + (4 * i + k) * value, arr + (k * n + i) * value, value);
 }
 }  // namespace
 
@@ -1333,7 +1343,7 @@ extern "C" int hb_checkpoint_size(hb_handle *h, size_t *bytes) {
     if (!h || !bytes) return hb::set_error(HB_E_INVALID, "null argument");
     size_t n = sizeof(CheckpointHeader);
     h->with_mesh([&](auto &m) {
-        for (auto &p : checkpoint_pieces(h, m)) n += p.second;
+        for (auto &p : checkpoint_pieces(h, m)) n += p.bytes;
         return HB_OK;
     });
     *bytes = n;
@@ -1356,8 +1366,14 @@ extern "C" int hb_checkpoint_save(hb_handle *h, void *buffer, size_t bytes) {
     int rc = h->with_mesh([&](auto &m) -> int {
         hd.nrecords = m.nrecords;
         for (auto &p : checkpoint_pieces(h, m)) {
-            HB_CUDA_RET(cudaMemcpy(out, p.first, p.second, cudaMemcpyDeviceToHost));
-            out += p.second;
+            if (p.value > 0) {
+                std::vector<char> rec(p.bytes);
+                HB_CUDA_RET(cudaMemcpy(rec.data(), p.p, p.bytes, cudaMemcpyDeviceToHost));
+                records_to_arrays(rec.data(), out, p.bytes / (4 * p.value), p.value);
+            } else {
+                HB_CUDA_RET(cudaMemcpy(out, p.p, p.bytes, cudaMemcpyDeviceToHost));
+            }
+            out += p.bytes;
         }
         return HB_OK;
     });
@@ -1385,8 +1401,14 @@ extern "C" int hb_checkpoint_load(hb_handle *h, const void *buffer, size_t bytes
     const char *in = (const char *)buffer + sizeof hd;
     int rc = h->with_mesh([&](auto &m) -> int {
         for (auto &p : checkpoint_pieces(h, m)) {
-            HB_CUDA_RET(cudaMemcpy(p.first, in, p.second, cudaMemcpyHostToDevice));
-            in += p.second;
+            if (p.value > 0) {
+                std::vector<char> rec(p.bytes);
+                arrays_to_records(in, rec.data(), p.bytes / (4 * p.value), p.value);
+                HB_CUDA_RET(cudaMemcpy(p.p, rec.data(), p.bytes, cudaMemcpyHostToDevice));
+            } else {
+                HB_CUDA_RET(cudaMemcpy(p.p, in, p.bytes, cudaMemcpyHostToDevice));
+            }
+            in += p.bytes;
         }
         return HB_OK;
     });
