@@ -25,7 +25,7 @@ enum : uint8_t { META_CODE = 0x0F, META_OWN_FIRST = 0x10, META_HAS_NB = 0x20 };
 enum Layout : int { LAYOUT_EDGE = HB_LAYOUT_EDGE, LAYOUT_TILE = HB_LAYOUT_TILE };
 struct LaunchConfig { int layout, threads, min_blocks, update_min_blocks; };
 constexpr LaunchConfig LAUNCH_CONFIGS[] = {
-    {LAYOUT_EDGE, 128, 7, 6}, {LAYOUT_EDGE, 128, 6, 8}, {LAYOUT_EDGE, 128, 8, 8}, {LAYOUT_EDGE, 256, 3, 6},
+    {LAYOUT_EDGE, 128, 8, 8}, {LAYOUT_EDGE, 128, 6, 8}, {LAYOUT_EDGE, 128, 7, 6}, {LAYOUT_EDGE, 256, 3, 6},
     {LAYOUT_EDGE, 256, 4, 8}, {LAYOUT_EDGE, 128, 7, 8}, {LAYOUT_EDGE, 256, 2, 6}, {LAYOUT_EDGE, 64, 12, 8},
     {LAYOUT_TILE, 256, 3, 0}, {LAYOUT_TILE, 256, 2, 0}, {LAYOUT_TILE, 128, 6, 0}, {LAYOUT_TILE, 128, 4, 0},
     {LAYOUT_TILE, 512, 1, 0}, {LAYOUT_TILE, 256, 4, 0},
@@ -551,8 +551,7 @@ __device__ __forceinline__ void update_core(const DevMesh<A> &m, int c, const Ce
     // For a finite state (h > 0) its fluxes are finite, so each addend is a
     // zero and leaves a non-zero partial sum unchanged bit for bit: the first
     // pass skips such slots.  Only a zero partial sum at a zero-length slot
-    // (whose sign the addend may change), a non-finite state, or the last
-    // step of a sequence (which writes the slot's fluxes) needs the slot's
+    // (whose sign the addend may change) or a non-finite state needs the slot's
     // flux: the second pass then evaluates it once (every zero-length slot of
     // a cell has the same inputs: the cell's state, no neighbour, zero
     // geometry and code 0) and redoes the sums with every slot in order.
@@ -570,25 +569,31 @@ __device__ __forceinline__ void update_core(const DevMesh<A> &m, int c, const Ce
             wh = A::madd(t[j].w, t[j].x, wh, M_WH);
             wu = A::add(wu, t[j].y);
             wv = A::add(wv, t[j].z);
-        } else if ((write_flux && TERMS != TERMS_SMEM_LATE) || !finite_state || wh == R(0) || wu == R(0) || wv == R(0)) {
+        } else if (!finite_state || wh == R(0) || wu == R(0) || wv == R(0)) {
             need_zero = true;
         }
     }
-    if (need_zero) {
-        const int exact = TERMS != TERMS_SMEM_LATE ? write_flux : 0;
-        const ZeroSlot<R> o = SMEM_TERMS ? zero_slot<A, VARIANT>(st, p, exact) : zero_slot_call<A, VARIANT>(st, p, exact);
-        if (exact) store_zero(m, c, mask, o);
-        wh = R(0); wu = R(0); wv = R(0);
+    // The last step of a sequence leaves such slots' fluxes too.  One evaluation
+    // serves both needs, and the sums are redone only where they need it: single
+    // steps at 207,234 cells 24.7 -> 22.1 us, at 60,000 14.0 -> 12.5 us.
+    const bool leave = TERMS != TERMS_SMEM_LATE && write_flux && (mask & 15u) != 15u;
+    if (need_zero || leave) {
+        const ZeroSlot<R> o =
+            SMEM_TERMS ? zero_slot<A, VARIANT>(st, p, leave) : zero_slot_call<A, VARIANT>(st, p, leave);
+        if (leave) store_zero(m, c, mask, o);
+        if (need_zero) {
+            wh = R(0); wu = R(0); wv = R(0);
 #pragma unroll 1
-        for (int j = 0; j < 4; j++) {
-            if (mask & (1u << j)) {
-                const Vec4<R> tj = terms_of(j);
-                wh = A::madd(tj.w, tj.x, wh, M_WH);
-                wu = A::add(wu, tj.y);
-                wv = A::add(wv, tj.z);
-            } else {
-                // zero-length slot: SIDE = SLCOS = SLSIN = 0 (mesh.cpp:293-306, :347-370)
-                wsum_add<A>(wh, wu, wv, o.f[0], o.f[1], o.f[2], o.f[3], R(0), R(0), R(0));
+            for (int j = 0; j < 4; j++) {
+                if (mask & (1u << j)) {
+                    const Vec4<R> tj = terms_of(j);
+                    wh = A::madd(tj.w, tj.x, wh, M_WH);
+                    wu = A::add(wu, tj.y);
+                    wv = A::add(wv, tj.z);
+                } else {
+                    // zero-length slot: SIDE = SLCOS = SLSIN = 0 (mesh.cpp:293-306, :347-370)
+                    wsum_add<A>(wh, wu, wv, o.f[0], o.f[1], o.f[2], o.f[3], R(0), R(0), R(0));
+                }
             }
         }
     }
@@ -636,9 +641,10 @@ __device__ __forceinline__ void update_one(const DevMesh<A> &m, int c, CellIn<A>
 //
 // Bound by issue (3.1 M warp instructions at 207,234 cells, half of them fp64
 // chains: a power, a square root and three quotients per cell) and by the tail:
-// 1,620 CTAs are 1.37 waves of 8 per SM and 1.82 of 6, and the step takes
-// 14.1 us with the first, 13.7 us with the second.  The constants' early loads:
-// 14.5 -> 14.1 us (8 per SM).
+// 1,620 CTAs are 1.37 waves of 8 per SM.  The constants' early loads: 14.5 ->
+// 14.1 us per step.  Shapes (flux, cell CTAs per SM), 207,234-cell channel /
+// mixed mesh / dam break / 2,000,000-cell dam break: (8, 8) 13.6 / 15.9 / 17.1 /
+// 141.8 us, (7, 6) 13.9 / 15.9 / 17.5 / 141.9, (7, 8) 13.7 / 15.9 / 16.6 / 143.4.
 template <class A, int VARIANT, int UMINB, bool SEG, bool COEF = false>
 __global__ void __launch_bounds__(UPDATE_THREADS, UMINB) update_kernel(DevMesh<A> m, int k, int write_flux) {
     // batches: the flux segments run forward, so the cells run reversed
