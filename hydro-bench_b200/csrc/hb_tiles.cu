@@ -2,6 +2,7 @@
 // the mesh's tiles, at the launch shape the handle holds.  A translation unit
 // of its own so the library's kernels compile in parallel.
 #include <algorithm>
+#include <mutex>
 #include <type_traits>
 
 #include "hb_handle.hpp"
@@ -49,6 +50,20 @@ int launch_tiles_t(hb_handle *h, hb::DevMesh<A> m, int n, cudaStream_t st) {
     return hb_launch_tick(h, n, st);
 }
 
+// Lets a tile kernel take `bytes` of shared memory.  The limit belongs to the
+// kernel, so every handle of the process shares it: it is only ever raised (a
+// smaller one would fail the launches of a handle with larger tiles).
+template <class Kernel>
+int raise_tile_smem(Kernel kernel, size_t bytes) {
+    static std::mutex lock;
+    std::lock_guard<std::mutex> hold(lock);
+    cudaFuncAttributes at{};
+    HB_CUDA_RET(cudaFuncGetAttributes(&at, kernel));
+    if ((size_t)at.maxDynamicSharedSizeBytes >= bytes) return HB_OK;
+    HB_CUDA_RET(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    return HB_OK;
+}
+
 // Lets every tile kernel of the handle's policy use the shared memory its
 // largest tile needs (beyond the 48 KB default).
 template <class A, int VARIANT>
@@ -56,10 +71,7 @@ int set_tile_smem(const hb::DevMesh<A> &m) {
     const size_t bytes = tile_smem_bytes(m.max_tile_cells, m.max_tile_queue, sizeof(typename A::real));
     for (int c = 0; c < hb::N_LAUNCH_CONFIGS; c++) {
         if (hb::LAUNCH_CONFIGS[c].layout != hb::LAYOUT_TILE) continue;
-        const int rc = with_tile_kernel<A, VARIANT>(c, [&](auto kernel, int) -> int {
-            HB_CUDA_RET(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-            return HB_OK;
-        });
+        const int rc = with_tile_kernel<A, VARIANT>(c, [&](auto kernel, int) { return raise_tile_smem(kernel, bytes); });
         if (rc != HB_OK) return rc;
     }
     return HB_OK;
@@ -84,7 +96,7 @@ int hb_tiles_resident(hb_handle *h, int config, int tile_cells, int *per_sm) {
         using A = typename std::remove_reference<decltype(m)>::type::Policy;
         const size_t bytes = tile_smem_bytes(cells, 3 * cells, sizeof(typename A::real));
         auto query = [&](auto kernel, int threads) -> int {
-            HB_CUDA_RET(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+            TRY(raise_tile_smem(kernel, bytes));
             HB_CUDA_RET(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, threads, bytes));
             return HB_OK;
         };
