@@ -610,9 +610,8 @@ struct SlotLin {
 __device__ __forceinline__ void linearise_osher(const CellStateA<A> &L, const CellStateA<A> &R, double cs, double sn,
                                                 bool mir, const StepParams &p, SlotLin &s) {
     s.kind = L.h <= p.hm1 && R.h <= p.hm1 ? LIN_ZERO : LIN_GENERAL;
-    const double HMX = fmax(p.hm1, p.hm2);
     const double qr0 = A::depth(R.z, L.zbc);
-    if (!(L.h > HMX && R.h > HMX && qr0 > HMX && L.z > R.zbc && R.z > R.zbc)) return;
+    if (!(edge_deep<A>(L, R, qr0, p) && R.z > R.zbc)) return;
     const double cl = A::sqrt(A::mul(A::c(9.81), L.h)), cr = A::sqrt(A::mul(A::c(9.81), qr0));
     const double q = A::div(R.h, qr0), ratio = A::fmin(q, A::c(1.5));
     const double ql1 = A::dot(L.u, cs, L.v, sn, M_QL1);

@@ -794,17 +794,27 @@ __device__ __forceinline__ void flux_slot(const SlotInA<A> &in, typename A::real
     else { o.f[0] = -fo[0]; o.f[3] = mirror_f3<A>(fo[3], in.nb.zbc, in.own.zbc); }
 }
 
+// Whether the edge from the lower-numbered cell a to b, with QR[0] = qr0, is deep
+// enough for both sides' branch chains to reach Osher and for its inputs
+// (osher_inputs) to take none of their bounds: both depths and QR[0] above HM1 and
+// HM2 (so max(H, HM1) = H and QR[1] is not the thin-water value), the right level
+// above its bed (so max(ZBC, Z) = Z), and each side's level above the other's bed
+// (which QR[0] > HM1 does not say where HM1 is negative).  The forward's common
+// case and the adjoint's share this test.
+template <class A>
+__device__ __forceinline__ bool edge_deep(const CellStateA<A> &a, const CellStateA<A> &b, typename A::real qr0,
+                                          const StepParams &p) {
+    using R = typename A::real;
+    const R HMX = A::c(fmax(p.hm1, p.hm2));
+    return a.h > HMX && b.h > HMX && qr0 > HMX && b.z > a.zbc && a.z > b.zbc && b.z >= b.zbc;
+}
+
 // The common case of an interior slot (code 0) across an edge from the
 // lower-numbered cell a to b, by the direct route (the slot of a) or the
 // mirrored one (that of b); (cosj, sinj) is the slot's own normal.  Both cells
-// deep and the flow across the edge subcritical, or both dry; false, and no
-// result, in any other case.  Deep enough: for both sides' branch chains to
-// reach Osher and for its inputs (osher_inputs) to take none of their bounds:
-// both depths and QR[0] above HM1 and HM2 (so max(H, HM1) = H and QR[1] is not
-// the thin-water value), the right level above its bed (so max(ZBC, Z) = Z), and
-// each side's level above the other's bed (of which QR[0] > 0 is one).  The
-// caller loads the cells in this order: selecting their five values instead
-// costs forty selects.
+// deep (edge_deep) and the flow across the edge subcritical, or both dry; false,
+// and no result, in any other case.  The caller loads the cells in this order:
+// selecting their five values instead costs forty selects.
 template <class A>
 __device__ __forceinline__ bool slot_common(const CellStateA<A> &a, const CellStateA<A> &b, bool direct,
                                             typename A::real cosj, typename A::real sinj, const StepParams &p,
@@ -812,9 +822,8 @@ __device__ __forceinline__ bool slot_common(const CellStateA<A> &a, const CellSt
     using R = typename A::real;
     using L = typename A::level;
     const R cs = direct ? cosj : -cosj, sn = direct ? sinj : -sinj;
-    const R HMX = A::c(fmax(p.hm1, p.hm2));
     const R qr0 = A::depth(b.z, a.zbc);
-    if (!(a.h > HMX && b.h > HMX && qr0 > HMX && a.z > b.zbc && b.z >= b.zbc)) {
+    if (!edge_deep<A>(a, b, qr0, p)) {
         f[0] = f[1] = f[2] = f[3] = R(0);
         return a.h <= A::c(p.hm1) && b.h <= A::c(p.hm1);   // both dry
     }

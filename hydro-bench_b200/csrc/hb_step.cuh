@@ -356,14 +356,8 @@ __device__ __forceinline__ void pair_record(const DevMesh<A> &m, int r, const Re
     using L = typename A::level;
     const CellStateA<A> a = load_cell(m, si.par, q.a), b = load_cell(m, si.par, q.b);
     const R cs = q.g.x, sn = q.g.y, side = q.g.z;
-    // Deep enough for both branch chains (functors.cu:98-150) to reach Osher and
-    // for its inputs (osher_inputs) to take none of their bounds: both depths
-    // and QR[0] above HM1 and HM2 (so max(H, HM1) = H and QR[1] is not the
-    // thin-water value), the right level above its bed (so max(ZBC, Z) = Z),
-    // and each side's level above the other's bed (of which QR[0] > 0 is one).
-    const R HMX = A::c(fmax(p.hm1, p.hm2));
     const R qr0 = A::depth(b.z, a.zbc);
-    if (a.h > HMX && b.h > HMX && qr0 > HMX && a.z > b.zbc && b.z >= b.zbc) {
+    if (edge_deep<A>(a, b, qr0, p)) {
         const R cl = A::sqrt(A::mul(A::c(9.81), a.h)), cr = A::sqrt(A::mul(A::c(9.81), qr0));
         const R ratio = A::fmin(A::div(b.h, qr0), A::c(1.5));
         const R ql1 = A::dot(a.u, cs, a.v, sn, M_QL1), ql2 = A::dot(a.v, cs, -a.u, sn, M_QL2);
