@@ -265,14 +265,16 @@ __device__ __forceinline__ void single_core(const DevMesh<A> &m, int r, int a, i
     const R cl = A::sqrt(A::mul(A::c(9.81), in.own.h));
     SlotOut<R> o;
     flux_slot<A, VARIANT>(in, cl, p, fetch, o);
-    if (o.mask != 0xF) {   // codes that leave fluxes unwritten keep the old values (functors.cu:525-565)
+    // A code that leaves fluxes unwritten keeps the old values (functors.cu:525-565),
+    // so it stores all four at every step, also where a supercritical one wrote them.
+    if (o.mask != 0xF) {
         const Vec4<R> old = ldg4(m.flux + 4 * (size_t)sa);
         if (!(o.mask & 1)) o.f[0] = old.x;
         if (!(o.mask & 2)) o.f[1] = old.y;
         if (!(o.mask & 4)) o.f[2] = old.z;
         if (!(o.mask & 8)) o.f[3] = old.w;
     }
-    if (write_flux || o.mask != 0xF) store_flux(m, sa, o.f);
+    if (write_flux || in.code == CODE_BOUNDA_OTHER) store_flux(m, sa, o.f);
     store_terms<A>(tout, sa, o.f, in.side, in.cosj, in.sinj);
     if (o.klas_to_zero) m.rmeta[r] = (uint8_t)((meta & ~META_CODE) | CODE_ZERO);
     if (o.undefined) atomicOr(m.err, ERRBIT_UNDEFINED);
