@@ -640,12 +640,12 @@ int launch_steps_t(hb_handle *h, hb::DevMesh<A> m, int n, cudaStream_t st) {
     int rc;
     using namespace hb;
     switch (h->launch_config) {
-    case 0: rc = go(flux_kernel<A, VARIANT, 128, 8, SEG>, 128, update_kernel<A, VARIANT, 8, SEG>); break;
+    case 0: rc = go(flux_kernel<A, VARIANT, 128, 7, SEG>, 128, update_kernel<A, VARIANT, 8, SEG>); break;
     case 1: rc = go(flux_kernel<A, VARIANT, 128, 6, SEG>, 128, update_kernel<A, VARIANT, 8, SEG>); break;
-    case 2: rc = go(flux_kernel<A, VARIANT, 128, 7, SEG>, 128, update_kernel<A, VARIANT, 6, SEG>); break;
+    case 2: rc = go(flux_kernel<A, VARIANT, 128, 8, SEG>, 128, update_kernel<A, VARIANT, 8, SEG>); break;
     case 3: rc = go(flux_kernel<A, VARIANT, 256, 3, SEG>, 256, update_kernel<A, VARIANT, 6, SEG>); break;
     case 4: rc = go(flux_kernel<A, VARIANT, 256, 4, SEG>, 256, update_kernel<A, VARIANT, 8, SEG>); break;
-    case 5: rc = go(flux_kernel<A, VARIANT, 128, 7, SEG>, 128, update_kernel<A, VARIANT, 8, SEG>); break;
+    case 5: rc = go(flux_kernel<A, VARIANT, 128, 7, SEG>, 128, update_kernel<A, VARIANT, 6, SEG>); break;
     case 6: rc = go(flux_kernel<A, VARIANT, 256, 2, SEG>, 256, update_kernel<A, VARIANT, 6, SEG>); break;
     case 7: rc = go(flux_kernel<A, VARIANT, 64, 12, SEG>, 64, update_kernel<A, VARIANT, 8, SEG>); break;
     case 14: rc = go(flux_kernel<A, VARIANT, 128, 6, SEG>, 128, update_kernel<A, VARIANT, 6, SEG>); break;
@@ -727,16 +727,16 @@ int enqueue_steps(hb_handle *h, int n, cudaStream_t st) {
     });
 }
 
-int default_config(int layout, int precision) {
-    if (layout != HB_LAYOUT_TILE) return hb::DEFAULT_EDGE_CONFIG;
-    return precision == HB_FP64 ? hb::DEFAULT_TILE_CONFIG_FP64 : hb::DEFAULT_TILE_CONFIG;
+int default_config(const hb_options &o) {
+    if (o.layout != HB_LAYOUT_TILE) return o.persistent ? hb::PERSISTENT_CONFIG : hb::DEFAULT_EDGE_CONFIG;
+    return o.precision == HB_FP64 ? hb::DEFAULT_TILE_CONFIG_FP64 : hb::DEFAULT_TILE_CONFIG;
 }
 
-// launch shape index of tile_config (0 = the layout's default), or -1
-int config_for(int layout, int precision, int tile_config) {
-    if (tile_config == 0) return default_config(layout, precision);
+// launch shape index of tile_config (0 = the handle's default), or -1
+int config_for(const hb_options &o, int tile_config) {
+    if (tile_config == 0) return default_config(o);
     if (tile_config < 0 || tile_config > hb::N_LAUNCH_CONFIGS) return -1;
-    return hb::LAUNCH_CONFIGS[tile_config - 1].layout == layout ? tile_config - 1 : -1;
+    return hb::LAUNCH_CONFIGS[tile_config - 1].layout == o.layout ? tile_config - 1 : -1;
 }
 
 int check_range(hb_handle *h, long long n) {
@@ -829,11 +829,11 @@ extern "C" int hb_create_batch(const hb_mesh_desc *meshes, int32_t n, const hb_o
         return hb::set_error(HB_E_INVALID, "hb_create: layout %d", opt.layout);
     if (opt.tile_cells < 0 || opt.tile_cells > 1024)   // 5/4 x 1024 fp64 cells: 160 KB of shared memory
         return hb::set_error(HB_E_INVALID, "hb_create: tile_cells %d outside 0..1024", opt.tile_cells);
-    if (config_for(opt.layout, opt.precision, opt.tile_config) < 0)
+    if (config_for(opt, opt.tile_config) < 0)
         return hb::set_error(HB_E_INVALID, "hb_create: tile_config %d is no shape of layout %d", opt.tile_config, opt.layout);
     if (opt.persistent != 0 && opt.persistent != 1)
         return hb::set_error(HB_E_INVALID, "hb_create: persistent %d", opt.persistent);
-    if (opt.persistent && (opt.layout != HB_LAYOUT_EDGE || config_for(opt.layout, opt.precision, opt.tile_config) != hb::DEFAULT_EDGE_CONFIG))
+    if (opt.persistent && (opt.layout != HB_LAYOUT_EDGE || config_for(opt, opt.tile_config) != hb::PERSISTENT_CONFIG))
         return hb::set_error(HB_E_INVALID, "hb_create: a persistent handle takes the edge layout's default launch shape");
     long long total = 0;
     for (int s = 0; s < n; s++) total += std::max(meshes[s].cells, 0);
@@ -841,7 +841,7 @@ extern "C" int hb_create_batch(const hb_mesh_desc *meshes, int32_t n, const hb_o
     HB_CUDA_RET(cudaSetDevice(opt.device));
     auto h = new hb_handle();
     h->opt = opt;
-    h->launch_config = config_for(opt.layout, opt.precision, opt.tile_config);
+    h->launch_config = config_for(opt, opt.tile_config);
     h->tile_cells = opt.tile_cells > 0 ? opt.tile_cells : 256;
     if (opt.layout == HB_LAYOUT_TILE && opt.tile_cells == 0 && opt.precision != HB_FP64) {
         // balanced default (fp32 state): about 512 cells per tile, adjusted so
@@ -1173,9 +1173,9 @@ extern "C" int hb_get_permutation_at(hb_handle *h, int32_t s, int32_t *perm) {
 
 extern "C" int hb_set_tile_config(hb_handle *h, int32_t tile_config) {
     if (!h) return hb::set_error(HB_E_INVALID, "null handle");
-    const int c = config_for(h->opt.layout, h->opt.precision, tile_config);
+    const int c = config_for(h->opt, tile_config);
     if (c < 0) return hb::set_error(HB_E_INVALID, "tile_config %d is no shape of this handle's layout", tile_config);
-    if (h->opt.persistent && c != hb::DEFAULT_EDGE_CONFIG)
+    if (h->opt.persistent && c != hb::PERSISTENT_CONFIG)
         return hb::set_error(HB_E_INVALID, "a persistent handle keeps the default launch shape");
     if (c != h->launch_config) h->drop_graph();
     h->launch_config = c;
