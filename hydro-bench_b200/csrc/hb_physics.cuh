@@ -354,26 +354,32 @@ __device__ __forceinline__ void osher(typename A::real cl, const typename A::rea
     if (p7) qf_acc<A>(out, false, qr[0], qr[1], qr[2]);
 }
 
-// The case of subcritical flow across the edge (K1 = 1, K2 = 2 or 3), which
-// adds piece 3 or piece 5 alone: osher()'s result for it, from `cr` =
-// sqrt(9.81*QR[0]).  False (and no result) in any other case, at UA = -CA, and
-// where CA leaves the range in which the policy's quotients by a constant need
-// no checks (quotient_range): with CA in it, D = +-2 CA, HA and FLUX3 are in
-// divk_raw's range too.
+// The cases of osher() that add one piece alone: subcritical flow across the edge
+// (K1 = 1, K2 = 2 or 3: piece 3 or 5) and supercritical flow either way (K1 = 2,
+// K2 = 1: piece 1; K1 = 3, K2 = 4: piece 7).  osher()'s result for them, from `cr`
+// = sqrt(9.81*QR[0]).  False (and no result) in any other case, at UA = -CA, and
+// where a depth or CA leaves the range in which the policy's quotients by a
+// constant need no checks (quotient_range): with CA or the depth in it, HA and
+// FLUX3 are in divk_raw's range too.
 template <class A>
-__device__ __forceinline__ bool osher_subcritical(typename A::real cl, typename A::real cr, typename A::real ql1,
-                                                  typename A::real ql2, typename A::real qr1, typename A::real qr2,
-                                                  typename A::real fil, typename A::real out[4]) {
+__device__ __forceinline__ bool osher_one_piece(typename A::real cl, typename A::real cr, const typename A::real ql[3],
+                                                const typename A::real qr[3], typename A::real fil,
+                                                typename A::real out[4]) {
     using R = typename A::real;
-    const R fir = A::sub(qr1, A::mul(A::c(2.0), cr));
+    const R fir = A::sub(qr[1], A::mul(A::c(2.0), cr));
     const R ua = A::mul(A::add(fil, fir), A::c(0.5));
     const R ca = A::fabs(A::mul(A::sub(fil, fir), A::c(0.25)));
     const bool p3 = A::nonnegative(ua);   // FIL + FIR is never -0
     const R d = A::sub(p3 ? fil : fir, ua);
-    const R ha = A::divk_raw(A::mul(d, d), 39.24);
+    R h = A::divk_raw(A::mul(d, d), 39.24), u = ua, v = p3 ? ql[2] : qr[2];
+    bool one = ql[1] < cl && qr[1] >= -cr && A::fabs(ua) < ca && A::quotient_range(ca);
+    if (!one) {
+        if (ca < ua && ql[1] >= cl && qr[1] >= -cr) { h = ql[0]; u = ql[1]; v = ql[2]; one = A::quotient_range(h); }
+        if (ua < -ca && ql[1] < cl && qr[1] < -cr) { h = qr[0]; u = qr[1]; v = qr[2]; one = A::quotient_range(h); }
+    }
     out[0] = out[1] = out[2] = out[3] = R(0);
-    qf_acc<A>(out, false, ha, ua, p3 ? ql2 : qr2);
-    return ql1 < cl && qr1 >= -cr && A::fabs(ua) < ca && A::quotient_range(ca);
+    qf_acc<A>(out, false, h, u, v);
+    return one;
 }
 
 // ---------------------------------------------------------------------------
@@ -614,8 +620,6 @@ __device__ __forceinline__ void bounda(const SlotInA<A> &in, const StepParams &p
 
 // ---------------------------------------------------------------------------
 // CalculateFluxKernel body for one slot, functors.cu:47-202
-// `cl_own` is sqrt(9.81*H) of the slot's cell (the caller may compute it once
-// per cell; it is bit-identical to the reference's per-slot value).
 //
 // ZERO_LEN: the slot is a zero-length edge without neighbour (the unused
 // fourth slot of a triangle, mesh.cpp:303-306), and only its contribution
@@ -634,8 +638,7 @@ __device__ __forceinline__ typename A::real pow15(typename A::real x) {
 // slot's fluxes are final (returns 0, `o` filled) or it needs Osher across the
 // edge: 1 = direct (functors.cu:151-164), 2 = mirrored (:165-200).
 template <class A, int VARIANT, class TableFetch, bool ZERO_LEN = false>
-__device__ __forceinline__ int flux_chain(const SlotInA<A> &in, typename A::real cl_own,
-                                          const StepParams &p, const TableFetch &fetch,
+__device__ __forceinline__ int flux_chain(const SlotInA<A> &in, const StepParams &p, const TableFetch &fetch,
                                           SlotOut<typename A::real> &o) {
     using R = typename A::real;
     using L = typename A::level;
@@ -660,7 +663,7 @@ __device__ __forceinline__ int flux_chain(const SlotInA<A> &in, typename A::real
         vc = in.nb.v;
     }
     if (code_is_bounda(in.code)) {
-        R fil = A::add(ql[1], A::mul(A::c(2.0), cl_own));
+        R fil = A::add(ql[1], A::mul(A::c(2.0), A::sqrt(A::mul(A::c(9.81), h1))));
         bounda<A, VARIANT>(in, p, fil, ql, zc, uc, vc, fetch, o);
     } else if (h1 <= HM1 && hc <= HM1) {
         o.f[0] = R(0); o.f[1] = R(0); o.f[2] = R(0); o.f[3] = R(0);
@@ -771,20 +774,17 @@ __device__ __forceinline__ typename A::real mirror_f3(typename A::real fo3, type
 }
 
 // CalculateFluxKernel body for one slot, functors.cu:47-202.
-// `cl_own` is sqrt(9.81*H) of the slot's cell (the caller may compute it once
-// per cell; it is bit-identical to the reference's per-slot value).
 template <class A, int VARIANT, class TableFetch, bool ZERO_LEN = false>
-__device__ __forceinline__ void flux_slot(const SlotInA<A> &in, typename A::real cl_own,
-                                          const StepParams &p, const TableFetch &fetch,
+__device__ __forceinline__ void flux_slot(const SlotInA<A> &in, const StepParams &p, const TableFetch &fetch,
                                           SlotOut<typename A::real> &o) {
     using R = typename A::real;
-    const int route = flux_chain<A, VARIANT, TableFetch, ZERO_LEN>(in, cl_own, p, fetch, o);
+    const int route = flux_chain<A, VARIANT, TableFetch, ZERO_LEN>(in, p, fetch, o);
     if (route == 0) return;
     const bool mir = route == 2;
     const CellStateA<A> &L = mir ? in.nb : in.own;
     const CellStateA<A> &Rc = mir ? in.own : in.nb;
     const R cs = mir ? -in.cosj : in.cosj, sn = mir ? -in.sinj : in.sinj;
-    const R clL = mir ? A::sqrt(A::mul(A::c(9.81), in.nb.h)) : cl_own;
+    const R clL = A::sqrt(A::mul(A::c(9.81), L.h));
     const OsherIn<R> oi = osher_inputs<A>(L, Rc, cs, sn, clL, mir, p);
     R fo[4];
     osher<A>(oi.cl, oi.ql, oi.qr, oi.fil, fo);
@@ -834,7 +834,8 @@ __device__ __forceinline__ bool slot_common(const CellStateA<A> &a, const CellSt
     const R ur = direct ? A::dot(b.u, cs, b.v, sn, M_UR) : A::dot(b.u, cs, b.v, sn, M_UR1);
     const R qr2 = A::dot(b.v, cs, -b.u, sn, M_QR2);
     const R fil = A::add(ql1, A::mul(A::c(2.0), cl));
-    if (!osher_subcritical<A>(cl, cr, ql1, ql2, A::mul(ur, ratio), qr2, fil, f)) return false;
+    const R ql[3] = {a.h, ql1, ql2}, qr[3] = {qr0, A::mul(ur, ratio), qr2};
+    if (!osher_one_piece<A>(cl, cr, ql, qr, fil, f)) return false;
     f[1] = osher_f1<A>(f[1], ratio, b.h, ur);
     if (!direct) {
         f[0] = -f[0];

@@ -47,9 +47,8 @@ __device__ __forceinline__ void ref_slot(const typename RefView<typename A::real
         b.nhq = m.NHQ;
         return b;
     };
-    const R cl = A::sqrt(A::mul(A::c(9.81), in.own.h));
     SlotOut<R> o;
-    flux_slot<A, VARIANT>(in, cl, p, fetch, o);
+    flux_slot<A, VARIANT>(in, p, fetch, o);
     if (o.undefined) atomicOr(&g_ref_errors, ERRBIT_UNDEFINED);
     if (o.klas_to_zero) sd.KLAS[idx] = R(0);
     if (o.mask & 1) sd.FLUX0[idx] = o.f[0];
@@ -68,10 +67,13 @@ __device__ __forceinline__ void ref_slot(const typename RefView<typename A::real
 // Bound by the gathers' latency and by issue.  207,234 triangles, flux kernel
 // alone: every slot through the whole chain in place 36 us and more, the common
 // case in place and the rest in the queue 35.5 us (11.4 M warp instructions),
-// sorted 26.4 us (9.6 M); the pair of calls 42.6 -> 29.5 us.
+// sorted 26.4 us (9.6 M); the pair of calls 42.6 -> 29.5 us.  8 CTAs per SM (64
+// registers) instead of 7, with the general slots' square root only where it is
+// used: the pair of calls 30.0 -> 28.9 us, thin sheet flow 45.6 -> 41.2 us (41.5
+// with the chain in place), supercritical 41.2 -> 30.6 us.
 constexpr int REF_THREADS = 128;
 template <class A, int VARIANT>
-__global__ void __launch_bounds__(REF_THREADS, 7) ref_flux_kernel(const __grid_constant__
+__global__ void __launch_bounds__(REF_THREADS, 8) ref_flux_kernel(const __grid_constant__
                                                                typename RefView<typename A::real>::type m,
                                                                int kt, int jt) {
     using R = typename A::real;
@@ -115,7 +117,7 @@ __global__ void __launch_bounds__(REF_THREADS, 7) ref_flux_kernel(const __grid_c
         }
     }
     __syncthreads();
-    for (int q = t; q < qn; q += REF_THREADS) ref_slot<A, VARIANT>(m, queue[q], kt, jt);
+    if (t < qn) ref_slot<A, VARIANT>(m, queue[t], kt, jt);
 }
 
 // The four values of a cell in a slot array: one vector load where every slot
@@ -340,7 +342,7 @@ __global__ void __launch_bounds__(256) static_flux_kernel(hb_ref_mesh_view m, in
         return b;
     };
     SlotOut<double> o;
-    flux_slot<A, VARIANT>(in, A::sqrt(A::mul(9.81, in.own.h)), p, fetch, o);
+    flux_slot<A, VARIANT>(in, p, fetch, o);
     if (o.undefined) atomicOr(&g_ref_errors, ERRBIT_UNDEFINED);
     if (o.klas_to_zero) sd.KLAS[idx] = 0.0;
     // fluxes this slot does not write keep their values (functors.cu:525-565)

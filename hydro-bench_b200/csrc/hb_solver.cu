@@ -658,14 +658,18 @@ int launch_steps_t(hb_handle *h, hb::DevMesh<A> m, int n, cudaStream_t st) {
 }
 
 // Persistent handles: the whole sequence as cooperative launches of
-// persistent_kernel (128 threads, 6 CTAs per SM), as many CTAs as are
+// persistent_kernel (128 threads, 4 CTAs per SM), as many CTAs as are
 // resident at once, each launch preceded by zeroing its barrier words.
 // A launch takes at most PERSIST_MAX_STEPS steps, and fewer where its grid
 // is larger: every step adds 2 x grid arrivals to the 32-bit arrival count,
 // which must stay below 2^32 (phantom arrivals included) so that no barrier
 // target wraps.  Longer sequences take several launches; the extra flux
 // writes at the end of each launch leave the same final fluxes.
-constexpr int PERSIST_THREADS = 128, PERSIST_MINB = 6, PERSIST_MAX_STEPS = 1 << 20;
+// 4 CTAs per SM hold the fp64 kernel without spills.  us per step, 207,234 cells,
+// 4 / 5 / 6 per SM: channel 23.5 / 25.0 / 24.1, all cells between HM1 and HM2
+// 36.2 / 35.2 / 34.4; split 16.3 / 16.4 / 17.9 and 23.7 / 23.9 / 24.8; 1,000,000
+// cells fp64 96.8 / 94.9 / 98.2; 24,021 cells 9.9 / 10.0 / 10.4.
+constexpr int PERSIST_THREADS = 128, PERSIST_MINB = 4, PERSIST_MAX_STEPS = 1 << 20;
 
 // Steps one cooperative launch of `grid` CTAs may take (>= 1).
 inline int persist_steps_per_launch(unsigned grid, unsigned phantom) {

@@ -264,9 +264,8 @@ __device__ __forceinline__ void single_core(const DevMesh<A> &m, int r, int a, i
         bi.nhq = m.nhq;
         return bi;
     };
-    const R cl = A::sqrt(A::mul(A::c(9.81), in.own.h));
     SlotOut<R> o;
-    flux_slot<A, VARIANT>(in, cl, p, fetch, o);
+    flux_slot<A, VARIANT>(in, p, fetch, o);
     // A code that leaves fluxes unwritten keeps the old values (functors.cu:525-565),
     // so it stores all four at every step, also where a supercritical one wrote them.
     if (o.mask != 0xF) {
@@ -313,9 +312,9 @@ __device__ __forceinline__ Record<A> load_record(const DevMesh<A> &m, int r) {
 
 // One side of record r on its own: a single record's slot, or slot a
 // (item = 2r) or b (item = 2r + 1) of a pair, computed as the reference
-// computes every slot.
+// computes every slot.  of_pair: the record is known to be a pair.
 template <class A, int VARIANT, class T>
-__device__ __forceinline__ void side_record(const DevMesh<A> &m, int item, const StepIndex &si,
+__device__ __forceinline__ void side_record(const DevMesh<A> &m, int item, bool of_pair, const StepIndex &si,
                                             const StepParams &p, int write_flux, const T &tout) {
     using R = typename A::real;
     using L = typename A::level;
@@ -323,7 +322,7 @@ __device__ __forceinline__ void side_record(const DevMesh<A> &m, int item, const
     const bool other = item & 1;
     const Record<A> q = load_record(m, r);
     Vec4<R> g = q.g;
-    uint8_t meta = m.rmeta[r];
+    uint8_t meta = of_pair ? (uint8_t)(CODE_ZERO | META_OWN_FIRST | META_HAS_NB) : m.rmeta[r];
     int c = q.a, n = q.b, s = q.sa;
     if (other) {   // negated normal, not the lower-numbered side
         c = q.b; n = q.a; s = q.sb;
@@ -337,30 +336,74 @@ __device__ __forceinline__ void side_record(const DevMesh<A> &m, int item, const
     single_core<A, VARIANT>(m, r, c, s, own, nb, meta, g, timed ? with_time(p, si) : p, write_flux, tout);
 }
 
+// One side of a pair on its own (item as above), without the boundary codes.
+template <class A, int VARIANT, class T>
+__device__ __forceinline__ void pair_side(const DevMesh<A> &m, int item, const StepIndex &si,
+                                          const StepParams &p, int write_flux, const T &tout) {
+    const bool other = item & 1;
+    const Record<A> q = load_record(m, item >> 1);
+    SlotInA<A> in;
+    in.own = load_cell(m, si.par, other ? q.b : q.a);
+    in.nb = load_cell(m, si.par, other ? q.a : q.b);
+    in.has_nb = true; in.own_first = !other; in.code = CODE_ZERO;
+    in.cosj = other ? -q.g.x : q.g.x; in.sinj = other ? -q.g.y : q.g.y; in.side = q.g.z;
+    const int s = other ? q.sb : q.sa;
+    SlotOut<typename A::real> o;
+    flux_slot<A, VARIANT>(in, p, []() { return BoundaryInA<A>{}; }, o);
+    if (write_flux) store_flux(m, s, o.f);
+    store_terms<A>(tout, s, o.f, in.side, in.cosj, in.sinj);
+}
+
+// The sides that a CTA computes after its main pass (side_record's items): entry i
+// of the front has its partner, or -1, in entry i of the back.  The two sides of
+// an edge take different branches of the chain (the lower one the inflow, the
+// higher one the weir's power) or different Osher routes, so they are kept apart
+// and a warp runs one of them: the thin sheet's flux kernel 16.2 -> 11.2 M warp
+// instructions.
+struct SideQueue {
+    int *e;
+    int cap;    // entries; a pair takes two, and so does a single
+    int *n;     // entries in the front, shared by the CTA
+    __device__ __forceinline__ void push(int front, int back) const {
+        const int i = atomicAdd(n, 1);
+        e[i] = front;
+        e[cap - 1 - i] = back;
+    }
+    __device__ __forceinline__ int item(int j, int count) const { return j < count ? e[j] : e[cap - 1 - (j - count)]; }
+};
+
 // One mirror-pair record: both sides' fluxes where both cells are deep and
-// the flow across the edge is subcritical (or both are dry), the bulk of any
-// mesh.  The two routes (functors.cu:151-200) have the same cells, normal and
-// inputs except two rotations that the reference build rounds differently
-// (policies with route_modes), so they share the square roots, the depth ratio
-// and their quotients, and each runs osher_subcritical from its own FIR.
-// Every other pair puts its two sides into the CTA's queue, which runs after
-// the main pass (side_record).  So the main pass holds neither the powers of
-// the one-sided branches nor Osher's other pieces.
+// Osher takes one piece (osher_one_piece: subcritical flow across the edge, or
+// supercritical either way), or both are dry: the bulk of any mesh.  The two
+// routes (functors.cu:151-200) have the same cells, normal and inputs except two
+// rotations that the reference build rounds differently (policies with
+// route_modes), so they share the square roots, the depth ratio and their
+// quotients, and each runs osher_one_piece from its own FIR.  Every other pair
+// puts its two sides into the CTA's queue, which runs after the main pass.  So
+// the main pass holds neither the powers of the one-sided branches nor Osher's
+// other pieces.
 //
 // Bound by the gathers' latency and by issue.  207,234 cells, flux kernel, warp
 // instructions per launch: both branch chains, Osher in full and a queue of
-// mirrored evaluations 7.47 M; this form 4.0 M, and 3.0 M after its comparisons
-// were cut to those below.  Step 22.2 -> 15.9 -> 14.4 us, 2M-cell dam break
-// 181 -> 153 -> 148 us; with one-load records and their loads ahead of the
-// dependency wait 14.0 and 146 us.
+// mirrored evaluations 7.5 M; this form 3.6 M, of which the supercritical pieces
+// are 0.2 M.  Step, still / supercritical / patchy wet and dry / thin sheet
+// (all cells between HM1 and HM2) flow, us: that whole form 25.4 / 27.0 / 33.3 /
+// 28.5; subcritical alone in the main pass, the two sides of an edge next to
+// each other in one queue of general slots 15.6 / 28.5 / 26.3 / 33.6; this form
+// 15.6 / 20.0 / 25.6 / 28.0.  Taken back: pairs instead of sides in the queue
+// (15.4 / 28.4 / 28.6 / 29.9: half of the threads idle where half of the pairs
+// are queued) and the chain of thin pairs in the main pass (16.5 / 21.1 / 29.9 /
+// 27.5).
 template <class A, class T>
 __device__ __forceinline__ void pair_record(const DevMesh<A> &m, int r, const Record<A> &q, const StepIndex &si,
-                                            const StepParams &p, int write_flux, const T &tout, int *queue, int *qn) {
+                                            const StepParams &p, int write_flux, const T &tout,
+                                            const SideQueue &queue) {
     using R = typename A::real;
     using L = typename A::level;
     const CellStateA<A> a = load_cell(m, si.par, q.a), b = load_cell(m, si.par, q.b);
     const R cs = q.g.x, sn = q.g.y, side = q.g.z;
     const R qr0 = A::depth(b.z, a.zbc);
+    bool low = true;   // a's side goes to the queue's front
     if (edge_deep<A>(a, b, qr0, p)) {
         const R cl = A::sqrt(A::mul(A::c(9.81), a.h)), cr = A::sqrt(A::mul(A::c(9.81), qr0));
         const R ratio = A::fmin(A::div(b.h, qr0), A::c(1.5));
@@ -369,11 +412,14 @@ __device__ __forceinline__ void pair_record(const DevMesh<A> &m, int r, const Re
         const R fil = A::add(ql1, A::mul(A::c(2.0), cl));
         const R ur = A::dot(b.u, cs, b.v, sn, M_UR);
         R fa[4], fb[4];
-        bool ok = osher_subcritical<A>(cl, cr, ql1, ql2, A::mul(ur, ratio), qr2, fil, fa);
+        R ql[3] = {a.h, ql1, ql2}, qr[3] = {qr0, A::mul(ur, ratio), qr2};
+        bool ok = osher_one_piece<A>(cl, cr, ql, qr, fil, fa);
         R urm = ur;
         if constexpr (A::route_modes) {
             urm = A::dot(b.u, cs, b.v, sn, M_UR1);
-            ok &= osher_subcritical<A>(cl, cr, ql1, A::dot(a.v, cs, -a.u, sn, M_QL2M), A::mul(urm, ratio), qr2, fil, fb);
+            ql[2] = A::dot(a.v, cs, -a.u, sn, M_QL2M);
+            qr[1] = A::mul(urm, ratio);
+            ok &= osher_one_piece<A>(cl, cr, ql, qr, fil, fb);
         } else {
 #pragma unroll
             for (int i = 0; i < 4; i++) fb[i] = fa[i];
@@ -398,20 +444,22 @@ __device__ __forceinline__ void pair_record(const DevMesh<A> &m, int r, const Re
         store_terms<A>(tout, q.sa, f, side, cs, sn);
         store_terms<A>(tout, q.sb, f, side, -cs, -sn);
         return;
+    } else {
+        low = a.z < b.z;
     }
-    const int i = atomicAdd(qn, 2);
-    queue[i] = 2 * r;
-    queue[i + 1] = 2 * r + 1;
+    queue.push(low ? 2 * r : 2 * r + 1, low ? 2 * r + 1 : 2 * r);
 }
 
 // Flux of every record of one step.  Single mesh (SEG = false): records
 // [0, npairs) are mirror pairs and the rest single slots, one per thread.
 // Batch (SEG = true): CTA b takes the scenario and record range of fseg[b].
-// Singles go through the queue as well, so side_record's code is there once.
+// Singles go through the queue as well, so that the main pass holds the common
+// case alone.
 template <class A, int VARIANT, int THREADS, int MINB, bool SEG>
 __global__ void __launch_bounds__(THREADS, MINB) flux_kernel(DevMesh<A> m, int k, int write_flux) {
-    __shared__ int queue[2 * THREADS];
+    __shared__ int entries[2 * THREADS];
     __shared__ int qn;
+    const SideQueue queue{entries, 2 * THREADS, &qn};
     if (threadIdx.x == 0) qn = 0;
     int r;
     bool valid, pair;
@@ -443,11 +491,16 @@ __global__ void __launch_bounds__(THREADS, MINB) flux_kernel(DevMesh<A> m, int k
     __syncthreads();
     const Terms<typename A::real> tout{m.slotw, 0};
     if (valid) {
-        if (pair) pair_record<A>(m, r, q, si, p, write_flux, tout, queue, &qn);
-        else queue[atomicAdd(&qn, 1)] = 2 * r;
+        if (pair) pair_record<A>(m, r, q, si, p, write_flux, tout, queue);
+        else queue.push(2 * r, -1);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < qn; i += THREADS) side_record<A, VARIANT>(m, queue[i], si, p, write_flux, tout);
+    const int nq = qn;
+    for (int j = threadIdx.x; j < 2 * nq; j += THREADS) {
+        const int e = queue.item(j, nq);
+        if (SEG ? pair : e >= 0 && (e >> 1) < m.npairs) pair_side<A, VARIANT>(m, e, si, p, write_flux, tout);
+        else if (e >= 0) side_record<A, VARIANT>(m, e, false, si, p, write_flux, tout);
+    }
 }
 
 // The fluxes of a cell's zero-length slot: the cell's state, no neighbour, zero
@@ -468,8 +521,8 @@ __device__ __forceinline__ ZeroSlot<typename A::real> zero_slot(const CellStateA
     in.cosj = R(0); in.sinj = R(0); in.side = R(0);
     auto nofetch = []() { return BoundaryInA<A>{}; };
     SlotOut<R> o;
-    if (write_flux) flux_slot<A, VARIANT, decltype(nofetch), false>(in, A::sqrt(A::mul(A::c(9.81), st.h)), p, nofetch, o);
-    else flux_chain<A, VARIANT, decltype(nofetch), true>(in, R(0), p, nofetch, o);
+    if (write_flux) flux_slot<A, VARIANT, decltype(nofetch), false>(in, p, nofetch, o);
+    else flux_chain<A, VARIANT, decltype(nofetch), true>(in, p, nofetch, o);
     return {{o.f[0], o.f[1], o.f[2], o.f[3]}};
 }
 // the fluxes of cell c's slots that are no real ones
@@ -844,9 +897,9 @@ __global__ void __launch_bounds__(THREADS, MINB) tile_kernel(DevMesh<A> m, int k
     using R = typename A::real;
     extern __shared__ __align__(16) unsigned char tile_smem[];
     R *terms = reinterpret_cast<R *>(tile_smem);                                       // [max cells][4 slots][4]
-    int *queue = reinterpret_cast<int *>(tile_smem + 16 * sizeof(R) * (size_t)m.max_tile_cells);
     __shared__ int qn;
     const TileDesc td = m.tiles[blockIdx.x];   // constant tables: read before the dependency wait
+    const SideQueue queue{reinterpret_cast<int *>(tile_smem + 16 * sizeof(R) * (size_t)m.max_tile_cells), 2 * td.npairs, &qn};
     const ScnParams sp = m.scn[td.scn];
     if (threadIdx.x == 0) qn = 0;
     Record<A> next{};
@@ -862,14 +915,16 @@ __global__ void __launch_bounds__(THREADS, MINB) tile_kernel(DevMesh<A> m, int k
     for (int i = threadIdx.x; i < td.npairs; i += THREADS) {
         const Record<A> q = next;
         if (i + THREADS < td.npairs) next = load_record(m, td.rec0 + i + THREADS);
-        pair_record<A>(m, td.rec0 + i, q, si, p, write_flux, tout, queue, &qn);
+        pair_record<A>(m, td.rec0 + i, q, si, p, write_flux, tout, queue);
     }
     __syncthreads();
     // the singles and the queued sides
-    const int sides = td.nsingles + qn;
-    for (int j = threadIdx.x; j < sides; j += THREADS)
-        side_record<A, VARIANT>(m, j < td.nsingles ? 2 * (td.rec0 + td.npairs + j) : queue[j - td.nsingles], si, p,
-                                write_flux, tout);
+    const int nq = qn, sides = td.nsingles + 2 * nq;
+    for (int j = threadIdx.x; j < sides; j += THREADS) {
+        const bool single = j < td.nsingles;
+        side_record<A, VARIANT>(m, single ? 2 * (td.rec0 + td.npairs + j) : queue.item(j - td.nsingles, nq), !single, si,
+                                p, write_flux, tout);
+    }
     CellIn<A> in{};
     if ((int)threadIdx.x < td.cells) in = load_cell_constants<A, VARIANT>(m, td.cell0 + threadIdx.x);
     __syncthreads();
@@ -957,15 +1012,21 @@ __global__ void __launch_bounds__(THREADS, MINB)
     // Every queued side is run before the grid barrier, as flux_kernel runs it
     // before it ends.
     constexpr int QCAP = 16 * THREADS;
-    __shared__ int queue[QCAP];
+    __shared__ int entries[QCAP];
     __shared__ int qn;
+    const SideQueue queue{entries, QCAP, &qn};
     const Terms<typename A::real> tout{m.slotw, 0};
     unsigned arrivals = 0;
     if (threadIdx.x == 0) qn = 0;
     __syncthreads();
-    auto run_queue = [&](const StepIndex &si, const StepParams &p, int wf) {   // all threads; empties the queue
+    // all threads; empties the queue (pairs: whether a batch's chunk holds pairs)
+    auto run_queue = [&](const StepIndex &si, const StepParams &p, int wf, bool pairs) {
         const int nq = qn;
-        for (int i = threadIdx.x; i < nq; i += THREADS) side_record<A, VARIANT>(m, queue[i], si, p, wf, tout);
+        for (int j = threadIdx.x; j < 2 * nq; j += THREADS) {
+            const int e = queue.item(j, nq);
+            if (SEG ? pairs : e >= 0 && (e >> 1) < m.npairs) pair_side<A, VARIANT>(m, e, si, p, wf, tout);
+            else if (e >= 0) side_record<A, VARIANT>(m, e, false, si, p, wf, tout);
+        }
         __syncthreads();
         if (threadIdx.x == 0) qn = 0;
         __syncthreads();
@@ -999,19 +1060,19 @@ __global__ void __launch_bounds__(THREADS, MINB)
             if ((int)threadIdx.x < cnt) {
                 const int r = r0 + (int)threadIdx.x;
                 const bool pair = SEG ? seg_pairs : r < m.npairs;
-                if (pair) pair_record<A>(m, r, load_record(m, r), si, p, wf, tout, queue, &qn);
-                else queue[atomicAdd(&qn, 1)] = 2 * r;
+                if (pair) pair_record<A>(m, r, load_record(m, r), si, p, wf, tout, queue);
+                else queue.push(2 * r, -1);
             }
             __syncthreads();   // the queue's count is complete
             // a batch chunk's sides have their scenario's parameters: its queue
             // runs at once; a single mesh's when another chunk might not fit
             bound += 2 * cnt;
             if (SEG || bound > QCAP - 2 * THREADS) {
-                run_queue(si, p, wf);
+                run_queue(si, p, wf, seg_pairs);
                 bound = 0;
             }
         }
-        if constexpr (!SEG) run_queue(si0, p0, wf);
+        if constexpr (!SEG) run_queue(si0, p0, wf, false);
         arrivals += gridDim.x;
         if (!grid_barrier(bar, arrivals + phantom, m.err, limit_ns)) return;
         for (int b = blockIdx.x; b < ncell; b += gridDim.x) {
