@@ -943,18 +943,15 @@ int get_flux_t(hb_handle *h, int s, hb::DevMesh<A> &m, double *F0, double *F1, d
     using R = typename A::real;
     const hb::Scenario &sc = h->scn[s];
     const int C = sc.cells;
-    const size_t S = 4 * (size_t)C;
-    std::vector<R> buf(4 * S);
     double *dst[4] = {F0, F1, F2, F3};
     HB_CUDA_RET(cudaDeviceSynchronize());
-    HB_CUDA_RET(cudaMemcpy(buf.data(), m.flux + 16 * (size_t)sc.cell0, 4 * S * sizeof(R), cudaMemcpyDeviceToHost));
-    for (int i = 0; i < C; i++)
-        for (int j = 0; j < 4; j++) {
-            const R *f = &buf[4 * (4 * (size_t)i + j)];
-            const size_t so = 4 * (size_t)sc.perm[i] + j;
-            for (int k = 0; k < 4; k++)
-                if (dst[k]) dst[k][so] = (double)f[k];
-        }
+    for (int k = 0; k < 4; k++) {
+        if (!dst[k]) continue;
+        hb::flux_out_kernel<R><<<(4 * C + 255) / 256, 256>>>(m.flux + 16 * (size_t)sc.cell0, C, k, h->d_perm + sc.cell0,
+                                                             h->d_stage);
+        HB_CUDA_RET(cudaGetLastError());
+        HB_CUDA_RET(cudaMemcpy(dst[k], h->d_stage, 4 * (size_t)C * sizeof(double), cudaMemcpyDeviceToHost));
+    }
     return HB_OK;
 }
 template <class A>
@@ -1321,25 +1318,39 @@ struct CheckpointHeader {
 };
 
 // The pieces of device memory a resumed run needs, in checkpoint order.  The
-// fluxes (`value` > 0, the size of one) are [slot][4] on the device and four
-// arrays in a checkpoint.
-struct CheckpointPiece { void *p; size_t bytes, value; };
+// fluxes are [slot][4] on the device and four arrays in a checkpoint.
+struct CheckpointPiece { void *p; size_t bytes; bool fluxes; };
 template <class A>
 std::vector<CheckpointPiece> checkpoint_pieces(hb_handle *h, hb::DevMesh<A> &m) {
     using R = typename A::real;
     const size_t C = (size_t)h->C;
     const int par = (int)(h->steps_done & 1);
-    return {{m.S[par], 4 * C * sizeof(R), 0}, {m.W, C * sizeof(R), 0}, {m.flux, 16 * C * sizeof(R), sizeof(R)},
-            {m.rmeta, (size_t)m.nrecords, 0}, {h->d_err, sizeof(uint32_t), 0}};
+    return {{m.S[par], 4 * C * sizeof(R), false}, {m.W, C * sizeof(R), false}, {m.flux, 16 * C * sizeof(R), true},
+            {m.rmeta, (size_t)m.nrecords, false}, {h->d_err, sizeof(uint32_t), false}};
 }
-// records of four values <-> four arrays of n values
-void records_to_arrays(const char *rec, char *arr, size_t n, size_t value) {
-    for (size_t i = 0; i < n; i++)
-        for (size_t k = 0; k < 4; k++) memcpy(arr + (k * n + i) * value, rec + (4 * i + k) * value, value);
-}
-void arrays_to_records(const char *arr, char *rec, size_t n, size_t value) {
-    for (size_t i = 0; i < n; i++)
-        for (size_t k = 0; k < 4; k++) memcpy(rec + (4 * i + k) * value, arr + (k * n + i) * value, value);
+// The fluxes to (or, `load`, from) a checkpoint's four arrays at `host`, through
+// the staging buffer, transposed on the device.
+template <class A>
+int checkpoint_fluxes(hb_handle *h, hb::DevMesh<A> &m, char *host, bool load) {
+    using R = typename A::real;
+    const size_t S = 4 * (size_t)h->C, room = 5 * (size_t)h->max_cells * sizeof(double) / sizeof(R);
+    R *stage = reinterpret_cast<R *>(h->d_stage);
+    for (int k = 0; k < 4; k++)
+        for (size_t s0 = 0; s0 < S; s0 += room) {
+            const size_t n = std::min(room, S - s0);
+            char *at = host + ((size_t)k * S + s0) * sizeof(R);
+            const unsigned blocks = (unsigned)((n + 255) / 256);
+            if (load) {
+                HB_CUDA_RET(cudaMemcpy(stage, at, n * sizeof(R), cudaMemcpyHostToDevice));
+                hb::flux_array_kernel<R, true><<<blocks, 256>>>(m.flux + 4 * s0, n, k, stage);
+                HB_CUDA_RET(cudaGetLastError());
+            } else {
+                hb::flux_array_kernel<R, false><<<blocks, 256>>>(m.flux + 4 * s0, n, k, stage);
+                HB_CUDA_RET(cudaGetLastError());
+                HB_CUDA_RET(cudaMemcpy(at, stage, n * sizeof(R), cudaMemcpyDeviceToHost));
+            }
+        }
+    return HB_OK;
 }
 }  // namespace
 
@@ -1370,13 +1381,8 @@ extern "C" int hb_checkpoint_save(hb_handle *h, void *buffer, size_t bytes) {
     int rc = h->with_mesh([&](auto &m) -> int {
         hd.nrecords = m.nrecords;
         for (auto &p : checkpoint_pieces(h, m)) {
-            if (p.value > 0) {
-                std::vector<char> rec(p.bytes);
-                HB_CUDA_RET(cudaMemcpy(rec.data(), p.p, p.bytes, cudaMemcpyDeviceToHost));
-                records_to_arrays(rec.data(), out, p.bytes / (4 * p.value), p.value);
-            } else {
-                HB_CUDA_RET(cudaMemcpy(out, p.p, p.bytes, cudaMemcpyDeviceToHost));
-            }
+            if (p.fluxes) TRY(checkpoint_fluxes(h, m, out, false));
+            else HB_CUDA_RET(cudaMemcpy(out, p.p, p.bytes, cudaMemcpyDeviceToHost));
             out += p.bytes;
         }
         return HB_OK;
@@ -1405,13 +1411,8 @@ extern "C" int hb_checkpoint_load(hb_handle *h, const void *buffer, size_t bytes
     const char *in = (const char *)buffer + sizeof hd;
     int rc = h->with_mesh([&](auto &m) -> int {
         for (auto &p : checkpoint_pieces(h, m)) {
-            if (p.value > 0) {
-                std::vector<char> rec(p.bytes);
-                arrays_to_records(in, rec.data(), p.bytes / (4 * p.value), p.value);
-                HB_CUDA_RET(cudaMemcpy(p.p, rec.data(), p.bytes, cudaMemcpyHostToDevice));
-            } else {
-                HB_CUDA_RET(cudaMemcpy(p.p, in, p.bytes, cudaMemcpyHostToDevice));
-            }
+            if (p.fluxes) TRY(checkpoint_fluxes(h, m, const_cast<char *>(in), true));
+            else HB_CUDA_RET(cudaMemcpy(p.p, in, p.bytes, cudaMemcpyHostToDevice));
             in += p.bytes;
         }
         return HB_OK;

@@ -1128,6 +1128,23 @@ struct SplitCodec {
     }
 };
 
+// Flux array k of one scenario's cells ([slot][4] records, device order) into
+// reference order.
+template <class R>
+__global__ void flux_out_kernel(const R *__restrict__ flux, int cells, int k, const int32_t *__restrict__ perm,
+                                double *__restrict__ out) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < 4 * cells) out[4 * (size_t)perm[s >> 2] + (s & 3)] = (double)flux[4 * (size_t)s + k];
+}
+// Flux array k of n records to an array of its own, or (SET) back.
+template <class R, bool SET>
+__global__ void flux_array_kernel(R *flux, size_t n, int k, R *array) {
+    const size_t s = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (s >= n) return;
+    if (SET) flux[4 * s + k] = array[s];
+    else array[s] = flux[4 * s + k];
+}
+
 // Reference-order staging <-> device-order state of one scenario: cells
 // [cell0, cell0 + C) of the device state, perm[new] = old within the scenario.
 template <class A>
