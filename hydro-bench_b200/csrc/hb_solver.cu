@@ -147,10 +147,9 @@ std::vector<int32_t> rcm_order(int C, const std::vector<int32_t> &nbr4) {
 // neighbours; then every tile under T/2 cells is merged into the adjacent
 // tile it shares most edges with, as long as the sum stays within 5T/4.
 // Returns order[new] = old with each tile contiguous, and the tile starts
-// (starts.back() == C).
-void tile_partition(int C, const std::vector<int32_t> &nbr4, int T, std::vector<int32_t> &order,
-                    std::vector<int32_t> &starts) {
-    const std::vector<int32_t> seeds = rcm_order(C, nbr4);
+// (starts.back() == C).  seeds: rcm_order(C, nbr4).
+void tile_partition(int C, const std::vector<int32_t> &nbr4, const std::vector<int32_t> &seeds, int T,
+                    std::vector<int32_t> &order, std::vector<int32_t> &starts) {
     std::vector<int32_t> tile(C, -1);
     std::vector<std::vector<int32_t>> cells;
     for (int seed : seeds) {
@@ -219,6 +218,76 @@ void tile_partition(int C, const std::vector<int32_t> &nbr4, int T, std::vector<
     starts.push_back((int32_t)order.size());
 }
 
+// The cells per tile that a balanced default starts from, and the whole waves
+// of `slots` resident CTAs that its tiles may fill (about 512 cells a tile).
+int balanced_tile_cells(long long total, long long slots, int &waves) {
+    waves = (int)std::max(1LL, (total + 512 * slots - 1) / (512 * slots));
+    const long long per_wave = waves * slots;
+    return (int)std::min(1024LL, std::max(64LL, (total + per_wave - 1) / per_wave));
+}
+
+// The tiles of every mesh (nbr4, seeds: per mesh) of up to `tile_cells` cells.
+// With waves > 0 (the balanced default) the size grows until the tiles fill at
+// most that many whole waves of `slots` resident CTAs (a tile count just above
+// a wave leaves most SMs idle while a few run the extra tiles).
+void tile_partitions(const std::vector<std::vector<int32_t>> &nbr4, const std::vector<std::vector<int32_t>> &seeds,
+                     long long slots, int waves, int &tile_cells, std::vector<std::vector<int32_t>> &order,
+                     std::vector<std::vector<int32_t>> &starts) {
+    const size_t n = nbr4.size();
+    order.assign(n, {});
+    starts.assign(n, {});
+    for (int pass = 0;; pass++) {
+        long long tiles = 0;
+        for (size_t s = 0; s < n; s++) {
+            tile_partition((int)seeds[s].size(), nbr4[s], seeds[s], tile_cells, order[s], starts[s]);
+            tiles += (long long)starts[s].size() - 1;
+        }
+        const long long cap = waves * slots;
+        if (waves <= 0 || pass == 3 || tiles <= cap || tile_cells >= 1024) return;
+        tile_cells = std::min(1024, (int)((tile_cells * tiles + cap - 1) / cap) + 1);
+    }
+}
+
+// The records of one scenario's slots (device order), tile by tile: the pairs
+// inside the tile, each listed from its lower-numbered side, then every other
+// real slot of the tile's cells.  nbr4: neighbour, -1 = none; meta4: the slot's
+// code byte; same_edge(sa, sb): the two slots have negated normals and the same
+// length, bit for bit (a zero component must have the opposite sign too: the
+// mirrored side is evaluated with the negated normal, and a wrongly signed zero
+// changes the sign of zero results).  on_tile(t) begins a tile, on_record(i, sa,
+// sb) lists a record of cell i (sb = -1: a single slot).
+template <class SameEdge, class OnTile, class OnRecord>
+void list_records(const std::vector<int32_t> &starts, const std::vector<int32_t> &nbr4,
+                  const std::vector<uint8_t> &meta4, const std::vector<char> &real4, const SameEdge &same_edge,
+                  const OnTile &on_tile, const OnRecord &on_record) {
+    std::vector<char> paired(nbr4.size(), 0);
+    for (size_t t = 0; t + 1 < starts.size(); t++) {
+        on_tile(t);
+        for (int i = starts[t]; i < starts[t + 1]; i++) {
+            for (int j = 0; j < 4; j++) {
+                const size_t sn = 4 * (size_t)i + j;
+                if (!real4[sn] || paired[sn] || (meta4[sn] & META_CODE) != CODE_ZERO || nbr4[sn] < 0) continue;
+                if (!(meta4[sn] & META_OWN_FIRST)) continue;
+                const int nb = nbr4[sn];
+                if (nb < starts[t] || nb >= starts[t + 1]) continue;
+                int jb = -1;
+                for (int q = 0; q < 4; q++)
+                    if (nbr4[4 * (size_t)nb + q] == i && !paired[4 * (size_t)nb + q]) { jb = q; break; }
+                if (jb < 0) continue;
+                const size_t sb = 4 * (size_t)nb + jb;
+                if ((meta4[sb] & META_CODE) != CODE_ZERO || !real4[sb] || !same_edge(sn, sb)) continue;
+                paired[sn] = paired[sb] = 1;
+                on_record(i, sn, (long long)sb);
+            }
+        }
+        for (int i = starts[t]; i < starts[t + 1]; i++)
+            for (int j = 0; j < 4; j++) {
+                const size_t sn = 4 * (size_t)i + j;
+                if (real4[sn] && !paired[sn]) on_record(i, sn, -1LL);
+            }
+    }
+}
+
 }  // namespace hb
 
 namespace {
@@ -252,11 +321,9 @@ struct HostMesh {
     std::vector<std::vector<R>> qw;
 };
 
-// Validates one scenario's mesh and appends it (renumbered) to hm.
-template <class A>
-int append_scenario(const hb_mesh_desc *md, int scn, const hb_options &opt, hb::Scenario &sc, HostMesh<A> &hm) {
-    using R = typename A::real;
-    using L = typename A::level;
+// Validates one scenario's mesh and returns its neighbour lists in input order,
+// for the renumbering.
+int scenario_neighbours(const hb_mesh_desc *md, std::vector<int32_t> &nbr_old) {
     if (md->cells <= 0 || md->ndays <= 0 || md->steps_per_day < 2 || md->nhq < 0)
         return hb::set_error(HB_E_INVALID, "mesh: cells=%d ndays=%d steps_per_day=%d", md->cells, md->ndays,
                              md->steps_per_day);
@@ -266,29 +333,28 @@ int append_scenario(const hb_mesh_desc *md, int scn, const hb_options &opt, hb::
     if (md->nhq > 0 && (!md->zw || !md->qw || !md->nhq1)) return hb::set_error(HB_E_INVALID, "mesh: missing rating tables");
     const int C = md->cells;
     const size_t S = 4 * (size_t)C;
-    sc.cells = C;
-    sc.cell0 = (int)hm.zbc.size();
-    sc.ndays = md->ndays; sc.nhq = md->nhq;
-    sc.steps_per_day = md->steps_per_day; sc.per_day = md->steps_per_day - 1;
-    sc.dt = md->dt; sc.hm1 = md->hm1; sc.hm2 = md->hm2; sc.jl = md->jl;
-    // neighbour lists in input order, for the renumbering
-    std::vector<int32_t> nbr_old(S, -1);
+    nbr_old.assign(S, -1);
     for (size_t s = 0; s < S; s++) {
         const int nc = (int)(md->nac[s] - 1.0);
         if (nc != -1 && (nc < 0 || nc >= C)) return hb::set_error(HB_E_BADMESH, "NAC[%zu] = %g out of range", s, md->nac[s]);
         nbr_old[s] = nc;
     }
-    std::vector<int32_t> starts;
-    if (opt.layout == HB_LAYOUT_TILE) {
-        hb::tile_partition(C, nbr_old, opt.tile_cells > 0 ? opt.tile_cells : 256, sc.perm, starts);
-    } else {
-        if (opt.renumber) sc.perm = hb::rcm_order(C, nbr_old);
-        else { sc.perm.resize(C); std::iota(sc.perm.begin(), sc.perm.end(), 0); }
-        starts = {0, C};
-    }
-    std::vector<int32_t> tile_of(C);
-    for (size_t t = 0; t + 1 < starts.size(); t++)
-        for (int i = starts[t]; i < starts[t + 1]; i++) tile_of[i] = (int32_t)t;
+    return HB_OK;
+}
+
+// Appends one scenario to hm in the order sc.perm, with the tiles at `starts`.
+template <class A>
+void append_scenario(const hb_mesh_desc *md, int scn, const std::vector<int32_t> &nbr_old,
+                     const std::vector<int32_t> &starts, hb::Scenario &sc, HostMesh<A> &hm) {
+    using R = typename A::real;
+    using L = typename A::level;
+    const int C = md->cells;
+    const size_t S = 4 * (size_t)C;
+    sc.cells = C;
+    sc.cell0 = (int)hm.zbc.size();
+    sc.ndays = md->ndays; sc.nhq = md->nhq;
+    sc.steps_per_day = md->steps_per_day; sc.per_day = md->steps_per_day - 1;
+    sc.dt = md->dt; sc.hm1 = md->hm1; sc.hm2 = md->hm2; sc.jl = md->jl;
     sc.inv.assign(C, -1);
     for (int i = 0; i < C; i++) sc.inv[sc.perm[i]] = i;
     sc.klas_orig.assign(md->klas, md->klas + S);
@@ -332,11 +398,8 @@ int append_scenario(const hb_mesh_desc *md, int scn, const hb_options &opt, hb::
             if (real4[4 * (size_t)i + j]) cm |= (uint8_t)(1u << j);
         hm.cmask.push_back(cm);
     }
-    // records, tile by tile: exact mirror pairs inside the tile first, then
-    // every other real slot of the tile's cells
     sc.rec0 = (int)hm.rix.size();
-    std::vector<char> paired(S, 0);
-    auto slot_of = [&](int i, int j) { return 4 * (size_t)perm[i] + j; };   // reference slot of device slot
+    auto slot_of = [&](size_t sn) { return 4 * (size_t)perm[sn >> 2] + (sn & 3); };   // reference slot of device slot
     auto push = [&](int a, int b, size_t sa, long long sb, uint8_t mt, size_t so) {
         hm.rix.push_back(make_int4(c0 + a, b < 0 ? -1 : c0 + b, (int)(4 * (size_t)c0 + sa),
                                    sb < 0 ? -1 : (int)(4 * (size_t)c0 + sb)));
@@ -354,45 +417,22 @@ int append_scenario(const hb_mesh_desc *md, int scn, const hb_options &opt, hb::
     sc.slot_index.assign(S, -1);
     sc.npairs = 0;
     sc.tiles.clear();
-    for (size_t t = 0; t + 1 < starts.size(); t++) {
-        hb::TileDesc td{scn, c0 + starts[t], starts[t + 1] - starts[t], (int)hm.rix.size(), 0, 0};
-        for (int i = starts[t]; i < starts[t + 1]; i++) {
-            for (int j = 0; j < 4; j++) {
-                const size_t sn = 4 * (size_t)i + j;
-                if (!real4[sn] || paired[sn] || (meta4[sn] & hb::META_CODE) != hb::CODE_ZERO || nbr4[sn] < 0) continue;
-                if (!(meta4[sn] & hb::META_OWN_FIRST)) continue;      // the pair is listed from its lower-numbered side
-                const int nb = nbr4[sn];
-                if (tile_of[nb] != (int32_t)t) continue;
-                int jb = -1;
-                for (int q = 0; q < 4; q++)
-                    if (nbr4[4 * (size_t)nb + q] == i && !paired[4 * (size_t)nb + q]) { jb = q; break; }
-                if (jb < 0) continue;
-                const size_t sb = 4 * (size_t)nb + jb;
-                const size_t oa = slot_of(i, j), ob = slot_of(nb, jb);
-                // the two slots must see one edge: code 0 both, negated normal, same
-                // length, bit for bit (a zero component must have the opposite sign
-                // too: the mirrored side is evaluated with the negated normal, and a
-                // wrongly signed zero changes the sign of zero results)
-                if ((meta4[sb] & hb::META_CODE) != hb::CODE_ZERO || !real4[sb] || !same_bits(md->cosf[ob], -md->cosf[oa]) ||
-                    !same_bits(md->sinf[ob], -md->sinf[oa]) || !same_bits(md->side[ob], md->side[oa]))
-                    continue;
-                paired[sn] = paired[sb] = 1;
-                push(i, nb, sn, (long long)sb, meta4[sn], oa);
-                td.npairs++;
-            }
-        }
-        for (int i = starts[t]; i < starts[t + 1]; i++) {
-            for (int j = 0; j < 4; j++) {
-                const size_t sn = 4 * (size_t)i + j;
-                if (!real4[sn] || paired[sn]) continue;
-                sc.slot_index[sn] = (int32_t)hm.rix.size();
-                push(i, nbr4[sn], sn, -1, meta4[sn], slot_of(i, j));
-                td.nsingles++;
-            }
-        }
-        sc.npairs += td.npairs;
-        sc.tiles.push_back(td);
-    }
+    hb::list_records(
+        starts, nbr4, meta4, real4,
+        [&](size_t sa, size_t sb) {
+            const size_t oa = slot_of(sa), ob = slot_of(sb);
+            return same_bits(md->cosf[ob], -md->cosf[oa]) && same_bits(md->sinf[ob], -md->sinf[oa]) &&
+                   same_bits(md->side[ob], md->side[oa]);
+        },
+        [&](size_t t) {
+            sc.tiles.push_back(hb::TileDesc{scn, c0 + starts[t], starts[t + 1] - starts[t], (int)hm.rix.size(), 0, 0});
+        },
+        [&](int i, size_t sa, long long sb) {
+            if (sb < 0) sc.slot_index[sa] = (int32_t)hm.rix.size();
+            push(i, nbr4[sa], sa, sb, meta4[sa], slot_of(sa));
+            (sb < 0 ? sc.tiles.back().nsingles : sc.tiles.back().npairs)++;
+            sc.npairs += sb >= 0;
+        });
     sc.nrecords = (int)hm.rix.size() - sc.rec0;
     // boundary table rows of the cells that need them
     const int NHQ = std::max(md->nhq, 0);
@@ -415,7 +455,6 @@ int append_scenario(const hb_mesh_desc *md, int scn, const hb_options &opt, hb::
         hm.nhq1.push_back(NHQ > 0 ? md->nhq1[old] : 0);
         hm.zw.push_back(zw); hm.qw.push_back(w);
     }
-    return HB_OK;
 }
 
 // Segment tables: CTAs of `threads` records (flux) or UPDATE_THREADS cells
@@ -446,25 +485,26 @@ int build_device_mesh(hb_handle *h, const hb_mesh_desc *mds, int n, hb::DevMesh<
     using R = typename A::real;
     using L = typename A::level;
     HostMesh<A> hm;
-    // tile layout: tiles of h->tile_cells cells; with the balanced default
-    // (tile_waves > 0) the size grows until the tiles fill at most tile_waves
-    // whole waves of tile_slots resident CTAs (a tile count just above a wave
-    // leaves most SMs idle while a few run the extra tiles)
-    hb_options opt = h->opt;
-    for (int pass = 0;; pass++) {
-        opt.tile_cells = h->tile_cells;
-        hm = HostMesh<A>();
-        h->scn.assign(n, hb::Scenario());
-        for (int s = 0; s < n; s++) {
-            const int st = append_scenario<A>(&mds[s], s, opt, h->scn[s], hm);
-            if (st != HB_OK) return n > 1 ? hb::set_error(st, "scenario %d: %s", s, hb_last_error_string()) : st;
+    h->scn.assign(n, hb::Scenario());
+    std::vector<std::vector<int32_t>> nbr(n), order(n), starts(n);
+    for (int s = 0; s < n; s++) {
+        const int st = scenario_neighbours(&mds[s], nbr[s]);
+        if (st != HB_OK) return n > 1 ? hb::set_error(st, "scenario %d: %s", s, hb_last_error_string()) : st;
+        if (h->opt.renumber || h->opt.layout == HB_LAYOUT_TILE) {
+            order[s] = hb::rcm_order(mds[s].cells, nbr[s]);
+        } else {
+            order[s].resize(mds[s].cells);
+            std::iota(order[s].begin(), order[s].end(), 0);
         }
-        if (opt.layout != HB_LAYOUT_TILE || h->tile_waves <= 0 || pass == 3) break;
-        long long tiles = 0;
-        for (const auto &sc : h->scn) tiles += (long long)sc.tiles.size();
-        const long long cap = (long long)h->tile_waves * h->tile_slots;
-        if (tiles <= cap || h->tile_cells >= 1024) break;
-        h->tile_cells = std::min(1024, (int)((h->tile_cells * tiles + cap - 1) / cap) + 1);
+        starts[s] = {0, mds[s].cells};
+    }
+    if (h->opt.layout == HB_LAYOUT_TILE) {
+        const std::vector<std::vector<int32_t>> seeds = std::move(order);
+        hb::tile_partitions(nbr, seeds, h->tile_slots, h->tile_waves, h->tile_cells, order, starts);
+    }
+    for (int s = 0; s < n; s++) {
+        h->scn[s].perm = std::move(order[s]);
+        append_scenario<A>(&mds[s], s, nbr[s], starts[s], h->scn[s], hm);
     }
     const int C = (int)hm.zbc.size();
     h->C = C;
@@ -861,9 +901,7 @@ extern "C" int hb_create_batch(const hb_mesh_desc *meshes, int32_t n, const hb_o
             return rs != HB_OK ? rs : hb::set_error(HB_E_CUDA, "hb_create: no tile CTA fits on an SM");
         }
         h->tile_slots = sms * per_sm;
-        h->tile_waves = (int)std::max(1LL, (total + 512LL * h->tile_slots - 1) / (512LL * h->tile_slots));
-        const long long per_wave = (long long)h->tile_waves * h->tile_slots;
-        h->tile_cells = (int)std::min(1024LL, std::max(64LL, (total + per_wave - 1) / per_wave));
+        h->tile_cells = hb::balanced_tile_cells(total, h->tile_slots, h->tile_waves);
     }
     int st;
     if ((st = dev_alloc(h, &h->d_err, 1)) != HB_OK || (st = dev_alloc(h, &h->d_ctr, 1)) != HB_OK ||
@@ -1352,6 +1390,157 @@ int checkpoint_fluxes(hb_handle *h, hb::DevMesh<A> &m, char *host, bool load) {
         }
     return HB_OK;
 }
+// Whether the record codes of a checkpoint are those of `codes` (a handle's or
+// a partition's), but for the slots that breach (KLAS 7 turns into 0).
+bool same_codes(const uint8_t *a, const uint8_t *b, size_t n) {
+    for (size_t r = 0; r < n; r++) {
+        if (a[r] == b[r]) continue;
+        const uint8_t ca = a[r] & hb::META_CODE, cb = b[r] & hb::META_CODE;
+        if ((a[r] ^ b[r]) & ~hb::META_CODE) return false;
+        if (!((ca == hb::CODE_K7 && cb == hb::CODE_ZERO) || (ca == hb::CODE_ZERO && cb == hb::CODE_K7))) return false;
+    }
+    return true;
+}
+
+// A checkpoint is in the device order of its handle.  With balanced tiles that
+// order follows from how many CTAs of the launch shape an SM holds, which
+// changes with the shape and from build to build (207,234 cells: 443 tiles at
+// 3 CTAs per SM, the default until 4 per SM was, 590 now).  So a handle with
+// balanced tiles recognises its own partition by the record codes, and
+// otherwise makes the partitions of 1 to 8 CTAs per SM until one has the
+// checkpoint's records, and moves the payload from it into its own order.
+// The mesh is read back from the device's records; edges of two of the
+// handle's tiles count as mirror pairs where their fp32 geometry mirrors.
+// payload: in, of hd.nrecords records; out: this handle's, empty if none fits.
+template <class A>
+int reorder_checkpoint(hb_handle *h, const hb::DevMesh<A> &m, int nrecords, const char *payload,
+                       std::vector<char> &out) {
+    using R = typename A::real;
+    out.clear();
+    const size_t C = (size_t)h->C, S = 4 * C, nr = (size_t)m.nrecords;
+    std::vector<int4> rix(nr);
+    std::vector<R> rgeo(4 * nr);
+    HB_CUDA_RET(cudaMemcpy(rix.data(), m.rix, nr * sizeof(int4), cudaMemcpyDeviceToHost));
+    HB_CUDA_RET(cudaMemcpy(rgeo.data(), m.rgeo, 4 * nr * sizeof(R), cudaMemcpyDeviceToHost));
+    // every scenario's slots in input order: neighbour, real or not, geometry
+    // {COSF, SINF, SIDE}, and the slot it is known to mirror or not (pairs and
+    // the edges within a tile: partner + 1, 0 = not, -1 = not known)
+    struct Mesh { std::vector<int32_t> nbr; std::vector<char> real; std::vector<R> geo; std::vector<long long> twin; };
+    const size_t n = h->scn.size();
+    std::vector<Mesh> mesh(n);
+    std::vector<std::vector<int32_t>> nbr(n), seeds(n);
+    for (size_t s = 0; s < n; s++) {
+        const hb::Scenario &sc = h->scn[s];
+        const size_t Ss = 4 * (size_t)sc.cells;
+        Mesh &g = mesh[s];
+        g.real.assign(Ss, 0);
+        g.geo.assign(3 * Ss, R(0));
+        g.twin.assign(Ss, 0);
+        nbr[s].assign(Ss, -1);
+        auto input = [&](int sd) {   // device slot -> the scenario's slot in input order
+            const int i = sd - 4 * sc.cell0;
+            return 4 * (size_t)sc.perm[i >> 2] + (i & 3);
+        };
+        auto cell = [&](int c) { return c < 0 ? -1 : sc.perm[c - sc.cell0]; };
+        for (const hb::TileDesc &td : sc.tiles)
+            for (int r = td.rec0; r < td.rec0 + td.npairs + td.nsingles; r++) {
+                const int4 ix = rix[r];
+                const size_t sa = input(ix.z);
+                const R *q = &rgeo[4 * (size_t)r];
+                g.real[sa] = 1;
+                nbr[s][sa] = cell(ix.y);
+                for (int k = 0; k < 3; k++) g.geo[3 * sa + k] = q[k];
+                const bool other_tile = ix.y >= 0 && (ix.y < td.cell0 || ix.y >= td.cell0 + td.cells);
+                g.twin[sa] = other_tile ? -1 : 0;
+                if (ix.w < 0) continue;
+                const size_t sb = input(ix.w);
+                g.real[sb] = 1;
+                nbr[s][sb] = cell(ix.x);
+                for (int k = 0; k < 3; k++) g.geo[3 * sb + k] = k < 2 ? -q[k] : q[k];
+                g.twin[sa] = (long long)sb + 1;
+                g.twin[sb] = (long long)sa + 1;
+            }
+        seeds[s] = hb::rcm_order(sc.cells, nbr[s]);
+    }
+    int sms = 0;
+    HB_CUDA_RET(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->opt.device));
+    const char *state = payload, *w = state + 4 * C * sizeof(R), *flux = w + C * sizeof(R), *codes = flux + 4 * S * sizeof(R);
+    for (int per_sm = 1; per_sm <= 8; per_sm++) {
+        if (sms * per_sm == h->tile_slots) continue;
+        int waves = 0, tile_cells = hb::balanced_tile_cells(h->C, sms * per_sm, waves);
+        std::vector<std::vector<int32_t>> order, starts;
+        hb::tile_partitions(nbr, seeds, sms * per_sm, waves, tile_cells, order, starts);
+        std::vector<uint8_t> want;                     // the partition's record codes
+        std::vector<int32_t> record_of(S, -1);         // this handle's device slot -> its record there
+        for (size_t s = 0; s < n; s++) {
+            const hb::Scenario &sc = h->scn[s];
+            const std::vector<int32_t> &perm = order[s];
+            std::vector<int32_t> inv(sc.cells), nb4(4 * (size_t)sc.cells, -1);
+            for (int i = 0; i < sc.cells; i++) inv[perm[i]] = i;
+            std::vector<uint8_t> meta4(4 * (size_t)sc.cells);
+            std::vector<char> real4(4 * (size_t)sc.cells);
+            auto input = [&](size_t sn) { return 4 * (size_t)perm[sn >> 2] + (sn & 3); };
+            for (size_t sn = 0; sn < meta4.size(); sn++) {
+                const size_t so = input(sn);
+                const int nc = nbr[s][so];
+                meta4[sn] = (uint8_t)hb::klas_code(sc.klas_orig[so]);
+                if (nc >= 0) {
+                    nb4[sn] = inv[nc];
+                    meta4[sn] |= hb::META_HAS_NB;
+                    if ((int)(so >> 2) < nc) meta4[sn] |= hb::META_OWN_FIRST;
+                }
+                real4[sn] = mesh[s].real[so];
+            }
+            hb::list_records(
+                starts[s], nb4, meta4, real4,
+                [&](size_t sa, size_t sb) {
+                    const Mesh &g = mesh[s];
+                    const size_t oa = input(sa), ob = input(sb);
+                    if (g.twin[oa] >= 0) return g.twin[oa] == (long long)ob + 1;
+                    const R *x = &g.geo[3 * oa], *y = &g.geo[3 * ob];
+                    return same_bits(y[0], -x[0]) && same_bits(y[1], -x[1]) && same_bits(y[2], x[2]);
+                },
+                [](size_t) {},
+                [&](int i, size_t sa, long long) {
+                    record_of[4 * ((size_t)sc.cell0 + sc.inv[perm[i]]) + (sa & 3)] = (int32_t)want.size();
+                    want.push_back(meta4[sa]);
+                });
+        }
+        if (want.size() != (size_t)nrecords || !same_codes(want.data(), (const uint8_t *)codes, want.size())) continue;
+        out.resize((5 * C + 4 * S) * sizeof(R) + nr + sizeof(uint32_t));
+        char *o_state = out.data(), *o_w = o_state + 4 * C * sizeof(R), *o_flux = o_w + C * sizeof(R),
+             *o_codes = o_flux + 4 * S * sizeof(R);
+        for (size_t s = 0; s < n; s++) {
+            const hb::Scenario &sc = h->scn[s];
+            for (int i = 0; i < sc.cells; i++) {
+                const size_t from = (size_t)sc.cell0 + i, to = (size_t)sc.cell0 + sc.inv[order[s][i]];
+                memcpy(o_state + 4 * to * sizeof(R), state + 4 * from * sizeof(R), 4 * sizeof(R));
+                memcpy(o_w + to * sizeof(R), w + from * sizeof(R), sizeof(R));
+                for (int k = 0; k < 4; k++)
+                    memcpy(o_flux + (k * S + 4 * to) * sizeof(R), flux + (k * S + 4 * from) * sizeof(R), 4 * sizeof(R));
+            }
+        }
+        // a single slot's code as the checkpoint has it; a pair's, and a slot
+        // that is a pair there, as the handle lists it
+        for (size_t r = 0; r < nr; r++) {
+            const int4 ix = rix[r];
+            const int old = record_of[ix.z];
+            const hb::Scenario &sc = *std::find_if(h->scn.begin(), h->scn.end(), [&](const hb::Scenario &q) {
+                return ix.x < q.cell0 + q.cells;
+            });
+            const size_t so = 4 * (size_t)sc.perm[ix.x - sc.cell0] + (ix.z & 3);
+            uint8_t meta = (uint8_t)hb::klas_code(sc.klas_orig[so]);
+            if (ix.y >= 0) {
+                meta |= hb::META_HAS_NB;
+                if ((int)(so >> 2) < sc.perm[ix.y - sc.cell0]) meta |= hb::META_OWN_FIRST;
+            }
+            o_codes[r] = (char)(old < 0 ? meta : (uint8_t)((meta & ~hb::META_CODE) | (codes[old] & hb::META_CODE)));
+        }
+        memcpy(o_codes + nr, codes + nrecords, sizeof(uint32_t));
+        return HB_OK;
+    }
+    return HB_OK;
+}
 }  // namespace
 
 extern "C" int hb_checkpoint_size(hb_handle *h, size_t *bytes) {
@@ -1399,16 +1588,38 @@ extern "C" int hb_checkpoint_load(hb_handle *h, const void *buffer, size_t bytes
     if (memcmp(hd.magic, "HBCKPT1", 8) != 0) return hb::set_error(HB_E_INVALID, "hb_checkpoint_load: not a checkpoint");
     int nrec = 0;
     h->with_mesh([&](auto &m) { nrec = m.nrecords; return HB_OK; });
+    const bool balanced = h->tile_waves > 0;
     if (hd.precision != h->opt.precision || hd.variant != h->opt.variant || hd.layout != h->opt.layout ||
         hd.tile_cells != h->opt.tile_cells || hd.renumber != h->opt.renumber || hd.cells != h->C ||
-        hd.nscen != (int32_t)h->scn.size() || hd.nrecords != nrec)
+        hd.nscen != (int32_t)h->scn.size() || (hd.nrecords != nrec && !balanced))
         return hb::set_error(HB_E_INVALID, "hb_checkpoint_load: the checkpoint is of another mesh or other options");
     if (hd.steps_done < 0 || hd.steps_done > h->step_limit())
         return hb::set_error(HB_E_INVALID, "hb_checkpoint_load: position %lld beyond the boundary tables", (long long)hd.steps_done);
-    if (bytes < sizeof hd + hd.payload) return hb::set_error(HB_E_INVALID, "hb_checkpoint_load: truncated checkpoint");
+    size_t own = 0;
+    TRY(hb_checkpoint_size(h, &own));
+    if (hd.nrecords < 0 || hd.payload != own - sizeof hd - (size_t)nrec + (size_t)hd.nrecords || bytes < sizeof hd + hd.payload)
+        return hb::set_error(HB_E_INVALID, "hb_checkpoint_load: truncated checkpoint");
     HB_CUDA_RET(cudaDeviceSynchronize());
-    h->steps_done = hd.steps_done;   // the state goes into buffer (steps_done & 1)
     const char *in = (const char *)buffer + sizeof hd;
+    std::vector<char> reordered;
+    if (balanced) {
+        const char *codes = in + hd.payload - sizeof(uint32_t) - (size_t)hd.nrecords;
+        TRY(h->with_mesh([&](auto &m) -> int {
+            std::vector<uint8_t> now((size_t)nrec);
+            HB_CUDA_RET(cudaMemcpy(now.data(), m.rmeta, now.size(), cudaMemcpyDeviceToHost));
+            if (hd.nrecords == nrec && same_codes(now.data(), (const uint8_t *)codes, now.size())) return HB_OK;
+            try {
+                TRY(reorder_checkpoint(h, m, hd.nrecords, in, reordered));
+            } catch (const std::bad_alloc &) {
+                return hb::set_error(HB_E_NOMEM, "hb_checkpoint_load: no host memory to reorder the checkpoint");
+            }
+            if (reordered.empty())
+                return hb::set_error(HB_E_INVALID, "hb_checkpoint_load: the checkpoint is of another mesh or other options");
+            in = reordered.data();
+            return HB_OK;
+        }));
+    }
+    h->steps_done = hd.steps_done;   // the state goes into buffer (steps_done & 1)
     int rc = h->with_mesh([&](auto &m) -> int {
         for (auto &p : checkpoint_pieces(h, m)) {
             if (p.fluxes) TRY(checkpoint_fluxes(h, m, const_cast<char *>(in), true));

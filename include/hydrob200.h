@@ -190,7 +190,10 @@ int hb_write_dump(hb_handle *h, int32_t s, const hb_mesh_desc *mesh, const char 
  * (KLAS 7 slots breach), the device error bits and the step position -- in
  * one host buffer of hb_checkpoint_size bytes.  A checkpoint loads into a
  * handle of the same mesh(es) and options (precision, variant, layout,
- * tile_cells, renumbering); a captured graph stays valid. */
+ * tile_cells, renumbering); a captured graph stays valid.  With balanced tiles
+ * (tile_cells = 0, fp32 or split) it also loads where the tiles were balanced
+ * for another number of CTAs per SM (another launch shape, or a build with
+ * another default), reordered on the host. */
 int hb_checkpoint_size(hb_handle *h, size_t *bytes);
 int hb_checkpoint_save(hb_handle *h, void *buffer, size_t bytes);
 int hb_checkpoint_load(hb_handle *h, const void *buffer, size_t bytes);
