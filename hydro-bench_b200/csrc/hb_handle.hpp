@@ -143,11 +143,11 @@ int hb_tiles_set_smem(hb_handle *h);
 // CTAs per SM of a tile-layout launch shape with tiles of about tile_cells cells
 int hb_tiles_resident(hb_handle *h, int config, int tile_cells, int *per_sm);
 // Small fp64 meshes (hb_cells.cu): whether the handle's steps run as one
-// cell_kernel launch each, the slot table those kernels read, and n such
-// steps (without the counter's tick; coef: also the update coefficients)
+// cell_kernel launch each, the slot table those kernels read (from the cells'
+// slot masks and the device mesh), and n such steps (tick: the counter's advance
+// after the last one; coef: also the update coefficients)
 bool hb_cells_used(const hb_handle *h);
-int hb_cells_build(hb_handle *h, const std::vector<int4> &rix, const std::vector<uint8_t> &rmeta,
-                   const std::vector<double> &rgeo);
+int hb_cells_build(hb_handle *h, const std::vector<uint8_t> &cmask);
 int hb_cells_launch(hb_handle *h, const hb::DevMesh<hb::F64Exact> &m, int k0, int n, int write_last, int tick,
                     bool coef, cudaStream_t st);
 // One fp64 edge-layout step t0 + k (the device step counter must hold t0)

@@ -563,13 +563,24 @@ int build_device_mesh(hb_handle *h, const hb_mesh_desc *mds, int n, hb::DevMesh<
     TRY(dev_upload(h, &lp, bzw)); m.bzw = lp;
     TRY(dev_upload(h, &rp, bqw)); m.bqw = rp;
     const size_t S = 4 * (size_t)C;
-    for (int b = 0; b < 2; b++) TRY(dev_alloc(h, &m.S[b], 4 * (size_t)C));
-    TRY(dev_alloc(h, &m.slotw, 16 * (size_t)C));
-    TRY(dev_alloc(h, &m.W, C));
-    TRY(dev_alloc(h, &m.flux, 4 * S));
+    // state, terms, fluxes and the like, zeroed: one allocation (an allocation
+    // beyond the driver's small blocks takes about 0.1 ms)
     R *dta = nullptr, *sidex = nullptr;
-    TRY(dev_alloc(h, &dta, C));
-    TRY(dev_alloc(h, &sidex, C));
+    {
+        const size_t Cs = (size_t)C;
+        const std::pair<R **, size_t> arrays[] = {{&m.S[0], 4 * Cs}, {&m.S[1], 4 * Cs}, {&m.slotw, 16 * Cs}, {&m.W, Cs},
+                                                  {&m.flux, 4 * S}, {&dta, Cs}, {&sidex, Cs}};
+        auto aligned = [](size_t bytes) { return (bytes + 255) & ~(size_t)255; };
+        size_t total = aligned(5 * (size_t)h->max_cells * sizeof(double));
+        for (const auto &a : arrays) total += aligned(a.second * sizeof(R));
+        char *block;
+        TRY(dev_alloc(h, &block, total));
+        for (const auto &a : arrays) {
+            *a.first = reinterpret_cast<R *>(block);
+            block += aligned(a.second * sizeof(R));
+        }
+        h->d_stage = reinterpret_cast<double *>(block);
+    }
     for (const auto &sc : h->scn) {
         const int blocks = (sc.cells + 255) / 256;
         const size_t c0 = sc.cell0;
@@ -626,8 +637,7 @@ int build_device_mesh(hb_handle *h, const hb_mesh_desc *mds, int n, hb::DevMesh<
     std::vector<int32_t> perms;
     for (const auto &sc : h->scn) perms.insert(perms.end(), sc.perm.begin(), sc.perm.end());
     TRY(dev_upload(h, &h->d_perm, perms));
-    TRY(dev_alloc(h, &h->d_stage, 5 * (size_t)h->max_cells));
-    if constexpr (std::is_same<A, hb::F64Exact>::value) TRY(hb_cells_build(h, hm.rix, hm.rmeta, hm.rgeo));
+    if constexpr (std::is_same<A, hb::F64Exact>::value) TRY(hb_cells_build(h, hm.cmask));
     return HB_OK;
 }
 

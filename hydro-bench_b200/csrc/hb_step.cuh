@@ -735,7 +735,7 @@ struct SlotRef {
     int place;                 // 4 * (cell - the CTA's first cell) + j
     uint8_t meta;
     int record;
-    static inline unsigned long long pack(int nb, int place, uint8_t meta, int record) {
+    static __device__ __forceinline__ unsigned long long pack(int nb, int place, uint8_t meta, int record) {
         return (unsigned long long)((unsigned)record << 8 | meta) << 32 |
                ((unsigned)place << 24 | (unsigned)(nb < 0 ? NO_NB : nb));
     }
