@@ -24,12 +24,13 @@ def _dp(a):
 
 
 class Adjoint:
-    """The rollout, its loss and gradient on one fp64 variant-H handle."""
+    """The rollout, its loss and gradient on one fp64 variant-H handle
+    (``tile_config``: its launch shape, as in ``Solver``)."""
 
     def __init__(self, deck: Deck, gauges: Sequence[int], obs_every: int, nsteps: int, checkpoint_every: int = 10,
-                 device: int = 0):
+                 device: int = 0, tile_config: int = 0):
         self.deck = deck
-        self.solver = Solver(deck, variant="H", precision="fp64", device=device, init_state=False)
+        self.solver = Solver(deck, variant="H", precision="fp64", device=device, tile_config=tile_config, init_state=False)
         self.gauges = np.ascontiguousarray(gauges, dtype=np.int32)
         self.obs_every, self.nsteps, self.k = int(obs_every), int(nsteps), int(checkpoint_every)
         self.nobs = self.nsteps // self.obs_every
