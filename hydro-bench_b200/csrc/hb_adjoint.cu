@@ -121,7 +121,7 @@ __device__ __forceinline__ OsherFwd osher_fwd(double cl, const double ql[3], con
         o.us6 = A::divk(o.p5 ? o.fir5 : o.fir, 3.0);
         o.hs6 = A::divk(A::mul(o.us6, o.us6), 9.81);
     }
-    // FLUX3 as qf_acc_if sums it: out3 += +-4.905 h * h over the active pieces in order
+    // FLUX3 as qf_acc sums it: out3 += +-4.905 h * h over the active pieces in order
     double o3 = 0.0;
     auto acc = [&](bool on, double sign, double h) {
         const double h4 = A::mul(A::c(4.905), h);
@@ -755,7 +755,7 @@ __device__ __forceinline__ void linearise_edge(const SlotInA<A> &in, double ql1,
 // |U2| < 15, the only case in which its adjoint passes (at the clamp, xn holds
 // +-15 and the adjoint is cut).
 //
-// Bound by that chain and, at 24,020 cells (751 CTAs, one wave at 6 CTAs per
+// Bound by that chain and, at 24,020 cells (754 CTAs, one wave at 6 CTAs per
 // SM), by the linearisation in front of it: 7.2 us per reverse step there and
 // 4.0 us at 6,000 cells.  Four lanes per cell, everything after the wait and
 // the general reverse of every slot (1,376 instructions per warp, 464 bytes of

@@ -10,12 +10,12 @@ namespace {
 // once (edge layout, default launch shape): about 33,000 triangles on a B200.
 // It halves the latencies of a step but computes every edge twice, and its
 // second wave costs as much as its first.  us per step, 40-step graphs, one
-// launch / two kernels, variant H:
+// launch / two kernels (the dam break after 1,500 steps), variant H:
 //   cells      24,021      32,000      40,000      60,000
-//   channel   4.6 / 6.8   4.6 / 7.7   7.7 / 7.7   8.7*/ 8.7
-//   mixed     5.2 / 7.9   7.7*/ 7.7   8.1*/ 8.0  10.1*/ 10.1
-//   dam break 6.7 / 8.8   6.8 / 8.9     -  / 9.1     -  / 11.4
-// (* two waves)
+//   channel   4.5 / 7.0   4.6 / 8.1   7.7*/ 8.2   8.7*/ 7.8
+//   mixed     5.2 / 7.8   7.7*/ 8.0   8.1*/ 8.5  10.1*/ 10.8
+//   dam break 6.3 / 8.7   6.9 / 9.0     -  / 9.3     -  / 10.0
+// (* two waves; a mesh with quads has fewer cells to a CTA)
 bool fits_at_once(const hb_handle *h, size_t ctas) {
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->opt.device) != cudaSuccess) return false;

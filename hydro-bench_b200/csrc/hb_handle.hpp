@@ -151,9 +151,9 @@ int hb_cells_build(hb_handle *h, const std::vector<uint8_t> &cmask);
 int hb_cells_launch(hb_handle *h, const hb::DevMesh<hb::F64Exact> &m, int k0, int n, int write_last, int tick,
                     bool coef, cudaStream_t st);
 // One fp64 edge-layout step t0 + k (the device step counter must hold t0)
-// from state `in` to state `out` ([C][4] each), keeping the slots' terms of
-// the cell sums in `terms` ([4C][4]) and the update coefficients of the wet
-// cells in `coef` ([C][UPDATE_COEF]); the handle's W is overwritten, its
-// fluxes only when `write_flux` is set.
+// from state `in` to state `out` ([C][4] each), with the update coefficients
+// of the wet cells in `coef` ([C][UPDATE_COEF]).  `terms` ([4C][4]) is scratch:
+// the two kernels pass the slots' terms through it, the one-launch step leaves
+// it as it is.  The handle's W and fluxes are written only with `write_flux`.
 int hb_forward_step_into(hb_handle *h, long long t0, int k, const double *in, double *out, double *terms,
                          double *coef, int write_flux, cudaStream_t st);

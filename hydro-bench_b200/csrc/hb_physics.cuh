@@ -292,8 +292,6 @@ __device__ __forceinline__ void qf_acc(typename A::real out[4], bool neg, typena
 // every case lists its pieces in increasing order.  Here the six pieces are
 // taken in that order and each is added when its case coefficient is
 // non-zero: the same sums in the same order, without one branch per case.
-// Pieces without a division are formed on every lane and selected; those
-// with one are formed only by the lanes that take them.
 // Piece 3 updates FIL and piece 5 updates FIR (QS<3>, QS<5>); no case has
 // both, and piece 6 sees the FIR that piece 5 left.
 template <class A>
@@ -359,8 +357,11 @@ __device__ __forceinline__ void osher(typename A::real cl, const typename A::rea
 // K2 = 1: piece 1; K1 = 3, K2 = 4: piece 7).  osher()'s result for them, from `cr`
 // = sqrt(9.81*QR[0]).  False (and no result) in any other case, at UA = -CA, and
 // where a depth or CA leaves the range in which the policy's quotients by a
-// constant need no checks (quotient_range): with CA or the depth in it, HA and
-// FLUX3 are in divk_raw's range too.
+// constant need no checks (quotient_range).  With CA or the depth in it, D^2, HA
+// and FLUX3 = 4.905 HA^2 are neither so large nor so small that a quotient or its
+// exact remainder (24 or 53 bits below it) leaves the normal numbers: in fp32
+// FLUX3 is at least 2^-65 (below divk's 2^-60, which has more room than needed)
+// and its remainder a multiple of 2^-111, in fp64 2^-805 and 2^-909.
 template <class A>
 __device__ __forceinline__ bool osher_one_piece(typename A::real cl, typename A::real cr, const typename A::real ql[3],
                                                 const typename A::real qr[3], typename A::real fil,

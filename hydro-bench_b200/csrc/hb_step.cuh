@@ -885,13 +885,13 @@ __global__ void __launch_bounds__(CELL_THREADS, CELL_CTAS) cell_kernel(DevMesh<A
 // step index and the first cell's constants are loaded ahead of what they
 // would wait behind.
 //
-// A 207,234-cell mesh is one wave of 443 CTAs, three to an SM, bound by issue
-// (half of the cycles) and the latencies of its phases.  us per step, split
-// precision, 207,234-cell channel / 500,001-cell dam break, and fp32, 61,003
-// mixed cells: 13.0 / 29.3 / 7.0 before pair_record's common case, 10.4 / 24.8 /
-// 5.8 with it, 10.0 / 23.5 / 5.8 with the next record's load, 9.8 / 23.5 / 5.6
-// with the early loads.  Chunks of 32 pairs drawn from a counter: 10.6 / 25.4 /
-// 5.8.
+// A 207,234-cell mesh is one wave of 590 CTAs, four to an SM (fp32 and split),
+// bound by issue (half of the cycles) and the latencies of its phases.  us per
+// step, split precision, 207,234-cell channel / 500,001-cell dam break, and fp32,
+// 61,003 mixed cells, three CTAs to an SM: 13.0 / 29.3 / 7.0 before pair_record's
+// common case, 10.4 / 24.8 / 5.8 with it, 10.0 / 23.5 / 5.8 with the next
+// record's load, 9.8 / 23.5 / 5.6 with the early loads (four: DEFAULT_TILE_CONFIG).
+// Chunks of 32 pairs drawn from a counter: 10.6 / 25.4 / 5.8.
 template <class A, int VARIANT, int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) tile_kernel(DevMesh<A> m, int k, int write_flux) {
     using R = typename A::real;
