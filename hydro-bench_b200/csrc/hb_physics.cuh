@@ -813,7 +813,7 @@ __device__ __forceinline__ bool edge_deep(const CellStateA<A> &a, const CellStat
 // The common case of an interior slot (code 0) across an edge from the
 // lower-numbered cell a to b, by the direct route (the slot of a) or the
 // mirrored one (that of b); (cosj, sinj) is the slot's own normal.  Both cells
-// deep (edge_deep) and the flow across the edge subcritical, or both dry; false,
+// deep (edge_deep) and Osher with one piece (osher_one_piece), or both dry; false,
 // and no result, in any other case.  The caller loads the cells in this order:
 // selecting their five values instead costs forty selects.
 template <class A>
